@@ -39,6 +39,7 @@
 // warp 13: TMA producer.  S^T/dP^T of tile i+1 are issued as soon as tile i
 // has been pulled into registers, so the tensor core overlaps the exp math.
 #include "attn_bwd128.h"
+#include "attn_bwd_split.h"
 #include "common.cuh"
 #include "host_util.h"
 
@@ -86,12 +87,12 @@ struct BwParams {
   const int* qlist;
   const uint8_t* qflags;
   int qmax;
-  // dense mode: the query tiles of a K/V tile are split over `qsplit` CTAs (blockIdx.z =
-  // batch * qsplit + part) to even out the last wave; each writes unscaled fp32 partial
-  // dK / dV to part[r] = (B, L, H, 64) and a second kernel adds them up
-  int qsplit;
-  float* part_dk;
-  float* part_dv;
+  int n_t;                // K/V tiles per (batch, head)
+  // dense mode: the query tiles of each K/V tile from n_whole on are split over `parts` CTAs to
+  // even out the last wave (attn_bwd_split.h); each writes unscaled fp32 partial dK / dV to
+  // part[(tile - n_whole) * parts + r] = [dK | dV][128][64] and a second kernel adds them up
+  int n_whole, parts;
+  float* part;
   // fixed-order dQ (null = adds land in arrival order): one counter per (batch, head, query
   // tile), zeroed before the launch.  The CTA whose ordinal equals the counter adds its tile
   // and then raises the counter.  Dense: ordinal = K/V tile index; block-sparse: qrank[entry]
@@ -123,12 +124,16 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // block-sparse lists can be very uneven (the always-attended tail tiles are attended by every
   // query tile and sit at the end): walk the K/V tiles from the back so the long ones start first
-  // grid = (chains, K/V tiles): blockIdx.x = head + H * (batch * qsplit + part) varies fastest,
-  // so the resident CTAs are a few K/V tiles of EVERY chain rather than many of one
-  const int kvb = p.qlist ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y;
-  const int h = blockIdx.x % p.H, bz = blockIdx.x / p.H;
-  const int b = bz / p.qsplit, qpart = bz % p.qsplit;
-  const size_t lrow = (((size_t)b * p.H + h) * gridDim.y + kvb) * (size_t)p.qmax;
+  // item = chain (batch, head) + chains * K/V tile: the resident CTAs are a few K/V tiles of
+  // EVERY chain rather than many of one
+  const int idx = (int)blockIdx.x;
+  const bool split = idx >= p.n_whole;
+  const int item = split ? p.n_whole + (idx - p.n_whole) / p.parts : idx;
+  const int qpart = split ? (idx - p.n_whole) % p.parts : 0;
+  const int chains = p.B * p.H, kv_ord = item / chains, chain = item % chains;
+  const int kvb = p.qlist ? p.n_t - 1 - kv_ord : kv_ord;
+  const int h = chain % p.H, b = chain / p.H;
+  const size_t lrow = ((size_t)chain * p.n_t + kvb) * (size_t)p.qmax;
   const int* qlist = p.qlist ? p.qlist + lrow : nullptr;
   const uint8_t* qflags = p.qflags ? p.qflags + lrow : nullptr;
   const uint16_t* qrank = (p.qlist && p.qrank) ? p.qrank + lrow : nullptr;
@@ -139,8 +144,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     n_q = 0;
     while (n_q < p.qmax && qlist[n_q] >= 0) ++n_q;
   } else {
-    q_first = (int)((long)qpart * n_q / p.qsplit);
-    n_q = (int)((long)(qpart + 1) * n_q / p.qsplit) - q_first;
+    const int parts = split ? p.parts : 1;
+    q_first = (int)((long)qpart * n_q / parts);
+    n_q = (int)((long)(qpart + 1) * n_q / parts) - q_first;
   }
 
   if (threadIdx.x == 0) {
@@ -465,9 +471,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           wg == 0 ? p.dk + (int64_t)b * p.dk_sb + (int64_t)kv_row * p.dk_sl + (int64_t)h * p.dk_sh
                   : p.dv + (int64_t)b * p.dv_sb + (int64_t)kv_row * p.dv_sl + (int64_t)h * p.dv_sh;
       float* pbase = nullptr;
-      if (p.qsplit > 1)
-        pbase = (wg == 0 ? p.part_dk : p.part_dv) +
-                ((((size_t)qpart * p.B + b) * p.L + kv_row) * p.H + h) * BW_HD;
+      if (split)
+        pbase = p.part + (((size_t)(idx - p.n_whole) * 2 + wg) * BW_T + row) * BW_HD;
 #pragma unroll
       for (int c = 0; c < BW_HD; c += 32) {
         uint32_t r[32];
@@ -628,57 +633,38 @@ __global__ void attn_bwd_post_kernel(const float* __restrict__ acc, __nv_bfloat1
   reinterpret_cast<uint2*>(dq)[i] = o;
 }
 
-// dk = scale * sum_r part_dk[r], dv = sum_r part_dv[r] (fixed order), rows of 64 channels.
-__global__ void attn_bwd_combine_kernel(const float* __restrict__ part_dk,
-                                        const float* __restrict__ part_dv,
-                                        __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv,
-                                        int qsplit, int B, int L, int H, int64_t dk_sb, int64_t dk_sl,
-                                        int64_t dk_sh, int64_t dv_sb, int64_t dv_sl, int64_t dv_sh,
-                                        float scale) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;     // one float4 of one row
-  const long rows = (long)B * L * H;
-  if (i >= rows * 16) return;
-  const long row = i >> 4;
-  const int c = (int)(i & 15) * 4;
-  const int h = (int)(row % H), l = (int)((row / H) % L), b = (int)(row / ((long)H * L));
-  const size_t plane = (size_t)rows * 64;
-  float4 a = make_float4(0.f, 0.f, 0.f, 0.f), v = a;
-  for (int r = 0; r < qsplit; ++r) {
-    const float4 x = *reinterpret_cast<const float4*>(part_dk + r * plane + row * 64 + c);
-    const float4 y = *reinterpret_cast<const float4*>(part_dv + r * plane + row * 64 + c);
+// dK = scale * sum_r part[r].dK, dV = sum_r part[r].dV (fixed order) of the split K/V tiles.  One
+// thread per 4 channels of a row of dK or dV.
+__global__ void attn_bwd_combine_kernel(const BwParams p, int n_split, float scale) {
+  constexpr int ROW4 = BW_HD / 4, TILE4 = BW_T * ROW4;
+  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (i >= n_split * 2 * TILE4) return;
+  const int c = (i % ROW4) * 4, row = (i / ROW4) % BW_T, which = (i / TILE4) & 1, t = i / (2 * TILE4);
+  const int item = p.n_whole + t, chains = p.B * p.H, chain = item % chains;
+  const int h = chain % p.H, b = chain / p.H;
+  const int kv_row = (item / chains) * BW_T + row;
+  if (kv_row >= p.L) return;
+  const float* src = p.part + (((size_t)t * p.parts * 2 + which) * BW_T + row) * BW_HD + c;
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int r = 0; r < p.parts; ++r) {
+    const float4 x = *reinterpret_cast<const float4*>(src + (size_t)r * 2 * BW_T * BW_HD);
     a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
-    v.x += y.x; v.y += y.y; v.z += y.z; v.w += y.w;
   }
+  const float mul = which == 0 ? scale : 1.f;
   uint2 o;
-  o.x = pack_bf16(a.x * scale, a.y * scale);
-  o.y = pack_bf16(a.z * scale, a.w * scale);
-  *reinterpret_cast<uint2*>(dk + b * dk_sb + (int64_t)l * dk_sl + h * dk_sh + c) = o;
-  o.x = pack_bf16(v.x, v.y);
-  o.y = pack_bf16(v.z, v.w);
-  *reinterpret_cast<uint2*>(dv + b * dv_sb + (int64_t)l * dv_sl + h * dv_sh + c) = o;
+  o.x = pack_bf16(a.x * mul, a.y * mul);
+  o.y = pack_bf16(a.z * mul, a.w * mul);
+  __nv_bfloat16* dst =
+      which == 0 ? p.dk + (int64_t)b * p.dk_sb + (int64_t)kv_row * p.dk_sl + (int64_t)h * p.dk_sh
+                 : p.dv + (int64_t)b * p.dv_sb + (int64_t)kv_row * p.dv_sl + (int64_t)h * p.dv_sh;
+  *reinterpret_cast<uint2*>(dst + c) = o;
 }
 
-// Number of CTAs the query tiles of one K/V tile are split over (dense mode): the smallest
-// of 1..3 whose last wave wastes less than 6 % on this GPU.
-static int bwd_qsplit(int B, int L, int H) {
-  int dev = 0, sms = 0;        // of the current device (a host may hold GPUs of different sizes)
-  cudaGetDevice(&dev);
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-    sms = 148;
-  const long n_t = (L + BW_T - 1) / BW_T;
-  const long items = n_t * H * B;
-  int best = 1;
-  double best_w = 1e9;
-  for (int s = 1; s <= 3 && s * 8 <= n_t; ++s) {
-    const double waves = (double)items * s / sms;
-    const double w = (double)((items * s + sms - 1) / sms) / waves;
-    if (w < best_w - 0.02) {
-      best_w = w;
-      best = s;
-    }
-    if (w < 1.06) break;
-  }
-  return best;
+// A CTA's start, pipeline fill and epilogue cost about 2.5 of its 1.8 us query steps.
+static BwdSplit bwd64_split(int B, int L, int H) {
+  const int n_t = (L + BW_T - 1) / BW_T;
+  return bwd_split((long)n_t * H * B, n_t, bwd_sm_count(), 2.5f);
 }
 
 static int make_map64(CUtensorMap* m, const void* ptr, int B, int L, int H, int64_t sb, int64_t sl,
@@ -696,8 +682,8 @@ static int make_map64(CUtensorMap* m, const void* ptr, int B, int L, int H, int6
 // are split) fp32 partial dK / dV.
 extern "C" long imf_attn_bwd_scratch_bytes(int B, int L, int H) {
   const long Lp = ((L + 127) / 128) * 128;
-  const int qs = imf::bwd_qsplit(B, L, H);
-  const long part = qs > 1 ? 2L * qs * B * L * H * 64 * 4 : 0;
+  const imf::BwdSplit sp = imf::bwd64_split(B, L, H);
+  const long part = 2L * sp.n_split * sp.parts * imf::BW_T * imf::BW_HD * 4;
   const long turns = (long)B * H * (Lp / 128) * 4 + 256;     // fixed-order dQ: one counter per query tile
   return (long)B * L * H * 64 * 4 + turns + 2 * (long)B * H * Lp * 32 + (long)B * L * H * 64 * 2 +
          1024 + part;
@@ -759,13 +745,8 @@ extern "C" int imf_attn_bwd(const void* q, const void* k, const void* v, const v
   cur += (size_t)B * H * Lp * 32;
   __nv_bfloat16* qs = reinterpret_cast<__nv_bfloat16*>(cur);
   cur += ((size_t)B * L * H * 64 * 2 + 255) & ~size_t(255);
-  const int qsplit = qlist ? 1 : bwd_qsplit(B, L, H);
-  float* part_dk = nullptr;
-  float* part_dv = nullptr;
-  if (qsplit > 1) {
-    part_dk = reinterpret_cast<float*>(cur);
-    part_dv = part_dk + (size_t)qsplit * B * L * H * 64;
-  }
+  const int n_t = (L + BW_T - 1) / BW_T;
+  const BwdSplit sp = qlist ? BwdSplit{n_t * B * H, 1, 0} : bwd64_split(B, L, H);
   if (cudaMemsetAsync(dq_acc, 0, acc_bytes + turn_bytes, st) != cudaSuccess) return IMF_ERR_LAUNCH;
   {
     const long rows = (long)B * H * Lp;
@@ -820,9 +801,10 @@ extern "C" int imf_attn_bwd(const void* q, const void* k, const void* v, const v
   prm.qlist = qlist;
   prm.qflags = qflags;
   prm.qmax = qlist ? qmax : 0;
-  prm.qsplit = qsplit;
-  prm.part_dk = part_dk;
-  prm.part_dv = part_dv;
+  prm.n_t = n_t;
+  prm.n_whole = sp.n_whole;
+  prm.parts = sp.parts;
+  prm.part = sp.n_split ? reinterpret_cast<float*>(cur) : nullptr;
   prm.turn = ordered ? turn : nullptr;
   prm.qrank = ordered ? qrank : nullptr;
   const size_t smem = sizeof(BwSmem) + 1024;
@@ -830,15 +812,12 @@ extern "C" int imf_attn_bwd(const void* q, const void* k, const void* v, const v
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return IMF_ERR_LAUNCH;
-  dim3 grid(H * B * qsplit, (L + BW_T - 1) / BW_T, 1);
-  kern<<<grid, BW_THREADS, smem, st>>>(mq, mk, mv, mdo, mdq, maq, mad, prm);
+  kern<<<sp.ctas(), BW_THREADS, smem, st>>>(mq, mk, mv, mdo, mdq, maq, mad, prm);
   if (cudaGetLastError() != cudaSuccess) return IMF_ERR_LAUNCH;
-  if (qsplit > 1) {
-    const long n = (long)B * L * H * 16;
-    attn_bwd_combine_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
-        part_dk, part_dv, static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), qsplit,
-        B, L, H, dk_strides[0], dk_strides[1], dk_strides[2], dv_strides[0], dv_strides[1],
-        dv_strides[2], 0.6931471805599453f);      // partial dK = dS^T (Q scale log2e)
+  if (sp.n_split) {
+    const int n = sp.n_split * 2 * BW_T * (BW_HD / 4);
+    attn_bwd_combine_kernel<<<(n + 255) / 256, 256, 0, st>>>(
+        prm, sp.n_split, 0.6931471805599453f);      // partial dK = dS^T (Q scale log2e)
     if (cudaGetLastError() != cudaSuccess) return IMF_ERR_LAUNCH;
   }
   const long n4 = (long)B * L * H * 64 / 4;

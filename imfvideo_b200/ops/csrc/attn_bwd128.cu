@@ -23,6 +23,7 @@
 // issuer; warp 13: TMA producer.  S^T / dP^T of tile i+1 are issued as soon as
 // tile i has been pulled into registers.
 #include "attn_bwd128.h"
+#include "attn_bwd_split.h"
 #include "common.cuh"
 #include "host_util.h"
 
@@ -71,11 +72,11 @@ struct Params {
   int64_t dk_sb, dk_sl, dk_sh, dv_sb, dv_sl, dv_sh;
   float scale;
   int* status;
-  // the query tiles of a K/V tile are split over `qsplit` CTAs (blockIdx.z = batch * qsplit +
-  // part); each writes unscaled fp32 partial dK / dV and a second kernel adds them up
-  int qsplit;
-  float* part_dk;
-  float* part_dv;
+  // the query tiles of each K/V tile from n_whole on are split over `parts` CTAs to even out the
+  // last wave (attn_bwd_split.h); each writes unscaled fp32 partial dK / dV to
+  // part[(tile - n_whole) * parts + r] = [dK | dV][128][128] and a second kernel adds them up
+  int n_whole, parts;
+  float* part;
   // fixed-order dQ (null = arrival order): one counter per (batch, head, 64-row query step),
   // zeroed before the launch; the CTA of K/V tile j adds when the counter shows j
   int* turn;
@@ -96,16 +97,19 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   auto& s = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                      ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // grid = (chains, K/V tiles) with blockIdx.x = head + H * (batch * qsplit + part) fastest: a
-  // CTA waits (fixed-order dQ) only for the K/V tile before it in its chain, whose block index
-  // is smaller, and the resident CTAs are a few tiles of every chain
-  const int kvb = (int)blockIdx.y;
-  const int h = blockIdx.x % p.H, bz = blockIdx.x / p.H;
-  const int b = bz / p.qsplit, qpart = bz % p.qsplit;
+  // item = chain (batch, head) + chains * K/V tile: a CTA waits (fixed-order dQ) only for the K/V
+  // tile before it in its chain, whose block index is smaller, and the resident CTAs are a few
+  // tiles of every chain
+  const int idx = (int)blockIdx.x;
+  const bool split = idx >= p.n_whole;
+  const int item = split ? p.n_whole + (idx - p.n_whole) / p.parts : idx;
+  const int qpart = split ? (idx - p.n_whole) % p.parts : 0, parts = split ? p.parts : 1;
+  const int chains = p.B * p.H, kvb = item / chains, chain = item % chains;
+  const int h = chain % p.H, b = chain / p.H;
   int n_q = (p.L + QT - 1) / QT;
   int* turn = p.turn ? p.turn + ((size_t)b * p.H + h) * n_q : nullptr;
-  const int q_first = (int)((long)qpart * n_q / p.qsplit);
-  n_q = (int)((long)(qpart + 1) * n_q / p.qsplit) - q_first;
+  const int q_first = (int)((long)qpart * n_q / parts);
+  n_q = (int)((long)(qpart + 1) * n_q / parts) - q_first;
 
   if (threadIdx.x == 0) {
     mbar_init(&s.kv_full, 1);
@@ -382,9 +386,7 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           wg == 0 ? p.dk + (int64_t)b * p.dk_sb + (int64_t)kv_row * p.dk_sl + (int64_t)h * p.dk_sh
                   : p.dv + (int64_t)b * p.dv_sb + (int64_t)kv_row * p.dv_sl + (int64_t)h * p.dv_sh;
       float* pbase = nullptr;
-      if (p.qsplit > 1)
-        pbase = (wg == 0 ? p.part_dk : p.part_dv) +
-                ((((size_t)qpart * p.B + b) * p.L + kv_row) * p.H + h) * HD;
+      if (split) pbase = p.part + (((size_t)(idx - p.n_whole) * 2 + wg) * KT + row) * HD;
 #pragma unroll 1
       for (int c = 0; c < HD; c += 32) {
         uint32_t r[32];
@@ -466,57 +468,38 @@ __global__ void attn_bwd128_post_kernel(const float* __restrict__ acc, __nv_bflo
   reinterpret_cast<uint2*>(dq)[i] = o;
 }
 
-// dk = scale * sum_r part_dk[r], dv = sum_r part_dv[r] (fixed order), rows of 128 channels.
-__global__ void attn_bwd128_combine_kernel(const float* __restrict__ part_dk,
-                                           const float* __restrict__ part_dv,
-                                           __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv,
-                                           int qsplit, int B, int L, int H, int64_t dk_sb,
-                                           int64_t dk_sl, int64_t dk_sh, int64_t dv_sb, int64_t dv_sl,
-                                           int64_t dv_sh, float scale) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;     // one float4 of one row
-  const long rows = (long)B * L * H;
-  if (i >= rows * (HD / 4)) return;
-  const long row = i / (HD / 4);
-  const int c = (int)(i % (HD / 4)) * 4;
-  const int h = (int)(row % H), l = (int)((row / H) % L), b = (int)(row / ((long)H * L));
-  const size_t plane = (size_t)rows * HD;
-  float4 a = make_float4(0.f, 0.f, 0.f, 0.f), v = a;
-  for (int r = 0; r < qsplit; ++r) {
-    const float4 x = *reinterpret_cast<const float4*>(part_dk + r * plane + row * HD + c);
-    const float4 y = *reinterpret_cast<const float4*>(part_dv + r * plane + row * HD + c);
+// dK = scale * sum_r part[r].dK, dV = sum_r part[r].dV (fixed order) of the split K/V tiles.  One
+// thread per 4 channels of a row of dK or dV.
+__global__ void attn_bwd128_combine_kernel(const Params p, int n_split, float scale) {
+  constexpr int ROW4 = HD / 4, TILE4 = KT * ROW4;
+  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (i >= n_split * 2 * TILE4) return;
+  const int c = (i % ROW4) * 4, row = (i / ROW4) % KT, which = (i / TILE4) & 1, t = i / (2 * TILE4);
+  const int item = p.n_whole + t, chains = p.B * p.H, chain = item % chains;
+  const int h = chain % p.H, b = chain / p.H;
+  const int kv_row = (item / chains) * KT + row;
+  if (kv_row >= p.L) return;
+  const float* src = p.part + (((size_t)t * p.parts * 2 + which) * KT + row) * HD + c;
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int r = 0; r < p.parts; ++r) {
+    const float4 x = *reinterpret_cast<const float4*>(src + (size_t)r * 2 * KT * HD);
     a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
-    v.x += y.x; v.y += y.y; v.z += y.z; v.w += y.w;
   }
+  const float mul = which == 0 ? scale : 1.f;
   uint2 o;
-  o.x = pack_bf16(a.x * scale, a.y * scale);
-  o.y = pack_bf16(a.z * scale, a.w * scale);
-  *reinterpret_cast<uint2*>(dk + b * dk_sb + (int64_t)l * dk_sl + h * dk_sh + c) = o;
-  o.x = pack_bf16(v.x, v.y);
-  o.y = pack_bf16(v.z, v.w);
-  *reinterpret_cast<uint2*>(dv + b * dv_sb + (int64_t)l * dv_sl + h * dv_sh + c) = o;
+  o.x = pack_bf16(a.x * mul, a.y * mul);
+  o.y = pack_bf16(a.z * mul, a.w * mul);
+  __nv_bfloat16* dst =
+      which == 0 ? p.dk + (int64_t)b * p.dk_sb + (int64_t)kv_row * p.dk_sl + (int64_t)h * p.dk_sh
+                 : p.dv + (int64_t)b * p.dv_sb + (int64_t)kv_row * p.dv_sl + (int64_t)h * p.dv_sh;
+  *reinterpret_cast<uint2*>(dst + c) = o;
 }
 
-// Number of CTAs the query tiles of one K/V tile are split over: the smallest of 1..3 whose
-// last wave wastes less than 6 % on this GPU.
-static int qsplit_for(int B, int L, int H) {
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-    sms = 148;
-  const long n_t = (L + KT - 1) / KT;
-  const long items = n_t * H * B;
-  int best = 1;
-  double best_w = 1e9;
-  for (int sp = 1; sp <= 3 && sp * 8 <= n_t; ++sp) {
-    const double waves = (double)items * sp / sms;
-    const double w = (double)((items * sp + sms - 1) / sms) / waves;
-    if (w < best_w - 0.02) {
-      best_w = w;
-      best = sp;
-    }
-    if (w < 1.06) break;
-  }
-  return best;
+// A CTA's start, pipeline fill and epilogue cost about 4 of its 64-row query steps.
+static BwdSplit split_for(int B, int L, int H) {
+  const int n_t = (L + KT - 1) / KT, n_q = (L + QT - 1) / QT;
+  return bwd_split((long)n_t * H * B, n_q, bwd_sm_count(), 4.f);
 }
 
 static int make_map(CUtensorMap* m, const void* ptr, int B, int L, int H, int64_t sb, int64_t sl,
@@ -531,8 +514,8 @@ static int make_map(CUtensorMap* m, const void* ptr, int B, int L, int H, int64_
 
 long attn_bwd128_scratch_bytes(int B, int L, int H) {
   const long Lp = ((L + 127) / 128) * 128;
-  const int qs = b128::qsplit_for(B, L, H);
-  const long part = qs > 1 ? 2L * qs * B * L * H * b128::HD * 4 : 0;
+  const BwdSplit sp = b128::split_for(B, L, H);
+  const long part = 2L * sp.n_split * sp.parts * b128::KT * b128::HD * 4;
   const long turns = (long)B * H * (Lp / b128::QT) * 4 + 256;   // fixed-order dQ counters
   return (long)B * L * H * b128::HD * 4 + turns + 2 * (long)B * H * Lp * 4 + 512 + part;
 }
@@ -550,14 +533,8 @@ int attn_bwd128_launch(const Bwd128Args& a) {
   const size_t turn_bytes = ((size_t)B * H * (Lp / QT) * 4 + 255) & ~size_t(255);
   float* lse2 = reinterpret_cast<float*>(static_cast<uint8_t*>(a.scratch) + acc_bytes + turn_bytes);
   float* delta = lse2 + (size_t)B * H * Lp;
-  const int qsplit = qsplit_for(B, L, H);
-  float* part_dk = nullptr;
-  float* part_dv = nullptr;
-  if (qsplit > 1) {
-    const uintptr_t end = (reinterpret_cast<uintptr_t>(delta + (size_t)B * H * Lp) + 255) & ~uintptr_t(255);
-    part_dk = reinterpret_cast<float*>(end);
-    part_dv = part_dk + (size_t)qsplit * B * L * H * HD;
-  }
+  const BwdSplit sp = split_for(B, L, H);
+  const uintptr_t end = (reinterpret_cast<uintptr_t>(delta + (size_t)B * H * Lp) + 255) & ~uintptr_t(255);
   if (cudaMemsetAsync(dq_acc, 0, acc_bytes + turn_bytes, st) != cudaSuccess) return IMF_ERR_LAUNCH;
   {
     const long warps = (long)B * H * Lp;
@@ -593,22 +570,19 @@ int attn_bwd128_launch(const Bwd128Args& a) {
   prm.dv_sb = a.dv_strides[0]; prm.dv_sl = a.dv_strides[1]; prm.dv_sh = a.dv_strides[2];
   prm.scale = a.scale;
   prm.status = a.status;
-  prm.qsplit = qsplit;
+  prm.n_whole = sp.n_whole;
+  prm.parts = sp.parts;
+  prm.part = sp.n_split ? reinterpret_cast<float*>(end) : nullptr;
   prm.turn = (a.fixed_order && a.status != nullptr) ? turn : nullptr;
-  prm.part_dk = part_dk;
-  prm.part_dv = part_dv;
   const size_t smem = sizeof(Smem) + 1024;
   if (cudaFuncSetAttribute(attn_bwd128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem) != cudaSuccess)
     return IMF_ERR_LAUNCH;
-  dim3 grid(H * B * qsplit, (L + KT - 1) / KT, 1);
-  attn_bwd128_kernel<<<grid, THREADS, smem, st>>>(mq, mk, mv, mdo, mdq, prm);
+  attn_bwd128_kernel<<<sp.ctas(), THREADS, smem, st>>>(mq, mk, mv, mdo, mdq, prm);
   if (cudaGetLastError() != cudaSuccess) return IMF_ERR_LAUNCH;
-  if (qsplit > 1) {
-    const long n = (long)B * L * H * (HD / 4);
-    attn_bwd128_combine_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
-        part_dk, part_dv, prm.dk, prm.dv, qsplit, B, L, H, prm.dk_sb, prm.dk_sl, prm.dk_sh,
-        prm.dv_sb, prm.dv_sl, prm.dv_sh, a.scale);
+  if (sp.n_split) {
+    const int n = sp.n_split * 2 * KT * (HD / 4);
+    attn_bwd128_combine_kernel<<<(n + 255) / 256, 256, 0, st>>>(prm, sp.n_split, a.scale);
     if (cudaGetLastError() != cudaSuccess) return IMF_ERR_LAUNCH;
   }
   const long n4 = (long)B * L * H * HD / 4;

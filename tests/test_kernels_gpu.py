@@ -211,6 +211,33 @@ def test_attention_autograd(K):
     K.check_status()
 
 
+@pytest.mark.parametrize("B,L,H,hd", [(1, 257, 1, 64), (1, 532, 4, 64), (2, 500, 3, 128),
+                                      (1, 2500, 9, 64), (1, 2500, 9, 128)])
+def test_attention_backward_split_tiles(K, B, L, H, hd):
+    """K/V tiles whose query walk is cut into parts: all of them (few tiles), the ragged last one,
+    and (2500 rows, 9 heads: 180 tiles) only those behind the last full wave.  Four roundings to
+    bf16 (P, dS, operands, result) of at most 2^-9 each bound the relative error."""
+    from imfvideo_b200.ops import reference as ref
+
+    g = torch.Generator(device="cuda").manual_seed(L)
+    q, k, v, go = (torch.randn(B, L, H, hd, device="cuda", generator=g).bfloat16() for _ in range(4))
+    o, _, lse = K.attn_fwd(q, k, v)
+    got = K.attn_bwd(q, k, v, o, lse, go)
+    qf, kf, vf = (t.float().requires_grad_(True) for t in (q, k, v))
+    ref.attention(qf, kf, vf).backward(go.float())
+    for a, b in zip(got, (qf.grad, kf.grad, vf.grad)):
+        assert _rel(a, b) < 8e-3
+    again = K.attn_bwd(q, k, v, o, lse, go)
+    assert torch.equal(got[1], again[1]) and torch.equal(got[2], again[2])   # parts: fixed order
+    K.set_deterministic(True)
+    try:
+        first, second = (K.attn_bwd(q, k, v, o, lse, go)[0] for _ in range(2))
+    finally:
+        K.set_deterministic(False)
+    assert torch.equal(first, second) and _rel(first, got[0]) < 1e-3
+    K.check_status()
+
+
 @pytest.mark.parametrize("B,L,H", [(1, 128, 1), (1, 300, 2), (2, 1000, 3), (1, 2049, 2)])
 def test_attention_backward(K, B, L, H):
     from imfvideo_b200.ops import reference as ref
