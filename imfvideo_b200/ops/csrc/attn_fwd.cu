@@ -10,32 +10,28 @@
 // flash-JVP kernel (reference models/flash_jvp_kernel.py:51-570,
 // models/triton_block_jvp.py:228-346) and the FA/SDPA primal forward.
 //
-// Work item = NT 128-row query tiles that share every K/V tile, of one (batch,
-// head): NT = 3 tiles against 64-row K/V tiles in the primal kernel (2 tiles
-// against 128-row K/V tiles when three would leave SMs without an item), 2
-// tiles in the tangent kernel.  Warps 4t .. 4t+3: softmax + O-correction + epilogue
-// of tile t (one query row per thread, rows live in TMEM lanes); then one warp
-// with the single-thread tcgen05.mma issuer, one TMA producer warp and two
-// warps that only donate registers (setmaxnreg).  The tiles take turns: while
+// Work item = NT 128-row query tiles that share every 64-row K/V tile, of one (batch,
+// head): four tiles in the primal kernel (three where rounding L up to 512 rows wastes more
+// than that gains), two in the tangent kernel; TMEM (512 columns) holds no more.  Warps
+// 4t .. 4t+3: softmax + O-correction + epilogue of tile t (one query row per thread, rows live
+// in TMEM lanes); then one warp with the single-thread tcgen05.mma issuer, one TMA producer
+// warp and two warps that only donate registers (setmaxnreg).  The tiles take turns: while
 // one tile's softmax runs on the CUDA cores the tensor core works on another.
-// The softmax warps are bound by instruction issue and dependency latency
-// (two of them per scheduler reach 0.43 instructions per cycle), which is why
-// the primal kernel keeps three tiles in flight.  P (and T) are written back
-// to TMEM as bf16 over the S (dS) columns and are the A operand of the second
-// GEMM.  In the primal kernel V carries 16 extra columns of ones, so the row
-// sum l comes out of the tensor core as column 64 of O.  O is rescaled lazily
-// (only when the running max grows by > 2^8).
+// The softmax warps are bound by dependency latency first (0.4 instructions per cycle and
+// scheduler, exponential unit three quarters busy), so what counts is how many tiles are in
+// flight: B 1, H 4, L 29,140 takes 1.02 ms with four tiles, 1.08 to 1.16 with three.  Pairs of
+// scores go through packed fp32 instructions.  P (and T) are written back to TMEM as bf16 over
+// the S (dS) columns and are the A operand of the second GEMM.  O is rescaled lazily (only
+// when the running max grows by > 2^8).
 //
-// Scheduling: the grid is persistent (one CTA per SM).  The flattened
-// (item, K/V tile) iteration space is cut into equal contiguous shares, so an
-// item may be split between two neighbouring CTAs; such partial results
-// (un-normalised accumulators + running max) go to a scratch buffer and a
-// small second kernel merges them.  This removes the wave quantisation that
-// equal items on 148 SMs would cost (304 items = 2.05 waves at 29,140 rows).
+// Scheduling: a persistent grid whose CTAs take equal shares of the flattened
+// (item, K/V tile) space (attn_fwd_split.h); the partial results of split items go
+// to a scratch buffer and a small second kernel merges them.
 //
 // Tensors are (B, L, H, 64) bf16 with arbitrary 16-byte-aligned strides;
 // ragged L is handled by TMA zero fill + masking of the last K/V tile.
 #include "attn_fwd128.h"
+#include "attn_fwd_split.h"
 #include "common.cuh"
 #include "host_util.h"
 
@@ -44,23 +40,18 @@ namespace imf {
 constexpr int ATT_HD = 64;
 constexpr int ATT_TILE_M = 128;
 
-// Work item = NT query tiles of 128 rows that share every K/V tile.
-//   tangent kernel : NT 2, K/V tiles of 64 rows, TMEM per tile S|dS|O|dO
-//   primal kernel  : NT 2, K/V tiles of 128 rows, row sum on the tensor core (ones column)
-//                    NT 3, K/V tiles of 64 rows, ones column
-//                    NT 4, K/V tiles of 64 rows, row sum in registers
-// More tiles in flight put more softmax warps on each scheduler (the softmax
-// warps are bound by instruction issue and dependency latency, not by a pipe).
+// Work item = NT query tiles of 128 rows that share every 64-row K/V tile.
+//   tangent kernel : NT 2, TMEM per tile S|dS|O|dO
+//   primal kernel  : NT 3 or 4, TMEM per tile S|O
 template <bool TANGENT, int NTP>
 struct AttCfg {
-  static constexpr int NT = TANGENT ? 2 : NTP;
+  static constexpr int NT = NTP;
   static constexpr int ITEM_M = NT * ATT_TILE_M;
-  static constexpr int BN = (TANGENT || NT > 2) ? 64 : 128;
+  static constexpr int BN = 64;
   static constexpr int NQ = TANGENT ? 2 : 1;       // q + dq
   static constexpr int NKV = TANGENT ? 4 : 2;      // k, v (+ dk, dv)
-  static constexpr int STAGES = (!TANGENT && NT > 2) ? 4 : 3;
-  static constexpr bool ONES = !TANGENT && NT < 4; // row sum on the tensor core
-  static constexpr int N_PV = ONES ? ATT_HD + 16 : ATT_HD;
+  static constexpr int V = TANGENT ? 2 : 1;        // v's place: k, v  or  k, dk, v, dv
+  static constexpr int STAGES = TANGENT ? 3 : 4;
   static constexpr int SOFT_WARPS = 4 * NT;
   static constexpr int WARP_MMA = SOFT_WARPS, WARP_TMA = SOFT_WARPS + 1;
   // softmax warps + one warpgroup holding the MMA warp, the TMA warp and two warps that
@@ -79,14 +70,15 @@ struct AttCfg {
   static constexpr int COL_DS = BN;
   static constexpr int COL_O = TANGENT ? 2 * BN : BN;
   static constexpr int COL_DO = COL_O + ATT_HD;    // tangent only
-  static constexpr int TILE_COLS = NT == 2 ? 256 : (NT == 3 ? 160 : 128);
+  static constexpr int TILE_COLS = TANGENT ? 256 : 128;
   static constexpr int TMEM_COLS = 512;
-  static_assert(COL_O + (TANGENT ? 2 * ATT_HD : N_PV) <= TILE_COLS && NT * TILE_COLS <= 512, "");
   static constexpr int ACC = TANGENT ? 2 * ATT_HD : ATT_HD;   // fp32 accumulators per row
+  static_assert(COL_O + ACC <= TILE_COLS && NT * TILE_COLS <= 512, "");
 };
 
-// scratch record of one half of a split item: [ITEM_M][ACC] accumulators,
-// then m, l, mu per row
+// scratch record of one part of a split item: [ACC][ITEM_M] accumulators (a column per row of the
+// record: the softmax threads own a query row each, so a warp stores 128 consecutive bytes), then
+// m, l, mu per query row
 template <bool TANGENT, int NTP>
 constexpr size_t att_part_floats() {
   return (size_t)AttCfg<TANGENT, NTP>::ITEM_M * (AttCfg<TANGENT, NTP>::ACC + 3);
@@ -96,8 +88,7 @@ template <bool TANGENT, int NTP>
 struct AttSmem {
   using C = AttCfg<TANGENT, NTP>;
   alignas(1024) uint8_t q[C::NQ][C::NT][ATT_TILE_M * 128];           // [q|dq][tile]
-  alignas(1024) uint8_t kv[C::STAGES][C::NKV][C::BN * 128];          // k, v, dk, dv
-  alignas(1024) uint8_t ones[C::ONES ? C::BN * 128 : 1024];          // bf16 1.0 panel
+  alignas(1024) uint8_t kv[C::STAGES][C::NKV][C::BN * 128];          // k, (dk,) v, (dv)
   uint64_t q_full, q_empty;
   uint64_t kv_full[C::STAGES];
   uint64_t kv_empty[C::STAGES];
@@ -113,43 +104,14 @@ struct AttParams {
   __nv_bfloat16* o;
   __nv_bfloat16* dout;     // tangent output (TANGENT only)
   float* lse;              // (B, H, L) natural-log LSE of scaled scores
-  float* scratch;          // split-item partials: [grid][2][part floats]
+  float* scratch;          // split-item partials: records of att_part_floats, two per CTA
   int B, H, L;
-  int n_qblk, n_items, n_kv;
-  long total_iters;        // n_items * n_kv
+  int n_qblk;
+  FwdShares sh;
   int64_t o_sb, o_sl, o_sh;   // output strides in elements
   float scale;
   int* status;
 };
-
-struct Segment {
-  int item, j0, j1;        // K/V tile range [j0, j1)
-  int slot, part;          // scratch slot / half when partial (slot < 0: complete item)
-};
-
-// Segment `s` of CTA `c` (its share is iterations [c*T/G, (c+1)*T/G)).
-__device__ __forceinline__ bool get_segment(const AttParams& p, int c, int G, int s, Segment& sg) {
-  const long it0 = (long)c * p.total_iters / G, it1 = (long)(c + 1) * p.total_iters / G;
-  const int first_item = (int)(it0 / p.n_kv);
-  const int item = first_item + s;
-  const long base = (long)item * p.n_kv;
-  if (base >= it1 || item >= p.n_items) return false;
-  sg.item = item;
-  sg.j0 = (int)(it0 > base ? it0 - base : 0);
-  sg.j1 = (int)(it1 < base + p.n_kv ? it1 - base : p.n_kv);
-  if (sg.j0 >= sg.j1) return false;
-  if (sg.j0 == 0 && sg.j1 == p.n_kv) {
-    sg.slot = -1;
-    sg.part = 0;
-  } else if (sg.j0 == 0) {   // head half: the item continues in CTA c + 1
-    sg.slot = c;
-    sg.part = 0;
-  } else {                   // tail half: the item started in CTA c - 1
-    sg.slot = c - 1;
-    sg.part = 1;
-  }
-  return true;
-}
 
 template <bool TANGENT, int NTP>
 __global__ void __launch_bounds__(AttCfg<TANGENT, NTP>::THREADS, 1)
@@ -181,11 +143,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     s.abort_flag = 0;
     fence_barrier_init();
   }
-  if (C::ONES) {
-    uint32_t* o32 = reinterpret_cast<uint32_t*>(s.ones);
-    for (int i = threadIdx.x; i < BN * 128 / 4; i += C::THREADS) o32[i] = 0x3f803f80u;  // bf16 1.0 x2
-    fence_proxy_async_smem();
-  }
   if (warp == C::WARP_MMA) {
     tmem_alloc(&s.tmem_base, C::TMEM_COLS);
     tmem_relinquish();
@@ -207,7 +164,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         long kv_it = 0;
         Segment sg;
         bool ok = true;
-        for (int si = 0; ok && get_segment(p, cta, G, si, sg); ++si) {
+        for (int si = 0; ok && get_segment(p.sh, cta, G, si, sg); ++si) {
           const int qb = sg.item % p.n_qblk, h = (sg.item / p.n_qblk) % p.H,
                     b = sg.item / (p.n_qblk * p.H);
           const int q0 = qb * C::ITEM_M;
@@ -228,21 +185,24 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             }
             mbar_arrive_expect_tx(&s.kv_full[st], C::NKV * BN * 128);
             tma_load_4d(s.kv[st][0], &tm_k, &s.kv_full[st], 0, h, j * BN, b);
-            tma_load_4d(s.kv[st][1], &tm_v, &s.kv_full[st], 0, h, j * BN, b);
-            if (TANGENT) {
-              tma_load_4d(s.kv[st][C::NKV - 2], &tm_dk, &s.kv_full[st], 0, h, j * BN, b);
-              tma_load_4d(s.kv[st][C::NKV - 1], &tm_dv, &s.kv_full[st], 0, h, j * BN, b);
-            }
+            if (TANGENT) tma_load_4d(s.kv[st][1], &tm_dk, &s.kv_full[st], 0, h, j * BN, b);
+            tma_load_4d(s.kv[st][C::V], &tm_v, &s.kv_full[st], 0, h, j * BN, b);
+            if (TANGENT) tma_load_4d(s.kv[st][C::NKV - 1], &tm_dv, &s.kv_full[st], 0, h, j * BN, b);
           }
         }
       }
     } else if (warp == C::WARP_MMA) {
       // ------------------------------------------------------ MMA issuer --
       if (elect_one()) {
-        constexpr uint32_t idesc_qk = idesc_bf16(ATT_TILE_M, BN, 0, 0);
-        constexpr uint32_t idesc_pv = idesc_bf16(ATT_TILE_M, C::N_PV, 0, 1);
-        constexpr uint32_t idesc_pv64 = idesc_bf16(ATT_TILE_M, ATT_HD, 0, 1);
-        const uint32_t ones_a = smem_u32(s.ones);
+        // Tangent: k | dk and v | dv lie next to one another in shared memory, and S | dS and
+        // O | dO in TMEM, so Q [K | dK]^T and P [V | dV] are one N = 128 product each.  An SM
+        // reads 128 B of operands per clock: M = N = 128 with both operands in shared memory
+        // needs 8 KB per 64 clocks, exactly that rate, where two N = 64 products need 6 KB per
+        // 32 clocks each and wait for them.
+        constexpr uint32_t idesc_qk = idesc_bf16(ATT_TILE_M, TANGENT ? 2 * BN : BN, 0, 0);
+        constexpr uint32_t idesc_dqk = idesc_bf16(ATT_TILE_M, BN, 0, 0);
+        constexpr uint32_t idesc_pv = idesc_bf16(ATT_TILE_M, C::ACC, 0, 1);
+        constexpr uint32_t idesc_tv = idesc_bf16(ATT_TILE_M, ATT_HD, 0, 1);
         auto issue_qk = [&](int t, int st, uint64_t* done) {
           const uint32_t tb = tmem + t * C::TILE_COLS;
           const uint32_t qa = smem_u32(s.q[0][t]), ka = smem_u32(s.kv[st][0]);
@@ -252,46 +212,32 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                    ks != 0);
           if (TANGENT) {
             const uint32_t dqa = smem_u32(s.q[C::NQ - 1][t]);
-            const uint32_t dka = smem_u32(s.kv[st][C::NKV - 2]);
 #pragma unroll
             for (int ks = 0; ks < ATT_HD / 16; ++ks)
               mma_ss(tb + C::COL_DS, sdesc_kmajor(dqa + ks * 32), sdesc_kmajor(ka + ks * 32),
-                     idesc_qk, ks != 0);
-#pragma unroll
-            for (int ks = 0; ks < ATT_HD / 16; ++ks)
-              mma_ss(tb + C::COL_DS, sdesc_kmajor(qa + ks * 32), sdesc_kmajor(dka + ks * 32),
-                     idesc_qk, 1);
+                     idesc_dqk, 1);
           }
           tc_commit(done);
         };
         auto issue_pv = [&](int t, int st, bool first) {
           const uint32_t tb = tmem + t * C::TILE_COLS;
-          const uint32_t va = smem_u32(s.kv[st][1]);
+          const uint32_t va = smem_u32(s.kv[st][C::V]);
 #pragma unroll
-          for (int ks = 0; ks < BN / 16; ++ks) {
-            // B = [V | ones]: panel 0 is the V tile, panel 1 (LBO away) the ones panel
-            const uint32_t vk = va + ks * 2048;
-            const uint64_t db = C::ONES ? sdesc_mnmajor(vk, (ones_a + ks * 2048) - vk)
-                                        : sdesc_mnmajor(vk, BN * 128);
-            mma_ts(tb + C::COL_O, tb + C::COL_S + ks * 8, db, idesc_pv, !(first && ks == 0));
-          }
+          for (int ks = 0; ks < BN / 16; ++ks)
+            mma_ts(tb + C::COL_O, tb + C::COL_S + ks * 8, sdesc_mnmajor(va + ks * 2048, BN * 128),
+                   idesc_pv, !(first && ks == 0));
           if (TANGENT) {
-            const uint32_t dva = smem_u32(s.kv[st][C::NKV - 1]);
 #pragma unroll
             for (int ks = 0; ks < BN / 16; ++ks)
               mma_ts(tb + C::COL_DO, tb + C::COL_DS + ks * 8,
-                     sdesc_mnmajor(va + ks * 2048, BN * 128), idesc_pv64, !(first && ks == 0));
-#pragma unroll
-            for (int ks = 0; ks < BN / 16; ++ks)
-              mma_ts(tb + C::COL_DO, tb + C::COL_S + ks * 8,
-                     sdesc_mnmajor(dva + ks * 2048, BN * 128), idesc_pv64, 1);
+                     sdesc_mnmajor(va + ks * 2048, BN * 128), idesc_tv, 1);
           }
           tc_commit(&s.o_done[t]);
         };
         long kv_it = 0, it = 0;
         Segment sg;
         bool ok = true;
-        for (int si = 0; ok && get_segment(p, cta, G, si, sg); ++si) {
+        for (int si = 0; ok && get_segment(p.sh, cta, G, si, sg); ++si) {
           const int n_j = sg.j1 - sg.j0;
           ok = mbar_wait(&s.q_full, si & 1, abort_flag, p.status, STATUS_TIMEOUT_TMA) &&
                mbar_wait(&s.kv_full[kv_it % C::STAGES], (uint32_t)((kv_it / C::STAGES) & 1),
@@ -343,7 +289,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     long it = 0;
     Segment sg;
     bool ok = true;
-    for (int si = 0; ok && get_segment(p, cta, G, si, sg); ++si) {
+    for (int si = 0; ok && get_segment(p.sh, cta, G, si, sg); ++si) {
       const int qb = sg.item % p.n_qblk, h = (sg.item / p.n_qblk) % p.H,
                 b = sg.item / (p.n_qblk * p.H);
       const int q_row = qb * C::ITEM_M + row_in_item;
@@ -353,49 +299,71 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                                                p.status, STATUS_TIMEOUT_MMA));
         if (!ok) break;
         tc_fence_after();
-        uint32_t sv[BN];
-#pragma unroll
-        for (int c = 0; c < BN; c += 32) tmem_ld32(tb + C::COL_S + c, sv + c);
-        uint32_t dsv[TANGENT ? BN : 1];
-        if (TANGENT) {
-#pragma unroll
-          for (int c = 0; c < BN; c += 32) tmem_ld32(tb + C::COL_DS + c, dsv + c);
-        }
-        tc_wait_ld();
         const int kv_rem = p.L - j * BN;
-        if (kv_rem < BN) {
+        if constexpr (TANGENT) {
+          // P = exp2(S scale - m) is computed against the reference maximum that the rows already
+          // have while the maximum of the new scores is taken alongside: the chain S -> max -> exp
+          // becomes S -> exp.  Only when a row has outgrown its reference by more than 2^8 (or has
+          // none yet) is the reference moved, O rescaled and the tile, still in TMEM, done again.
+          // (B 1, H 4, L 29,140: 2.23 -> 2.12 ms.  The primal kernel, with four warps per scheduler
+          // to fill the gaps, gets slower this way: 1.08 -> 1.31 ms.)
+          const bool first = j == sg.j0;
+          uint32_t pk[BN / 2];
+          uint32_t tk[BN / 2];
+          float alpha = 1.f;
+          f32x2 l_new, mu_new;
+          for (bool redo = false;; redo = true) {
+            const f32x2 neg_m2 = dup2(-m_used * scale_log2);
+            l_new = mu_new = dup2(0.f);
+            float mx0 = -INFINITY, mx1 = -INFINITY;
+            // 32-column chunks, the next one on its way from TMEM while one is worked on
+            uint32_t sv[2][32], dsv[2][32];
+            tmem_ld32(tb + C::COL_S, sv[0]);
+            tmem_ld32(tb + C::COL_DS, dsv[0]);
+            tc_wait_ld();
 #pragma unroll
-          for (int i = 0; i < BN; ++i)
-            if (i >= kv_rem) sv[i] = 0xff800000u;  // -inf
-        }
-        float mx0 = -INFINITY, mx1 = -INFINITY;
+            for (int c = 0; c < BN; c += 32) {
+              uint32_t* s_ = sv[(c / 32) & 1];
+              const uint32_t* d_ = dsv[(c / 32) & 1];
+              if (c + 32 < BN) {
+                tmem_ld32(tb + C::COL_S + c + 32, sv[((c / 32) & 1) ^ 1]);
+                tmem_ld32(tb + C::COL_DS + c + 32, dsv[((c / 32) & 1) ^ 1]);
+              }
+              if (kv_rem < c + 32) {
 #pragma unroll
-        for (int i = 0; i < BN; i += 4) {
-          asm("max.f32 %0, %0, %1, %2;" : "+f"(mx0) : "f"(__uint_as_float(sv[i])), "f"(__uint_as_float(sv[i + 1])));
-          asm("max.f32 %0, %0, %1, %2;" : "+f"(mx1) : "f"(__uint_as_float(sv[i + 2])), "f"(__uint_as_float(sv[i + 3])));
-        }
-        const float mx = fmaxf(mx0, mx1);
-        if (j == sg.j0) {
-          m_used = mx;
-        } else {
-          const bool need = (mx - m_used) * scale_log2 > 8.0f;
-          if (__any_sync(0xffffffffu, need)) {
-            float alpha = 1.f;
+                for (int i = 0; i < 32; ++i)
+                  if (c + i >= kv_rem) s_[i] = 0xff800000u;  // -inf
+              }
+#pragma unroll
+              for (int i = 0; i < 32; i += 2) {
+                float& mx = (i & 2) ? mx1 : mx0;
+                asm("max.f32 %0, %0, %1, %2;" : "+f"(mx) : "f"(__uint_as_float(s_[i])), "f"(__uint_as_float(s_[i + 1])));
+                const f32x2 e = fma2(pair2(s_[i], s_[i + 1]), dup2(scale_log2), neg_m2);
+                const float p0 = ex2(lo2(e)), p1 = ex2(hi2(e));
+                pk[(c + i) / 2] = pack_bf16(p0, p1);
+                const f32x2 pp = pair2(__float_as_uint(p0), __float_as_uint(p1));
+                l_new = add2(l_new, pp);
+                const f32x2 tt = mul2(mul2(pp, pair2(d_[i], d_[i + 1])), dup2(p.scale));
+                mu_new = add2(mu_new, tt);
+                tk[(c + i) / 2] = pack_bf16(lo2(tt), hi2(tt));
+              }
+              if (c + 32 < BN) tc_wait_ld();
+            }
+            if (redo) break;
+            const float mx = fmaxf(mx0, mx1);
+            const bool need = first || (mx - m_used) * scale_log2 > 8.0f;
+            if (!__any_sync(0xffffffffu, need)) break;
             if (need) {
-              alpha = ex2((m_used - mx) * scale_log2);
+              if (!first) alpha = ex2((m_used - mx) * scale_log2);
               m_used = mx;
             }
-            l_sum *= alpha;
-            l_sum2 *= alpha;
-            mu_sum *= alpha;
-            mu_sum2 *= alpha;
+            if (first) continue;               // nothing in O yet
             ok = __all_sync(0xffffffffu, mbar_wait(&s.o_done[t], (uint32_t)((it - 1) & 1),
                                                    abort_flag, p.status, STATUS_TIMEOUT_MMA));
             if (!ok) break;
             tc_fence_after();
-            constexpr int NRES = TANGENT ? 2 * ATT_HD : C::N_PV;   // 128 or 80 columns
 #pragma unroll
-            for (int c = 0; c + 32 <= NRES; c += 32) {
+            for (int c = 0; c < C::ACC; c += 32) {
               uint32_t ov[32];
               tmem_ld32(tb + C::COL_O + c, ov);
               tc_wait_ld();
@@ -403,41 +371,98 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
               tmem_st32(tb + C::COL_O + c, ov);
             }
-            if (NRES % 32) {
-              uint32_t ov[16];
-              tmem_ld16(tb + C::COL_O + (NRES / 32) * 32, ov);
-              tc_wait_ld();
-#pragma unroll
-              for (int i = 0; i < 16; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
-              tmem_st16(tb + C::COL_O + (NRES / 32) * 32, ov);
-            }
             tc_wait_st();
           }
-        }
-        const float neg_m = -m_used * scale_log2;
+          if (!ok) break;
+          l_sum = fmaf(l_sum, alpha, lo2(l_new));
+          l_sum2 = fmaf(l_sum2, alpha, hi2(l_new));
+          mu_sum = fmaf(mu_sum, alpha, lo2(mu_new));
+          mu_sum2 = fmaf(mu_sum2, alpha, hi2(mu_new));
 #pragma unroll
-        for (int c = 0; c < BN; c += 64) {
-          uint32_t pk[32];
-          uint32_t tk[TANGENT ? 32 : 1];
+          for (int c = 0; c < BN; c += 64) {
+            tmem_st32(tb + C::COL_S + c / 2, pk + c / 2);
+            tmem_st32(tb + C::COL_DS + c / 2, tk + c / 2);
+          }
+        } else {
+          // Maximum first, then the exponentials, with the scores read from TMEM again in between:
+          // 64 scores held across the vote do not fit the registers of four tiles' warps.
+          float mx0 = -INFINITY, mx1 = -INFINITY;
+          auto load = [&](int c, uint32_t* x) {
+            tmem_ld32(tb + C::COL_S + c, x);
+          };
+          auto mask = [&](int c, uint32_t* x) {
+            if (kv_rem < c + 32) {
 #pragma unroll
-          for (int i = 0; i < 64; i += 2) {
-            const float p0 = ex2(fmaf(__uint_as_float(sv[c + i]), scale_log2, neg_m));
-            const float p1 = ex2(fmaf(__uint_as_float(sv[c + i + 1]), scale_log2, neg_m));
-            pk[i / 2] = pack_bf16(p0, p1);
-            if (!C::ONES) {
-              l_sum += p0;
-              l_sum2 += p1;
+              for (int i = 0; i < 32; ++i)
+                if (c + i >= kv_rem) x[i] = 0xff800000u;  // -inf
             }
-            if (TANGENT) {
-              const float t0 = p0 * __uint_as_float(dsv[c + i]) * p.scale;
-              const float t1 = p1 * __uint_as_float(dsv[c + i + 1]) * p.scale;
-              mu_sum += t0;
-              mu_sum2 += t1;
-              tk[i / 2] = pack_bf16(t0, t1);
+          };
+          {
+            uint32_t sv[BN / 32][32];
+#pragma unroll
+            for (int c = 0; c < BN; c += 32) load(c, sv[c / 32]);
+            tc_wait_ld();
+#pragma unroll
+            for (int c = 0; c < BN; c += 32) {
+              const uint32_t* x = sv[c / 32];
+              mask(c, sv[c / 32]);
+#pragma unroll
+              for (int i = 0; i < 32; i += 4) {
+                asm("max.f32 %0, %0, %1, %2;" : "+f"(mx0) : "f"(__uint_as_float(x[i])), "f"(__uint_as_float(x[i + 1])));
+                asm("max.f32 %0, %0, %1, %2;" : "+f"(mx1) : "f"(__uint_as_float(x[i + 2])), "f"(__uint_as_float(x[i + 3])));
+              }
             }
           }
-          tmem_st32(tb + C::COL_S + c / 2, pk);
-          if (TANGENT) tmem_st32(tb + C::COL_DS + c / 2, tk);
+          const float mx = fmaxf(mx0, mx1);
+          if (j == sg.j0) {
+            m_used = mx;
+          } else {
+            const bool need = (mx - m_used) * scale_log2 > 8.0f;
+            if (__any_sync(0xffffffffu, need)) {
+              float alpha = 1.f;
+              if (need) {
+                alpha = ex2((m_used - mx) * scale_log2);
+                m_used = mx;
+              }
+              l_sum *= alpha;
+              l_sum2 *= alpha;
+              mu_sum *= alpha;
+              mu_sum2 *= alpha;
+              ok = __all_sync(0xffffffffu, mbar_wait(&s.o_done[t], (uint32_t)((it - 1) & 1),
+                                                     abort_flag, p.status, STATUS_TIMEOUT_MMA));
+              if (!ok) break;
+              tc_fence_after();
+#pragma unroll
+              for (int c = 0; c < C::ACC; c += 32) {
+                uint32_t ov[32];
+                tmem_ld32(tb + C::COL_O + c, ov);
+                tc_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
+                tmem_st32(tb + C::COL_O + c, ov);
+              }
+              tc_wait_st();
+            }
+          }
+          const f32x2 neg_m2 = dup2(-m_used * scale_log2);
+          f32x2 l2 = pair2(__float_as_uint(l_sum), __float_as_uint(l_sum2));
+#pragma unroll
+          for (int c = 0; c < BN; c += 32) {
+            uint32_t x[32], pk[16];
+            load(c, x);
+            tc_wait_ld();
+            mask(c, x);
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) {
+              const f32x2 e = fma2(pair2(x[i], x[i + 1]), dup2(scale_log2), neg_m2);
+              const float p0 = ex2(lo2(e)), p1 = ex2(hi2(e));
+              pk[i / 2] = pack_bf16(p0, p1);
+              l2 = add2(l2, pair2(__float_as_uint(p0), __float_as_uint(p1)));
+            }
+            tmem_st16(tb + C::COL_S + c / 2, pk);
+          }
+          l_sum = lo2(l2);
+          l_sum2 = hi2(l2);
         }
         tc_wait_st();
         tc_fence_before();
@@ -450,16 +475,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      float l_tot = l_sum + l_sum2;
-      const float mu_tot = mu_sum + mu_sum2;
-      if (C::ONES) {
-        uint32_t lv[8];
-        tmem_ld8(tb + C::COL_O + ATT_HD, lv);
-        tc_wait_ld();
-        l_tot = __uint_as_float(lv[0]);
-      }
+      const float l_tot = l_sum + l_sum2, mu_tot = mu_sum + mu_sum2;
       const bool live = q_row < p.L;
-      if (sg.slot < 0) {
+      if (sg.rec < 0) {
         const float inv_l = 1.f / l_tot;
         const int64_t off = (int64_t)b * p.o_sb + (int64_t)q_row * p.o_sl + (int64_t)h * p.o_sh;
 #pragma unroll
@@ -503,18 +521,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           p.lse[((int64_t)b * p.H + h) * p.L + q_row] = m_used * p.scale + __logf(l_tot);
       } else {
         // partial result of a split item: raw accumulators + (m, l, mu)
-        float* part = p.scratch + ((size_t)sg.slot * 2 + sg.part) * att_part_floats<TANGENT, NTP>();
-        float* acc = part + (size_t)row_in_item * C::ACC;
+        float* part = p.scratch + (size_t)sg.rec * att_part_floats<TANGENT, NTP>();
 #pragma unroll
         for (int c = 0; c < C::ACC; c += 32) {
           uint32_t ov[32];
           tmem_ld32(tb + C::COL_O + c, ov);
           tc_wait_ld();
-          float4* dst = reinterpret_cast<float4*>(acc + c);
+          float* acc = part + (size_t)c * C::ITEM_M + row_in_item;
 #pragma unroll
-          for (int i = 0; i < 8; ++i)
-            dst[i] = make_float4(__uint_as_float(ov[4 * i]), __uint_as_float(ov[4 * i + 1]),
-                                 __uint_as_float(ov[4 * i + 2]), __uint_as_float(ov[4 * i + 3]));
+          for (int i = 0; i < 32; ++i) acc[i * C::ITEM_M] = __uint_as_float(ov[i]);
         }
         float* stats = part + (size_t)C::ITEM_M * C::ACC;
         stats[row_in_item] = m_used;
@@ -534,56 +549,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   }
 }
 
-// Merge the two halves of every split item (one CTA per share boundary).
-constexpr int ATT_COMBINE_THREADS = 1024;
 template <bool TANGENT, int NTP>
-__global__ void __launch_bounds__(ATT_COMBINE_THREADS)
+__global__ void __launch_bounds__(32 * ATT_HD / COMBINE_COLS)
 attn_fwd_combine_kernel(const AttParams p, int G) {
-  using C = AttCfg<TANGENT, NTP>;
-  const int c = blockIdx.x;              // boundary between CTA c and c + 1
-  const long bound = (long)(c + 1) * p.total_iters / G;
-  if (bound % p.n_kv == 0) return;       // boundary falls on an item start: nothing was split
-  const int item = (int)(bound / p.n_kv);
-  if (item >= p.n_items) return;
-  const int qb = item % p.n_qblk, h = (item / p.n_qblk) % p.H, b = item / (p.n_qblk * p.H);
-  const float* pa = p.scratch + ((size_t)c * 2 + 0) * att_part_floats<TANGENT, NTP>();
-  const float* pb = p.scratch + ((size_t)c * 2 + 1) * att_part_floats<TANGENT, NTP>();
-  const float* sa = pa + (size_t)C::ITEM_M * C::ACC;
-  const float* sb = pb + (size_t)C::ITEM_M * C::ACC;
-  const float scale_log2 = p.scale * 1.4426950408889634f;
-  // one warp per row, a lane per pair of columns: 256-byte reads of the two partial rows and
-  // a 128-byte write of the merged row (a thread per row would touch a cache line per value).
-  // The CTA is alone on its SM with one item to merge, so it is as wide as a CTA gets (32
-  // warps) and the row loop is unrolled: the time goes into load latency, not into bytes.
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-#pragma unroll 4
-  for (int r = warp; r < C::ITEM_M; r += nwarps) {
-    const int q_row = qb * C::ITEM_M + r;
-    if (q_row >= p.L) continue;
-    const float ma = sa[r], mb = sb[r];
-    const float m = fmaxf(ma, mb);
-    const float wa = ex2((ma - m) * scale_log2), wb = ex2((mb - m) * scale_log2);
-    const float l = sa[C::ITEM_M + r] * wa + sb[C::ITEM_M + r] * wb;
-    const float mu = sa[2 * C::ITEM_M + r] * wa + sb[2 * C::ITEM_M + r] * wb;
-    const float inv_l = 1.f / l;
-    const float* aa = pa + (size_t)r * C::ACC;
-    const float* ab = pb + (size_t)r * C::ACC;
-    const int64_t off = (int64_t)b * p.o_sb + (int64_t)q_row * p.o_sl + (int64_t)h * p.o_sh;
-    const int col = 2 * lane;
-    const float2 xa = *reinterpret_cast<const float2*>(aa + col);
-    const float2 xb = *reinterpret_cast<const float2*>(ab + col);
-    const float o0 = (xa.x * wa + xb.x * wb) * inv_l;
-    const float o1 = (xa.y * wa + xb.y * wb) * inv_l;
-    *reinterpret_cast<uint32_t*>(p.o + off + col) = pack_bf16(o0, o1);
-    if (TANGENT) {
-      const float2 ya = *reinterpret_cast<const float2*>(aa + ATT_HD + col);
-      const float2 yb = *reinterpret_cast<const float2*>(ab + ATT_HD + col);
-      const float d0 = (ya.x * wa + yb.x * wb) * inv_l - mu * inv_l * o0;
-      const float d1 = (ya.y * wa + yb.y * wb) * inv_l - mu * inv_l * o1;
-      *reinterpret_cast<uint32_t*>(p.dout + off + col) = pack_bf16(d0, d1);
-    }
-    if (p.lse && lane == 0) p.lse[((int64_t)b * p.H + h) * p.L + q_row] = m * p.scale + __logf(l);
-  }
+  combine_split_items<ATT_HD, AttCfg<TANGENT, NTP>::ITEM_M, TANGENT>(p, G);
 }
 
 static int make_qkv_map(CUtensorMap* m, const void* ptr, int B, int L, int H, int64_t sb,
@@ -592,30 +561,6 @@ static int make_qkv_map(CUtensorMap* m, const void* ptr, int B, int L, int H, in
   uint64_t str[4] = {2, (uint64_t)sh * 2, (uint64_t)sl * 2, (uint64_t)sb * 2};
   uint32_t box[4] = {(uint32_t)ATT_HD, 1, (uint32_t)rows, 1};
   return make_tmap(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(ptr), dims, str, box);
-}
-
-// SM count of the CURRENT device (cached per device index: a host may hold GPUs of
-// different sizes, and a persistent grid larger than the device would not be co-resident).
-static int att_grid(int n_items) {
-  constexpr int MAX_DEVICES = 64;
-  static int sms_of_device[MAX_DEVICES] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  int sms = (dev >= 0 && dev < MAX_DEVICES) ? sms_of_device[dev] : 0;
-  if (!sms) {
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-      sms = 148;
-    if (dev >= 0 && dev < MAX_DEVICES) sms_of_device[dev] = sms;   // same value from every thread
-  }
-  return n_items < sms ? n_items : sms;
-}
-
-// Query tiles per work item of the primal kernel: three, unless that leaves SMs without an
-// item while two tiles per item would not (problems of about one wave).
-static int primal_nt(int B, int L, int H) {
-  const int items3 = ((L + 383) / 384) * H * B, items2 = ((L + 255) / 256) * H * B;
-  const int sms = att_grid(1 << 30);
-  return (items3 < sms && items2 > items3) ? 2 : 3;
 }
 
 template <bool TANGENT, int NTP>
@@ -627,11 +572,11 @@ static int launch_attn_fwd(const void* q, const void* k, const void* v, const vo
   int rc;
   const int B = prm.B, L = prm.L, H = prm.H;
   prm.n_qblk = (L + C::ITEM_M - 1) / C::ITEM_M;
-  prm.n_items = prm.n_qblk * H * B;
-  prm.n_kv = (L + C::BN - 1) / C::BN;
-  prm.total_iters = (long)prm.n_items * prm.n_kv;
-  const int G = att_grid(prm.n_items);
-  if (G > 1 && prm.n_items > G) {
+  prm.sh.n_items = prm.n_qblk * H * B;
+  prm.sh.n_kv = (L + C::BN - 1) / C::BN;
+  prm.sh.total = (long)prm.sh.n_items * prm.sh.n_kv;
+  const int G = fwd_grid(prm.sh.n_items, prm.sh.n_kv);
+  if (G != prm.sh.n_items) {
     if (prm.scratch == nullptr ||
         scratch_bytes < (size_t)G * 2 * att_part_floats<TANGENT, NTP>() * sizeof(float))
       return IMF_ERR_ARG;
@@ -659,11 +604,27 @@ static int launch_attn_fwd(const void* q, const void* k, const void* v, const vo
     return IMF_ERR_LAUNCH;
   kern<<<G, C::THREADS, smem, stream>>>(mq, mk, mv, mdq, mdk, mdv, prm);
   if (cudaGetLastError() != cudaSuccess) return IMF_ERR_LAUNCH;
-  if (G > 1 && prm.n_items > G) {
-    attn_fwd_combine_kernel<TANGENT, NTP><<<G - 1, ATT_COMBINE_THREADS, 0, stream>>>(prm, G);
+  if (G != prm.sh.n_items) {
+    const dim3 grid(G - 1, C::ITEM_M / COMBINE_ROWS);
+    attn_fwd_combine_kernel<TANGENT, NTP><<<grid, 32 * ATT_HD / COMBINE_COLS, 0, stream>>>(prm, G);
     if (cudaGetLastError() != cudaSuccess) return IMF_ERR_LAUNCH;
   }
   return IMF_OK;
+}
+
+template <bool TANGENT, int NTP>
+static size_t att_scratch_bytes(int B, int L, int H) {
+  using C = AttCfg<TANGENT, NTP>;
+  const long n_items = (long)((L + C::ITEM_M - 1) / C::ITEM_M) * H * B;
+  const int G = fwd_grid(n_items, (L + C::BN - 1) / C::BN);
+  return G == n_items ? 0 : (size_t)G * 2 * att_part_floats<TANGENT, NTP>() * sizeof(float);
+}
+
+// Query tiles per work item of the primal kernel: four (1.04 ms at B 1, H 4, L 29,140; three:
+// 1.16 ms), unless rounding L up to 512 rows wastes more than that gains over 384.
+static int primal_nt(int L) {
+  const int rows4 = (L + 511) / 512 * 512, rows3 = (L + 383) / 384 * 384;
+  return rows4 * 9L <= rows3 * 10L ? 4 : 3;
 }
 
 }  // namespace imf
@@ -671,14 +632,9 @@ static int launch_attn_fwd(const void* q, const void* k, const void* v, const vo
 // Bytes of scratch the forward needs for (B, L, H): 0 when no item is split.
 extern "C" long imf_attn_fwd_scratch_bytes(int B, int L, int H, int tangent) {
   using namespace imf;
-  const int nt = tangent ? 2 : primal_nt(B, L, H);
-  const int item_m = nt * ATT_TILE_M;
-  const int n_items = ((L + item_m - 1) / item_m) * H * B;
-  const int G = att_grid(n_items);
-  if (G <= 1 || n_items <= G) return 0;
-  const size_t per = tangent ? att_part_floats<true, 2>()
-                             : (nt == 3 ? att_part_floats<false, 3>() : att_part_floats<false, 2>());
-  return (long)((size_t)G * 2 * per * sizeof(float));
+  return (long)(tangent ? att_scratch_bytes<true, 2>(B, L, H)
+                        : (primal_nt(L) == 4 ? att_scratch_bytes<false, 4>(B, L, H)
+                                             : att_scratch_bytes<false, 3>(B, L, H)));
 }
 
 // Same for either head_dim (64 or 128).
@@ -726,10 +682,10 @@ extern "C" int imf_attn_fwd(const void* q, const void* k, const void* v, const v
     if (dout == nullptr || (reinterpret_cast<uintptr_t>(dout) & 15)) return IMF_ERR_ARG;
     return launch_attn_fwd<true, 2>(q, k, v, dq, dk, dv, strides, prm, (size_t)scratch_bytes, st);
   }
-  if (primal_nt(B, L, H) == 3)
-    return launch_attn_fwd<false, 3>(q, k, v, nullptr, nullptr, nullptr, strides, prm,
+  if (primal_nt(L) == 4)
+    return launch_attn_fwd<false, 4>(q, k, v, nullptr, nullptr, nullptr, strides, prm,
                                      (size_t)scratch_bytes, st);
-  return launch_attn_fwd<false, 2>(q, k, v, nullptr, nullptr, nullptr, strides, prm,
+  return launch_attn_fwd<false, 3>(q, k, v, nullptr, nullptr, nullptr, strides, prm,
                                    (size_t)scratch_bytes, st);
 }
 
@@ -740,7 +696,7 @@ extern "C" int imf_attn_fwd(const void* q, const void* k, const void* v, const v
 
 namespace imf {
 constexpr size_t NOALLOC_FLOATS =
-    (size_t)IMF_ATTN_NOALLOC_MAX_CTAS * 2 * ((size_t)AttCfg<false, 3>::ITEM_M * (ATT_HD + 3));
+    (size_t)IMF_ATTN_NOALLOC_MAX_CTAS * 2 * ((size_t)AttCfg<false, 4>::ITEM_M * (ATT_HD + 3));
 // Split-item partials of the primal forward.  In host code this name is only a
 // stand-in for the symbol, not a device address: the address comes from
 // cudaGetSymbolAddress below.
@@ -752,7 +708,7 @@ extern "C" int imf_attn_fwd_noalloc(const void* q, const void* k, const void* v,
                                     const int64_t* strides, int64_t o_sb, int64_t o_sl,
                                     int64_t o_sh, float scale, int* status, void* stream) {
   using namespace imf;
-  static_assert(NOALLOC_FLOATS == (size_t)IMF_ATTN_NOALLOC_MAX_CTAS * 2 * att_part_floats<false, 3>(),
+  static_assert(NOALLOC_FLOATS == (size_t)IMF_ATTN_NOALLOC_MAX_CTAS * 2 * att_part_floats<false, 4>(),
                 "scratch array and partial record size disagree");
   constexpr int MAX_DEVICES = 64;
   static float* scratch_of_device[MAX_DEVICES] = {nullptr};

@@ -385,6 +385,32 @@ IMF_DEVICE float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// Two fp32 values in a register pair: fma / mul / add on both with one instruction (each rounds
+// as its scalar form does).
+typedef unsigned long long f32x2;
+IMF_DEVICE f32x2 pair2(uint32_t lo, uint32_t hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+  return r;
+}
+IMF_DEVICE f32x2 dup2(float v) { return pair2(__float_as_uint(v), __float_as_uint(v)); }
+IMF_DEVICE float lo2(f32x2 v) { return __uint_as_float((uint32_t)v); }
+IMF_DEVICE float hi2(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
+IMF_DEVICE f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+IMF_DEVICE f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+IMF_DEVICE f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
 IMF_DEVICE uint32_t pack_bf16(float lo, float hi) {
   uint32_t r;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));

@@ -178,6 +178,36 @@ def test_attention_forward_tangent_hd128(K, B, L, H):
     K.check_status()
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("B,L,H,grow", [(1, 129, 1, False), (1, 532, 4, False), (1, 2049, 2, True),
+                                        (2, 1300, 3, True), (1, 7000, 10, False), (1, 513, 1, True)])
+def test_attention_forward_shares(K, hd, B, L, H, grow):
+    """Few items (each spread over several CTAs), one more than fits evenly, more items than SMs,
+    and every query-tile count of the last item.  ``grow``: the keys grow along the sequence, so
+    rows outgrow their reference maximum again and again (tile redone, accumulators rescaled) and
+    the parts of a split item have very different maxima.  P (and T) and the result are rounded to
+    bf16, 2^-9 each, and the tangent is a difference of two such sums."""
+    from imfvideo_b200.ops import reference as ref
+
+    g = torch.Generator(device="cuda").manual_seed(L + hd)
+    mk = lambda s=1.0: (torch.randn(B, L, H, hd, device="cuda", generator=g) * s).bfloat16()
+    q, k, v, dq, dk, dv = mk(), mk(), mk(), mk(.5), mk(.5), mk(.5)
+    if grow:
+        k = (k * torch.linspace(0.05, 8.0, L, device="cuda").view(1, L, 1, 1)).bfloat16()
+    ro, rdo = ref.attention_jvp(*(t.float() for t in (q, k, v, dq, dk, dv)))
+    rl = ref.attention_lse(q.float(), k.float())
+    o, _, lse = K.attn_fwd(q, k, v)
+    o2, do, lse2 = K.attn_fwd(q, k, v, dq, dk, dv)
+    for a in (o, o2):
+        assert _rel(a, ro) < 6e-3
+    assert _rel(do, rdo) < 1.2e-2
+    # the row sum is taken in fp32 before P is rounded; 1e-3 is the envelope of every LSE here
+    assert (lse - rl).abs().max() < 1e-3 and (lse2 - rl).abs().max() < 1e-3
+    again = K.attn_fwd(q, k, v, dq, dk, dv)
+    assert torch.equal(again[0], o2) and torch.equal(again[1], do) and torch.equal(again[2], lse2)
+    K.check_status()
+
+
 def test_attention_strided_views_and_run_twice(K):
     """v as a slice of a wider kv tensor (as in MLA); two runs are bit-equal."""
     torch.manual_seed(0)
