@@ -25,9 +25,10 @@
 // K (+dK) and V (+dV) travel in separate TMA rings: a K stage is free again as
 // soon as its Q K^T has run, long before the matching V stage.
 // Scheduling, split items, scratch layout and the merge kernel follow
-// attn_fwd.cu: persistent grid, equal shares of the flattened (item, K/V tile)
-// space, partial results of an item split between two CTAs merged afterwards.
+// attn_fwd.cu and attn_fwd_split.h: persistent grid, equal shares of the flattened
+// (item, K/V tile) space, partial results of split items merged afterwards.
 #include "attn_fwd128.h"
+#include "attn_fwd_split.h"
 #include "common.cuh"
 #include "host_util.h"
 
@@ -98,39 +99,12 @@ struct Params {
   float* lse;
   float* scratch;
   int B, H, L;
-  int n_qblk, n_items, n_kv;
-  long total_iters;
+  int n_qblk;
+  FwdShares sh;
   int64_t o_sb, o_sl, o_sh;
   float scale;
   int* status;
 };
-
-struct Segment {
-  int item, j0, j1;
-  int slot, part;
-};
-
-__device__ __forceinline__ bool get_segment(const Params& p, int c, int G, int s, Segment& sg) {
-  const long it0 = (long)c * p.total_iters / G, it1 = (long)(c + 1) * p.total_iters / G;
-  const int item = (int)(it0 / p.n_kv) + s;
-  const long base = (long)item * p.n_kv;
-  if (base >= it1 || item >= p.n_items) return false;
-  sg.item = item;
-  sg.j0 = (int)(it0 > base ? it0 - base : 0);
-  sg.j1 = (int)(it1 < base + p.n_kv ? it1 - base : p.n_kv);
-  if (sg.j0 >= sg.j1) return false;
-  if (sg.j0 == 0 && sg.j1 == p.n_kv) {
-    sg.slot = -1;
-    sg.part = 0;
-  } else if (sg.j0 == 0) {
-    sg.slot = c;
-    sg.part = 0;
-  } else {
-    sg.slot = c - 1;
-    sg.part = 1;
-  }
-  return true;
-}
 
 template <bool TANGENT>
 __global__ void __launch_bounds__(Cfg<TANGENT>::THREADS, 1)
@@ -188,7 +162,7 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         long kv_it = 0;
         Segment sg;
         bool ok = true;
-        for (int si = 0; ok && get_segment(p, cta, G, si, sg); ++si) {
+        for (int si = 0; ok && get_segment(p.sh, cta, G, si, sg); ++si) {
           const int qb = sg.item % p.n_qblk, h = (sg.item / p.n_qblk) % p.H,
                     b = sg.item / (p.n_qblk * p.H);
           const int q0 = qb * C::ITEM_M;
@@ -211,10 +185,9 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             }
             mbar_arrive_expect_tx(&s.k_full[st], C::NK * 2 * KPANEL);
             for (int pn = 0; pn < 2; ++pn) {
-              tma_load_4d(s.k[st][0] + pn * KPANEL, &tm_k, &s.k_full[st], pn * 64, h, j * BN, b);
-              if (TANGENT)
-                tma_load_4d(s.k[st][C::NK - 1] + pn * KPANEL, &tm_dk, &s.k_full[st], pn * 64, h,
-                            j * BN, b);
+              uint8_t* kp = s.k[st][0] + pn * C::NK * KPANEL;      // per panel: k rows, then dk rows
+              tma_load_4d(kp, &tm_k, &s.k_full[st], pn * 64, h, j * BN, b);
+              if (TANGENT) tma_load_4d(kp + KPANEL, &tm_dk, &s.k_full[st], pn * 64, h, j * BN, b);
             }
             if (kv_it >= C::STAGES) {
               ok = mbar_wait(&s.v_empty[st], par, abort_flag, p.status, STATUS_TIMEOUT_EMPTY);
@@ -233,8 +206,14 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     } else if (warp == C::WARP_MMA) {
       // -------------------------------------------------------- MMA issuer --
       if (elect_one()) {
-        constexpr uint32_t idesc_qk = idesc_bf16(TM, BN, 0, 0);
-        constexpr uint32_t idesc_pv = idesc_bf16(TM, HD, 0, 1);
+        // Tangent: Q [K | dK]^T -> S | dS and P [V | dV] -> O | dO are one product each (operands
+        // adjacent in shared memory, accumulators adjacent in TMEM).  An SM reads 128 B of
+        // operands per clock, exactly what M = N = 128 from shared memory asks for; the N = 64
+        // products, 6 KB per 32 clocks, wait for it.
+        constexpr uint32_t idesc_qk = idesc_bf16(TM, C::NK * BN, 0, 0);
+        constexpr uint32_t idesc_dqk = idesc_bf16(TM, BN, 0, 0);
+        constexpr uint32_t idesc_pv = idesc_bf16(TM, C::NK * HD, 0, 1);
+        constexpr uint32_t idesc_tv = idesc_bf16(TM, HD, 0, 1);
         // S[buf] (and dS[buf]) of tile t from K stage st
         auto issue_qk = [&](int t, int buf, int st) {
           const uint32_t tb = tmem + t * C::TILE_COLS;
@@ -242,18 +221,13 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 #pragma unroll
           for (int ks = 0; ks < HD / 16; ++ks)
             mma_ss(tb + C::col_s(buf), sdesc_kmajor(qa + (ks / 4) * QPANEL + (ks % 4) * 32),
-                   sdesc_kmajor(ka + (ks / 4) * KPANEL + (ks % 4) * 32), idesc_qk, ks != 0);
+                   sdesc_kmajor(ka + (ks / 4) * C::NK * KPANEL + (ks % 4) * 32), idesc_qk, ks != 0);
           if (TANGENT) {
             const uint32_t dqa = smem_u32(s.q[C::NQ - 1][t]);
-            const uint32_t dka = smem_u32(s.k[st][C::NK - 1]);
 #pragma unroll
             for (int ks = 0; ks < HD / 16; ++ks)
               mma_ss(tb + C::col_ds(buf), sdesc_kmajor(dqa + (ks / 4) * QPANEL + (ks % 4) * 32),
-                     sdesc_kmajor(ka + (ks / 4) * KPANEL + (ks % 4) * 32), idesc_qk, ks != 0);
-#pragma unroll
-            for (int ks = 0; ks < HD / 16; ++ks)
-              mma_ss(tb + C::col_ds(buf), sdesc_kmajor(qa + (ks / 4) * QPANEL + (ks % 4) * 32),
-                     sdesc_kmajor(dka + (ks / 4) * KPANEL + (ks % 4) * 32), idesc_qk, 1);
+                     sdesc_kmajor(ka + (ks / 4) * C::NK * KPANEL + (ks % 4) * 32), idesc_dqk, 1);
           }
           tc_commit(&s.s_full[t][buf]);
           tc_commit(&s.k_empty[st]);      // counted once per stage: see the calls
@@ -270,15 +244,10 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             mma_ts(tb + C::COL_O, tb + C::col_s(buf) + ks * 8, sdesc_mnmajor(va + ks * 2048, KPANEL),
                    idesc_pv, !(first && ks == 0));
           if (TANGENT) {
-            const uint32_t dva = smem_u32(s.v[st][C::NK - 1]);
 #pragma unroll
             for (int ks = 0; ks < BN / 16; ++ks)
               mma_ts(tb + C::COL_DO, tb + C::col_ds(buf) + ks * 8,
-                     sdesc_mnmajor(va + ks * 2048, KPANEL), idesc_pv, !(first && ks == 0));
-#pragma unroll
-            for (int ks = 0; ks < BN / 16; ++ks)
-              mma_ts(tb + C::COL_DO, tb + C::col_s(buf) + ks * 8,
-                     sdesc_mnmajor(dva + ks * 2048, KPANEL), idesc_pv, 1);
+                     sdesc_mnmajor(va + ks * 2048, KPANEL), idesc_tv, 1);
           }
           tc_commit(&s.o_done[t]);
           if (last) tc_commit(&s.o_final[t]);
@@ -286,7 +255,7 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         long kv_it = 0, it = 0;
         Segment sg;
         bool ok = true;
-        for (int si = 0; ok && get_segment(p, cta, G, si, sg); ++si) {
+        for (int si = 0; ok && get_segment(p.sh, cta, G, si, sg); ++si) {
           const int n_j = sg.j1 - sg.j0;
           ok = mbar_wait(&s.q_full, si & 1, abort_flag, p.status, STATUS_TIMEOUT_TMA) &&
                mbar_wait(&s.k_full[kv_it % C::STAGES], (uint32_t)((kv_it / C::STAGES) & 1),
@@ -395,7 +364,7 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     uint32_t xn = 0;                                // exchanges done so far (phase of xbar)
     Segment sg;
     bool ok = true;
-    for (int si = 0; ok && get_segment(p, cta, G, si, sg); ++si) {
+    for (int si = 0; ok && get_segment(p.sh, cta, G, si, sg); ++si) {
       const int qb = sg.item % p.n_qblk, h = (sg.item / p.n_qblk) % p.H,
                 b = sg.item / (p.n_qblk * p.H);
       const int q_row = qb * C::ITEM_M + row_in_item;
@@ -422,80 +391,84 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           for (int i = 0; i < NC; ++i)
             if (i >= kv_rem) sv[i] = 0xff800000u;  // -inf
         }
-        float mx0 = -INFINITY, mx1 = -INFINITY;
+        // The exponentials are taken against the reference maximum that the rows already have
+        // while the new maximum is formed alongside; only when a row has outgrown its reference
+        // by more than 2^8 (or has none yet) is the reference moved, O rescaled and the tile done
+        // again from the scores, which are still in registers.
+        const bool first = j == sg.j0;
+        uint32_t pk[NC / 2];
+        uint32_t tk[TANGENT ? NC / 2 : 1];
+        float alpha = 1.f;
+        f32x2 l_new, mu_new;
+        for (bool redo = false;; redo = true) {
+          const f32x2 neg_m2 = dup2(-m_used * scale_log2);
+          l_new = mu_new = dup2(0.f);
+          float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
-        for (int i = 0; i < NC; i += 4) {
-          asm("max.f32 %0, %0, %1, %2;" : "+f"(mx0) : "f"(__uint_as_float(sv[i])), "f"(__uint_as_float(sv[i + 1])));
-          asm("max.f32 %0, %0, %1, %2;" : "+f"(mx1) : "f"(__uint_as_float(sv[i + 2])), "f"(__uint_as_float(sv[i + 3])));
-        }
-        float mx = fmaxf(mx0, mx1);
-        if (C::SPLIT) {
-          // both column halves of a row must use the same maximum.  The exchange is also the
-          // point after which every S / dS column of this buffer has been read, so the bf16
-          // P / T written below may overlap the partner's score columns.
-          s.xmx[it & 1][half][row] = mx;
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&s.xbar);
-          ok = __all_sync(0xffffffffu, mbar_wait(&s.xbar, xn & 1, abort_flag, p.status,
-                                                 STATUS_TIMEOUT_SOFTMAX));
-          ++xn;
-          if (!ok) break;
-          mx = fmaxf(mx, s.xmx[it & 1][half ^ 1][row]);
-        }
-        if (j == sg.j0) {
-          m_used = mx;
-        } else {
-          const bool need = (mx - m_used) * scale_log2 > 8.0f;
-          if (__any_sync(0xffffffffu, need)) {
-            float alpha = 1.f;
-            if (need) {
-              alpha = ex2((m_used - mx) * scale_log2);
-              m_used = mx;
+          for (int i = 0; i < NC; i += 2) {
+            float& mxi = (i & 2) ? mx1 : mx0;
+            asm("max.f32 %0, %0, %1, %2;" : "+f"(mxi) : "f"(__uint_as_float(sv[i])), "f"(__uint_as_float(sv[i + 1])));
+            const f32x2 e = fma2(pair2(sv[i], sv[i + 1]), dup2(scale_log2), neg_m2);
+            const float p0 = ex2(lo2(e)), p1 = ex2(hi2(e));
+            const f32x2 pp = pair2(__float_as_uint(p0), __float_as_uint(p1));
+            pk[i / 2] = pack_bf16(p0, p1);
+            l_new = add2(l_new, pp);
+            if (TANGENT) {
+              const f32x2 tt = mul2(mul2(pp, pair2(dsv[i], dsv[i + 1])), dup2(p.scale));
+              mu_new = add2(mu_new, tt);
+              tk[i / 2] = pack_bf16(lo2(tt), hi2(tt));
             }
-            l_sum *= alpha;
-            l_sum2 *= alpha;
-            mu_sum *= alpha;
-            mu_sum2 *= alpha;
-            ok = __all_sync(0xffffffffu, mbar_wait(&s.o_done[t], (uint32_t)((it - 1) & 1),
-                                                   abort_flag, p.status, STATUS_TIMEOUT_MMA));
-            if (!ok) break;
-            tc_fence_after();
-            // split rows: half 0 rescales O, half 1 rescales dO
-            const uint32_t rb = tb + (C::SPLIT && half ? C::COL_DO : C::COL_O);
-#pragma unroll
-            for (int c = 0; c < HD; c += 32) {
-              uint32_t ov[32];
-              tmem_ld32(rb + c, ov);
-              tc_wait_ld();
-#pragma unroll
-              for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
-              tmem_st32(rb + c, ov);
-            }
-            tc_wait_st();
           }
+          if (redo) break;
+          float mx = fmaxf(mx0, mx1);
+          if (C::SPLIT) {
+            // both column halves of a row must use the same maximum.  The exchange is also the
+            // point after which every S / dS column of this buffer has been read, so the bf16
+            // P / T written below may overlap the partner's score columns.
+            s.xmx[it & 1][half][row] = mx;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s.xbar);
+            ok = __all_sync(0xffffffffu, mbar_wait(&s.xbar, xn & 1, abort_flag, p.status,
+                                                   STATUS_TIMEOUT_SOFTMAX));
+            ++xn;
+            if (!ok) break;
+            mx = fmaxf(mx, s.xmx[it & 1][half ^ 1][row]);
+          }
+          const bool need = first || (mx - m_used) * scale_log2 > 8.0f;
+          if (!__any_sync(0xffffffffu, need)) break;
+          if (need) {
+            if (!first) alpha = ex2((m_used - mx) * scale_log2);
+            m_used = mx;
+          }
+          if (first) continue;               // nothing in O yet
+          ok = __all_sync(0xffffffffu, mbar_wait(&s.o_done[t], (uint32_t)((it - 1) & 1),
+                                                 abort_flag, p.status, STATUS_TIMEOUT_MMA));
+          if (!ok) break;
+          tc_fence_after();
+          // split rows: half 0 rescales O, half 1 rescales dO
+          const uint32_t rb = tb + (C::SPLIT && half ? C::COL_DO : C::COL_O);
+#pragma unroll 1
+          for (int c = 0; c < HD; c += 32) {
+            uint32_t ov[32];
+            tmem_ld32(rb + c, ov);
+            tc_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
+            tmem_st32(rb + c, ov);
+          }
+          tc_wait_st();
         }
-        const float neg_m = -m_used * scale_log2;
+        if (!ok) break;
+        l_sum = fmaf(l_sum, alpha, lo2(l_new));
+        l_sum2 = fmaf(l_sum2, alpha, hi2(l_new));
+        if (TANGENT) {
+          mu_sum = fmaf(mu_sum, alpha, lo2(mu_new));
+          mu_sum2 = fmaf(mu_sum2, alpha, hi2(mu_new));
+        }
 #pragma unroll
         for (int c = 0; c < NC; c += 32) {
-          uint32_t pk[16];
-          uint32_t tk[TANGENT ? 16 : 1];
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const float p0 = ex2(fmaf(__uint_as_float(sv[c + i]), scale_log2, neg_m));
-            const float p1 = ex2(fmaf(__uint_as_float(sv[c + i + 1]), scale_log2, neg_m));
-            pk[i / 2] = pack_bf16(p0, p1);
-            l_sum += p0;
-            l_sum2 += p1;
-            if (TANGENT) {
-              const float t0 = p0 * __uint_as_float(dsv[c + i]) * p.scale;
-              const float t1 = p1 * __uint_as_float(dsv[c + i + 1]) * p.scale;
-              mu_sum += t0;
-              mu_sum2 += t1;
-              tk[i / 2] = pack_bf16(t0, t1);
-            }
-          }
-          tmem_st16(tb + C::col_s(buf) + (c0 + c) / 2, pk);
-          if (TANGENT) tmem_st16(tb + C::col_ds(buf) + (c0 + c) / 2, tk);
+          tmem_st16(tb + C::col_s(buf) + (c0 + c) / 2, pk + c / 2);
+          if (TANGENT) tmem_st16(tb + C::col_ds(buf) + (c0 + c) / 2, tk + c / 2);
         }
         tc_wait_st();
         tc_fence_before();
@@ -523,7 +496,7 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         mu_tot += s.xlm[half ^ 1][1][row];
       }
       const bool live = q_row < p.L;
-      if (sg.slot < 0) {
+      if (sg.rec < 0) {
         const float inv_l = 1.f / l_tot;
         const int64_t off = (int64_t)b * p.o_sb + (int64_t)q_row * p.o_sl + (int64_t)h * p.o_sh;
         // split rows: each half writes 64 of the 128 output columns (of o and of dout)
@@ -567,20 +540,18 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         if (live && p.lse && half == 0)
           p.lse[((int64_t)b * p.H + h) * p.L + q_row] = m_used * p.scale + __logf(l_tot);
       } else {
-        // partial result of a split item: raw accumulators + (m, l, mu); with split rows half 0
-        // stores the O accumulators (columns 0-127), half 1 the dO accumulators (128-255)
-        float* part = p.scratch + ((size_t)sg.slot * 2 + sg.part) * part_floats<TANGENT>();
-        float* acc = part + (size_t)row_in_item * C::ACC + (C::SPLIT ? half * HD : 0);
+        // partial result of a split item: raw accumulators, [column][row] so that a warp stores
+        // 128 consecutive bytes, + (m, l, mu); with split rows half 0 stores the O accumulators
+        // (columns 0-127), half 1 the dO accumulators (128-255)
+        float* part = p.scratch + (size_t)sg.rec * part_floats<TANGENT>();
         const uint32_t rb = tb + (C::SPLIT && half ? C::COL_DO : C::COL_O);
         for (int c = 0; c < HD; c += 32) {
           uint32_t ov[32];
           tmem_ld32(rb + c, ov);
           tc_wait_ld();
-          float4* dst = reinterpret_cast<float4*>(acc + c);
+          float* acc = part + (size_t)(c + (C::SPLIT ? half * HD : 0)) * C::ITEM_M + row_in_item;
 #pragma unroll
-          for (int i = 0; i < 8; ++i)
-            dst[i] = make_float4(__uint_as_float(ov[4 * i]), __uint_as_float(ov[4 * i + 1]),
-                                 __uint_as_float(ov[4 * i + 2]), __uint_as_float(ov[4 * i + 3]));
+          for (int i = 0; i < 32; ++i) acc[i * C::ITEM_M] = __uint_as_float(ov[i]);
         }
         if (half == 0) {
           float* stats = part + (size_t)C::ITEM_M * C::ACC;
@@ -602,45 +573,10 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   }
 }
 
-// Merge the two halves of every split item (one CTA per share boundary).
 template <bool TANGENT>
-__global__ void __launch_bounds__(Cfg<TANGENT>::ITEM_M)
+__global__ void __launch_bounds__(32 * HD / COMBINE_COLS)
 attn_fwd128_combine_kernel(const Params p, int G) {
-  using C = Cfg<TANGENT>;
-  const int c = blockIdx.x;
-  const long bound = (long)(c + 1) * p.total_iters / G;
-  if (bound % p.n_kv == 0) return;
-  const int item = (int)(bound / p.n_kv);
-  if (item >= p.n_items) return;
-  const int qb = item % p.n_qblk, h = (item / p.n_qblk) % p.H, b = item / (p.n_qblk * p.H);
-  const int r = threadIdx.x;
-  const int q_row = qb * C::ITEM_M + r;
-  if (q_row >= p.L) return;
-  const float* pa = p.scratch + ((size_t)c * 2 + 0) * part_floats<TANGENT>();
-  const float* pb = p.scratch + ((size_t)c * 2 + 1) * part_floats<TANGENT>();
-  const float* sa = pa + (size_t)C::ITEM_M * C::ACC;
-  const float* sb = pb + (size_t)C::ITEM_M * C::ACC;
-  const float ma = sa[r], mb = sb[r];
-  const float m = fmaxf(ma, mb);
-  const float scale_log2 = p.scale * 1.4426950408889634f;
-  const float wa = ex2((ma - m) * scale_log2), wb = ex2((mb - m) * scale_log2);
-  const float l = sa[C::ITEM_M + r] * wa + sb[C::ITEM_M + r] * wb;
-  const float mu = sa[2 * C::ITEM_M + r] * wa + sb[2 * C::ITEM_M + r] * wb;
-  const float inv_l = 1.f / l;
-  const float* aa = pa + (size_t)r * C::ACC;
-  const float* ab = pb + (size_t)r * C::ACC;
-  const int64_t off = (int64_t)b * p.o_sb + (int64_t)q_row * p.o_sl + (int64_t)h * p.o_sh;
-  for (int col = 0; col < HD; col += 2) {
-    const float o0 = (aa[col] * wa + ab[col] * wb) * inv_l;
-    const float o1 = (aa[col + 1] * wa + ab[col + 1] * wb) * inv_l;
-    *reinterpret_cast<uint32_t*>(p.o + off + col) = pack_bf16(o0, o1);
-    if (TANGENT) {
-      const float d0 = (aa[HD + col] * wa + ab[HD + col] * wb) * inv_l - mu * inv_l * o0;
-      const float d1 = (aa[HD + col + 1] * wa + ab[HD + col + 1] * wb) * inv_l - mu * inv_l * o1;
-      *reinterpret_cast<uint32_t*>(p.dout + off + col) = pack_bf16(d0, d1);
-    }
-  }
-  if (p.lse) p.lse[((int64_t)b * p.H + h) * p.L + q_row] = m * p.scale + __logf(l);
+  combine_split_items<HD, Cfg<TANGENT>::ITEM_M, TANGENT>(p, G);
 }
 
 // 4-D map over a (B, L, H, 128) bf16 tensor whose box is one 64-column panel of `rows` rows
@@ -650,20 +586,6 @@ static int make_map(CUtensorMap* m, const void* ptr, int B, int L, int H, int64_
   uint64_t str[4] = {2, (uint64_t)sh * 2, (uint64_t)sl * 2, (uint64_t)sb * 2};
   uint32_t box[4] = {64, 1, (uint32_t)rows, 1};
   return make_tmap(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(ptr), dims, str, box);
-}
-
-static int grid_for(int n_items) {
-  constexpr int MAX_DEVICES = 64;
-  static int sms_of_device[MAX_DEVICES] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  int sms = (dev >= 0 && dev < MAX_DEVICES) ? sms_of_device[dev] : 0;
-  if (!sms) {
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-      sms = 148;
-    if (dev >= 0 && dev < MAX_DEVICES) sms_of_device[dev] = sms;
-  }
-  return n_items < sms ? n_items : sms;
 }
 
 template <bool TANGENT>
@@ -679,11 +601,11 @@ static int launch(const Fwd128Args& a) {
   prm.scale = a.scale;
   prm.status = a.status;
   prm.n_qblk = (a.L + C::ITEM_M - 1) / C::ITEM_M;
-  prm.n_items = prm.n_qblk * a.H * a.B;
-  prm.n_kv = (a.L + BN - 1) / BN;
-  prm.total_iters = (long)prm.n_items * prm.n_kv;
-  const int G = grid_for(prm.n_items);
-  if (G > 1 && prm.n_items > G) {
+  prm.sh.n_items = prm.n_qblk * a.H * a.B;
+  prm.sh.n_kv = (a.L + BN - 1) / BN;
+  prm.sh.total = (long)prm.sh.n_items * prm.sh.n_kv;
+  const int G = fwd_grid(prm.sh.n_items, prm.sh.n_kv);
+  if (G != prm.sh.n_items) {
     if (prm.scratch == nullptr ||
         (size_t)a.scratch_bytes < (size_t)G * 2 * part_floats<TANGENT>() * sizeof(float))
       return IMF_ERR_ARG;
@@ -711,8 +633,9 @@ static int launch(const Fwd128Args& a) {
   cudaStream_t stream = static_cast<cudaStream_t>(a.stream);
   kern<<<G, C::THREADS, smem, stream>>>(mq, mk, mv, mdq, mdk, mdv, prm);
   if (cudaGetLastError() != cudaSuccess) return IMF_ERR_LAUNCH;
-  if (G > 1 && prm.n_items > G) {
-    attn_fwd128_combine_kernel<TANGENT><<<G - 1, C::ITEM_M, 0, stream>>>(prm, G);
+  if (G != prm.sh.n_items) {
+    const dim3 grid(G - 1, C::ITEM_M / COMBINE_ROWS);
+    attn_fwd128_combine_kernel<TANGENT><<<grid, 32 * HD / COMBINE_COLS, 0, stream>>>(prm, G);
     if (cudaGetLastError() != cudaSuccess) return IMF_ERR_LAUNCH;
   }
   return IMF_OK;
@@ -722,9 +645,9 @@ static int launch(const Fwd128Args& a) {
 
 long attn_fwd128_scratch_bytes(int B, int L, int H, int tangent) {
   const int item_m = tangent ? a128::Cfg<true>::ITEM_M : a128::Cfg<false>::ITEM_M;
-  const int n_items = ((L + item_m - 1) / item_m) * H * B;
-  const int G = a128::grid_for(n_items);
-  if (G <= 1 || n_items <= G) return 0;
+  const long n_items = (long)((L + item_m - 1) / item_m) * H * B;
+  const int G = fwd_grid(n_items, (L + a128::BN - 1) / a128::BN);
+  if (G == n_items) return 0;
   const size_t per = tangent ? a128::part_floats<true>() : a128::part_floats<false>();
   return (long)((size_t)G * 2 * per * sizeof(float));
 }
