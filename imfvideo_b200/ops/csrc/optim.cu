@@ -247,12 +247,30 @@ constexpr int NS_CHUNKS = 32;
 __global__ void __launch_bounds__(256)
 ns_sumsq_kernel(const float* __restrict__ g, long numel, double* __restrict__ part) {
   const float* src = g + (long)blockIdx.y * numel;
-  const long per = (numel + NS_CHUNKS - 1) / NS_CHUNKS;
-  const long lo = blockIdx.x * per, hi = lo + per < numel ? lo + per : numel;
+  const long per = ((numel + NS_CHUNKS - 1) / NS_CHUNKS + 3) / 4 * 4;
+  const long lo = blockIdx.x * per < numel ? blockIdx.x * per : numel;
+  const long hi = lo + per < numel ? lo + per : numel;
   double ss = 0.0;
-  for (long i = lo + threadIdx.x; i < hi; i += 256) {
-    const float v = src[i];
-    ss += (double)v * v;
+  if (numel % 4 == 0 && (reinterpret_cast<uintptr_t>(g) & 15) == 0) {
+    // four values per load, two loads in flight; `per` is a multiple of four then
+    const float4* s4 = reinterpret_cast<const float4*>(src);
+    double s1 = 0.0;
+    long i = lo / 4 + threadIdx.x;
+    auto sq = [](const float4& v) {
+      return ((double)v.x * v.x + (double)v.y * v.y) + ((double)v.z * v.z + (double)v.w * v.w);
+    };
+    for (; i + 256 < hi / 4; i += 512) {
+      const float4 u = s4[i], v = s4[i + 256];
+      ss += sq(u);
+      s1 += sq(v);
+    }
+    if (i < hi / 4) ss += sq(s4[i]);
+    ss += s1;
+  } else {
+    for (long i = lo + threadIdx.x; i < hi; i += 256) {
+      const float v = src[i];
+      ss += (double)v * v;
+    }
   }
   __shared__ double s_part[8];
 #pragma unroll
@@ -276,6 +294,20 @@ ns_scale_kernel(const float* __restrict__ g, __nv_bfloat16* __restrict__ x, int 
   const float* src = g + (long)z * n * m;
   __nv_bfloat16* dst = x + (long)z * n * mp;
   const long total = (long)n * mp;
+  if (m == mp && (reinterpret_cast<uintptr_t>(g) & 15) == 0) {   // mp is a multiple of eight
+    // nothing to pad: 32 bytes in, 16 bytes out per thread, no division (24 x 1,024 x 1,024:
+    // 71 us with a value per thread and its row and column by 64-bit division)
+    for (long i = (long)blockIdx.x * 256 + threadIdx.x; i < total / 8; i += (long)gridDim.x * 256) {
+      const float4 a = reinterpret_cast<const float4*>(src)[2 * i];
+      const float4 b = reinterpret_cast<const float4*>(src)[2 * i + 1];
+      auto pk = [&](float lo, float hi) {
+        return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(lo * inv)) |
+               (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(hi * inv)) << 16;
+      };
+      reinterpret_cast<uint4*>(dst)[i] = make_uint4(pk(a.x, a.y), pk(a.z, a.w), pk(b.x, b.y), pk(b.z, b.w));
+    }
+    return;
+  }
   for (long i = (long)blockIdx.x * 256 + threadIdx.x; i < total; i += (long)gridDim.x * 256) {
     const int r = (int)(i / mp), c = (int)(i % mp);
     dst[i] = __float2bfloat16_rn(c < m ? src[(long)r * m + c] * inv : 0.f);

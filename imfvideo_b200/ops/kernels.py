@@ -570,6 +570,8 @@ def newton_schulz(G: torch.Tensor, coeffs, steps: int = 5, eps: float = 1e-7,
         nrm = Gf.flatten(1).norm(dim=1).view(k, 1, 1) + eps
         X.zero_()
         X[:, :, :m] = (Gf / nrm).to(torch.bfloat16)
+    if out is None and mp == m:
+        out = torch.empty(k, n, m, dtype=torch.bfloat16, device=G.device)   # not a workspace view
     if mp != m:
         Y.zero_()        # the pad columns of the other iterate stay zero through a X + B X
     direct = (out is not None and mp == m and out.dtype == torch.bfloat16 and out.is_contiguous()
