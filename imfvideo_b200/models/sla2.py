@@ -564,9 +564,8 @@ class SparseCore:
                 _, _, qq = SP.quantize_blocks(K._tma_ok(q), self.qblk, want_q=False, want_fq=True)
                 _, _, kk = SP.quantize_blocks(K._tma_ok(k), 64, want_q=False, want_fq=True)
                 _, _, vv = SP.quantize_blocks(K._tma_ok(v), 64, want_q=False, want_fq=True)
-            qlist, qflags, qrank = SP.kv_lists(flags, want_rank=True)   # `flags`: the maps (see fwd)
-            gq_s, gk_s, gv_s = K.attn_bwd(qq, kk, vv, o_s, lse, g_os, qlist=qlist, qflags=qflags,
-                                          qrank=qrank)
+            gq_s, gk_s, gv_s = K.attn_bwd(qq, kk, vv, o_s, lse, g_os,
+                                          **SP.bwd_lists(flags))   # `flags`: the maps (see fwd)
             back = lambda t: t.permute(0, 2, 1, 3)
             gq = (gq_s.float() + back(gq_l)).to(q.dtype)
             gk = (gk_s.float() + back(gk_l)).to(q.dtype)
@@ -606,10 +605,9 @@ def _sparse_core_bwd_kernels(self, q, k, v, saved, go, gv_out, alpha_param, cube
             _, _, qq = SP.quantize_blocks(K._tma_ok(q), self.qblk, want_q=False, want_fq=True)
             _, _, kk = SP.quantize_blocks(K._tma_ok(k), 64, want_q=False, want_fq=True)
             _, _, vv = SP.quantize_blocks(K._tma_ok(v), 64, want_q=False, want_fq=True)
-        qlist, qflags, qrank = SP.kv_lists(flags, want_rank=True)       # `flags`: the maps (see fwd)
         # the linear branch's query gradient rides into the block-sparse backward's dQ epilogue
-        gq, gk_s, gv_s = K.attn_bwd(qq, kk, vv, o_s, lse, g_os, qlist=qlist, qflags=qflags,
-                                    qrank=qrank, dq_add=gq_l)
+        gq, gk_s, gv_s = K.attn_bwd(qq, kk, vv, o_s, lse, g_os, dq_add=gq_l,
+                                    **SP.bwd_lists(flags))         # `flags`: the maps (see fwd)
         gk, gv = LA.backward_kv(q, k, v, gnum, gden, sel, gk_s, gv_s, self.qblk, self.bk,
                                 self.n_comp, gv_out=gv_out)
     return gq, gk, gv

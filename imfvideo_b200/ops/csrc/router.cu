@@ -161,6 +161,52 @@ kv_lists_kernel(const uint8_t* __restrict__ fm, const uint16_t* __restrict__ rk,
   }
 }
 
+// fm: (B, H, n_kvt, n_mt) nibbles -> qlist / qflags (B, H, n_kvt, n_mt), -1 terminated: the live
+// 64-row query blocks of a K/V tile in ascending order, two to an entry (ids in the low and high
+// 16 bits; an odd last one is paired with block 2 n_mt, past the end).  Flag bits as in
+// kv_lists_kernel: kv half * 2 + place in the entry.
+__global__ void __launch_bounds__(RT_THREADS)
+kv_pair_lists_kernel(const uint8_t* __restrict__ fm, int* __restrict__ qlist,
+                     uint8_t* __restrict__ qflags, int n_mt) {
+  extern __shared__ uint16_t s_ids[];                            // [2 n_mt] ids, then [2 n_mt] bytes
+  uint8_t* s_fl = reinterpret_cast<uint8_t*>(s_ids + 2 * n_mt);  // bit = kv half
+  const size_t rowi = ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  const uint8_t* row = fm + rowi * n_mt;
+  const int tid = threadIdx.x;
+  const int per = (n_mt + RT_THREADS - 1) / RT_THREADS;
+  const int lo = min(n_mt, tid * per), hi = min(n_mt, lo + per);
+  int n = 0;
+  for (int i = lo; i < hi; ++i) {
+    const int f = row[i];
+    n += ((f & 5) != 0) + ((f & 10) != 0);
+  }
+  int total;
+  int pos = block_excl_scan(n, &total);
+  for (int i = lo; i < hi; ++i) {
+    const int f = row[i];
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int kv = ((f >> half) & 1) | (((f >> (2 + half)) & 1) << 1);
+      if (kv) {
+        s_ids[pos] = (uint16_t)(2 * i + half);
+        s_fl[pos++] = (uint8_t)kv;
+      }
+    }
+  }
+  __syncthreads();
+  for (int j = tid; j < n_mt; j += RT_THREADS) {
+    int e = -1, f = 0;
+    if (2 * j < total) {
+      const bool two = 2 * j + 1 < total;
+      const int fa = s_fl[2 * j], fb = two ? s_fl[2 * j + 1] : 0;
+      e = (int)s_ids[2 * j] | (two ? (int)s_ids[2 * j + 1] : 2 * n_mt) << 16;
+      f = (fa & 1) | (fb & 1) << 1 | (fa & 2) << 1 | (fb & 2) << 2;
+    }
+    qlist[rowi * n_mt + j] = e;
+    qflags[rowi * n_mt + j] = (uint8_t)f;
+  }
+}
+
 // --------------------------------------------------------------------------
 // Block means: x (B, L, H, 64) bf16 with element strides (sb, sl, sh) ->
 // out (B, H, nb, 64) fp32, mean over the valid rows of each block.  Fixed
@@ -410,5 +456,15 @@ extern "C" int imf_build_kv_lists(const uint8_t* fm, const uint16_t* rk, int* ql
   if ((rk == nullptr) != (qrank == nullptr)) return -1;
   kv_lists_kernel<<<dim3(n_kvt, H, B), RT_THREADS, 0, (cudaStream_t)stream>>>(
       fm, rk, qlist, qflags, qrank, n_mt, qmax);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+// Block ids are 16 bits with the sign bit of an entry left alone, and the staging fits 48 KB.
+extern "C" int imf_build_kv_pair_lists(const uint8_t* fm, int* qlist, uint8_t* qflags, int B, int H,
+                                       int n_kvt, int n_mt, void* stream) {
+  if (B <= 0 || H <= 0 || n_kvt <= 0 || n_mt <= 0) return -1;
+  if (n_mt > 8192) return -4;
+  kv_pair_lists_kernel<<<dim3(n_kvt, H, B), RT_THREADS, 6 * n_mt, (cudaStream_t)stream>>>(
+      fm, qlist, qflags, n_mt);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }

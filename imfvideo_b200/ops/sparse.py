@@ -33,6 +33,8 @@ if K._has("imf_build_tile_lut"):
     _lib.imf_build_tile_lut.argtypes = [vp] * 6 + [ci] * 7 + [vp]
     _lib.imf_build_kv_lists.restype = ci
     _lib.imf_build_kv_lists.argtypes = [vp] * 5 + [ci] * 5 + [vp]
+    _lib.imf_build_kv_pair_lists.restype = ci
+    _lib.imf_build_kv_pair_lists.argtypes = [vp] * 3 + [ci] * 4 + [vp]
 
 
 ROUTER_KERNELS = K._has("imf_route_topk")
@@ -124,6 +126,33 @@ def kv_lists(maps: torch.Tensor, want_rank: bool = False):
                                      n_mt, n_mt, K._stream()), "imf_build_kv_lists")
     K.LAUNCHES.count += 1
     return (qlist, qflags, qrank) if want_rank else (qlist, qflags)
+
+
+def kv_pair_lists(maps: torch.Tensor):
+    """Inverted lists in steps of two live 64-row query blocks, for ``kernels.attn_bwd(...,
+    qpairs=True)``, from the maps of ``route_tables`` (or a bare (B, H, n_kvt, n_mt) nibble
+    matrix): (qlist int32 (B,H,n_kvt,n_mt) with the two block ids in its low and high 16 bits,
+    padded with -1, qflags uint8).  Routing selects 64-row blocks, so most 128-row query tiles of
+    ``kv_lists`` attend a K/V tile with one half only; here every step but a list's last is full."""
+    fm = maps[2] if maps.dim() == 5 else maps
+    B, H, n_kvt, n_mt = fm.shape
+    qlist = torch.empty(B, H, n_kvt, n_mt, dtype=torch.int32, device=fm.device)
+    qflags = torch.empty(B, H, n_kvt, n_mt, dtype=torch.uint8, device=fm.device)
+    K._check(_lib.imf_build_kv_pair_lists(K._ptr(fm), K._ptr(qlist), K._ptr(qflags), B, H, n_kvt,
+                                          n_mt, K._stream()), "imf_build_kv_pair_lists")
+    K.LAUNCHES.count += 1
+    return qlist, qflags
+
+
+def bwd_lists(maps: torch.Tensor):
+    """Arguments of ``kernels.attn_bwd`` that describe the routing: block pairs, or whole query
+    tiles with their ranks where the order of dQ additions is fixed (it is kept per tile) or the
+    block ids do not fit an entry."""
+    if K.DETERMINISTIC or maps.shape[-1] > 8192:
+        qlist, qflags, qrank = kv_lists(maps, want_rank=True)
+        return dict(qlist=qlist, qflags=qflags, qrank=qrank)
+    qlist, qflags = kv_pair_lists(maps)
+    return dict(qlist=qlist, qflags=qflags, qpairs=True)
 
 
 def quantize_blocks(x: torch.Tensor, block: int, want_q: bool = True, want_fq: bool = False):

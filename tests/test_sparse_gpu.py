@@ -188,6 +188,46 @@ def test_sparse_backward_kernel(SP, qblk, L):
     kernels.check_status()
 
 
+@pytest.mark.parametrize("qblk,L,T", [(64, 583, 3), (64, 64, 1), (64, 130, 2), (128, 640, 3), (64, 4300, 20)])
+def test_sparse_backward_block_pairs(SP, qblk, L, T):
+    """Lists of block pairs: exactly the live (K/V tile, 64-row query block) pairs in ascending
+    order, two to an entry, an odd last one beside the block past the end; the backward on them
+    equals the one on whole query tiles but for the order of fp32 sums and of dQ additions
+    (results are rounded to bf16: 2^-9).  The last case has steps of two distant blocks."""
+    from imfvideo_b200.ops import kernels
+
+    torch.manual_seed(L)
+    B, H = 2, 3
+    mk = lambda: torch.randn(B, L, H, 64, device="cuda").bfloat16()
+    q, k, v, go = mk(), mk(), mk(), mk()
+    Mb, Nb = -(-L // qblk), -(-L // 64)
+    sel = torch.rand(B, H, Mb, Nb, device="cuda").argsort(-1)[..., :T].int()
+    lut, flags, cnt, maps = SP.route_tables(sel, qblk, L)
+    fm = maps[2].cpu()
+    ql, qf = (t.cpu() for t in SP.kv_pair_lists(maps))
+    n_mt = fm.shape[-1]
+    for b, h, t in [(0, 0, 0), (B - 1, H - 1, fm.shape[2] - 1), (1, 1, fm.shape[2] // 2)]:
+        want = [(2 * i + half, (int(f) >> half) & 5) for i, f in enumerate(fm[b, h, t])
+                for half in range(2) if (int(f) >> half) & 5]
+        got = []
+        n = int((ql[b, h, t] >= 0).sum())
+        assert n == -(-len(want) // 2) and bool((ql[b, h, t, n:] < 0).all())
+        for e, f in zip(ql[b, h, t, :n].tolist(), qf[b, h, t, :n].tolist()):
+            got += [(e & 0xffff, f & 5), (e >> 16, (f >> 1) & 5)]
+        if len(want) % 2:
+            assert got.pop() == (2 * n_mt, 0)
+        assert got == want
+    o, _, lse = SP.sparse_fwd(q, k, v, None, None, None, lut, flags, qblk, False, quant_p=False,
+                              cnt=cnt)
+    tl, tf = SP.kv_lists(maps)
+    tiles = kernels.attn_bwd(q, k, v, o, lse, go, qlist=tl, qflags=tf)
+    pl, pf = SP.kv_pair_lists(maps)
+    pairs = kernels.attn_bwd(q, k, v, o, lse, go, qlist=pl, qflags=pf, qpairs=True)
+    for a, b in zip(pairs, tiles):
+        assert _rel(a, b) < 2e-3
+    kernels.check_status()
+
+
 def test_sparse_backward_bitwise_repeatable(SP):
     from imfvideo_b200.ops import kernels
     """Block-sparse backward with the device-built lists and ranks: dQ bit-identical from run
