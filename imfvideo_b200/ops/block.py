@@ -5,7 +5,8 @@ the primal rows, so every GEMM is one launch over 2*b*l rows); backward is the
 hand-scheduled reverse pass through the primal only.  Per block the forward is
 11 fused launches + attention, instead of ~120 framework kernels; this is the
 production path on CUDA, the generic ``ops.dual`` composition stays as the CPU
-path and oracle.
+path and oracle.  The launches before and after the attention core are issued by
+native code (``csrc/block_forward.cu``), one call each.
 
 Block structure (reference ``models/imf_dit_video.py:909-972``, ``:422-467``):
     n1  = norm1(remix(prefix, snaps; w1))
@@ -18,12 +19,21 @@ Block structure (reference ``models/imf_dit_video.py:909-972``, ``:422-467``):
 
 from __future__ import annotations
 
+import ctypes
 from typing import List, Optional, Sequence, Tuple
 
 import torch
 
 from . import kernels as K
 from . import rowops as R
+
+_lib, c_int = K._lib, ctypes.c_int
+if K._has("imf_block_pre"):
+    _lib.imf_block_pre.restype = c_int
+    _lib.imf_block_pre.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_float, ctypes.c_void_p]
+    _lib.imf_block_post.restype = c_int
+    _lib.imf_block_post.argtypes = [ctypes.c_void_p, ctypes.c_void_p] + [ctypes.c_float] * 3 + \
+        [ctypes.c_void_p]
 
 BF16, F32 = torch.bfloat16, torch.float32
 
@@ -142,67 +152,54 @@ class _BlockFn(torch.autograd.Function):
         dsn = [flat(s) if has_t else None for s in dsnaps] if has_t else [None] * nsnap
         new = lambda *shape, dt=BF16: torch.empty(*shape, dtype=dt, device=dev)
 
-        # 1. remix + norm1
-        n1 = new(T, rows, d)
-        R.resnorm_fwd(pfx, dpfx, None, None, None, sn, dsn, w1 if (use_res and nsnap) else None,
-                      g_n1, eps, n1[0], n1[1] if has_t else None, None, None)
-        # 2. fused projection GEMM over primal+tangent rows
-        a_ = K.gemm(n1.view(T * rows, d), W_a)                       # [T*rows, na]
-        na = g.na
-        # 3. latent norms
+        W_a, W_qb, W_kvb, W_out, W13, W2 = mats = tuple(
+            w if w.stride(1) == 1 else w.contiguous() for w in (W_a, W_qb, W_kvb, W_out, W13, W2))
+        na, hv = g.na, g.H * g.dv
+        nq, nkv = g.H * g.hd, g.H * (g.dn + g.dv)
+        assert [tuple(w.shape) for w in mats] == [(na, d), (nq, g.dq), (nkv, g.dc), (d, hv),
+                                                  (2 * g.fp, d), (d, g.fp)]
+        assert all(w.dtype == BF16 for w in mats)
+        ptr, stream, status = R._p, K._stream(), K.status_word(dev).data_ptr()
+        sn2, dsn2 = (sn + [pfx], dsn + [dpfx]) if fresh else (sn, dsn)
+
+        def dims(ns):
+            return (c_int * 21)(rows, L, d, T, g.H, g.dq, g.dc, g.dn, g.dr, g.dv, na, g.fp, ns, int(g.gate),
+                                int(lbeta is not None), *[w.stride(0) for w in mats])
+        # 1.-5. remix + norm1, fused projection GEMM over primal + tangent rows, latent norms,
+        # up-projections, q / k preparation
+        n1, a_ = new(T, rows, d), new(T * rows, na)
         qlat, kvlat = new(T, rows, g.dq), new(T, rows, g.dc)
-        a0, a1 = a_[:rows], (a_[rows:] if has_t else None)
-        R.rmsnorm_seg_fwd(
-            [(a0, a1, g_qa, qlat[0], qlat[1] if has_t else None, g.dq, na, g.dq),
-             (a0[:, g.dq:], None if a1 is None else a1[:, g.dq:], g_kva, kvlat[0],
-              kvlat[1] if has_t else None, g.dc, na, g.dc)], rows, eps, has_t)
-        # 4. up-projections
-        qb = K.gemm(qlat.view(T * rows, g.dq), W_qb)                 # [T*rows, H*hd]
-        kvb = K.gemm(kvlat.view(T * rows, g.dc), W_kvb)              # [T*rows, H*(dn+dv)]
-        # 5. q / k preparation
+        qb, kvb = new(T * rows, nq), new(T * rows, nkv)
         q, k = new(T, B, L, g.H, g.hd), new(T, B, L, g.H, g.hd)
-        kr0 = a0[:, g.dq + g.dc:]
-        kr1 = None if a1 is None else a1[:, g.dq + g.dc:]
-        R.qkprep_fwd(qb[:rows], qb[rows:] if has_t else None, kvb[:rows],
-                     kvb[rows:] if has_t else None, kr0, kr1, cos, sin, g_qn, g_kn,
-                     q[0], q[1] if has_t else None, k[0], k[1] if has_t else None,
-                     rows, L, g.H, g.dn, g.dr, g.dv, na, eps)
+        ptrs = [ptr(pfx), ptr(dpfx), ptr(w1) if (use_res and nsnap) else 0, ptr(g_n1), ptr(W_a), ptr(g_qa),
+                ptr(g_kva), ptr(W_qb), ptr(W_kvb), ptr(cos), ptr(sin), ptr(g_qn), ptr(g_kn), ptr(n1),
+                ptr(a_), ptr(qlat), ptr(kvlat), ptr(qb), ptr(kvb), ptr(q), ptr(k), status]
+        ptrs += [ptr(s) for s in sn] + [ptr(s) for s in dsn]
+        K._check(_lib.imf_block_pre(R._ptr_array(ptrs), dims(nsnap), float(eps), stream), "imf_block_pre")
+        K.LAUNCHES.count += 6
         kv4 = kvb.view(T, B, L, g.H, g.dn + g.dv)
         v0 = kv4[0][..., g.dn:]
         v1 = kv4[1][..., g.dn:] if has_t else None
         # 6. attention core
         o, do, core_saved = core.fwd(q[0], k[0], v0, q[1] if has_t else None,
                                      k[1] if has_t else None, v1, need_bwd)
-        hv = g.H * g.dv
-        # 7. output gate
+        # 7.-11. output gate, output projection, residual + remix + norm2, MLP, residual
         if g.gate:
             og = new(T, rows, hv)
-            gcol = g.dq + g.dc + g.dr
-            R.outgate_fwd(o.view(rows, hv), None if do is None else do.view(rows, hv),
-                          a0[:, gcol:], None if a1 is None else a1[:, gcol:], og[0],
-                          og[1] if has_t else None, rows, hv, hv, na)
         else:
             og = torch.stack([o.view(rows, hv), do.view(rows, hv)]) if has_t else o.view(1, rows, hv)
-        # 8. output projection
-        a_out = K.gemm(og.view(T * rows, hv), W_out)                 # [T*rows, d]
-        # 9. residual + remix + norm2
+        a_out, m = new(T * rows, d), new(T * rows, d)
         p2, n2 = new(T, rows, d, dt=F32), new(T, rows, d)
-        sn2 = sn + [pfx] if fresh else sn
-        dsn2 = (dsn + [dpfx]) if fresh else dsn
-        R.resnorm_fwd(None if fresh else pfx, None if fresh else dpfx, a_out[:rows],
-                      a_out[rows:] if has_t else None, a_scale, sn2, dsn2,
-                      w2 if use_res else None, g_n2, eps, n2[0], n2[1] if has_t else None,
-                      p2[0], p2[1] if has_t else None)
-        # 10. MLP
-        gu = K.gemm(n2.view(T * rows, d), W13)                       # [T*rows, 2*fp]
-        act = new(T * rows, g.fp)
-        R.situ_fwd(gu[:rows], gu[rows:] if has_t else None, act[:rows],
-                   act[rows:] if has_t else None, rows, g.fp, beta, lbeta)
-        m = K.gemm(act, W2)                                          # [T*rows, d]
-        # 11. residual
+        gu, act = new(T * rows, 2 * g.fp), new(T * rows, g.fp)
         out = new(T, rows, d, dt=F32)
-        R.scale_add_fwd(p2[0], p2[1] if has_t else None, m[:rows], m[rows:] if has_t else None,
-                        m_scale, out[0], out[1] if has_t else None, rows, d)
+        ptrs = [ptr(o), ptr(do), ptr(a_), ptr(og), ptr(W_out), ptr(a_out), ptr(a_scale),
+                0 if fresh else ptr(pfx), 0 if fresh else ptr(dpfx), ptr(p2), ptr(n2),
+                ptr(w2) if use_res else 0, ptr(g_n2), ptr(W13), ptr(gu), ptr(act), ptr(W2), ptr(m),
+                ptr(m_scale), ptr(out), status]
+        ptrs += [ptr(s) for s in sn2] + [ptr(s) for s in dsn2]
+        K._check(_lib.imf_block_post(R._ptr_array(ptrs), dims(len(sn2)), float(eps), float(beta),
+                                     float(lbeta or 0.0), stream), "imf_block_post")
+        K.LAUNCHES.count += 7 if g.gate else 6
         if need_bwd:
             ctx.save_for_backward(prefix, *snaps, w1, w2, g_n1, g_n2, g_qa, g_kva, g_qn, g_kn,
                                   a_scale, m_scale, W_a, W_qb, W_kvb, W_out, W13, W2, cos, sin,

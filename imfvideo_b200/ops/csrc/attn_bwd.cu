@@ -846,9 +846,8 @@ extern "C" int imf_attn_bwd(const void* q, const void* k, const void* v, const v
   prm.qrank = ordered ? qrank : nullptr;
   const size_t smem = sizeof(BwSmem) + 1024;
   auto kern = qlist != nullptr ? attn_bwd_kernel<true> : attn_bwd_kernel<false>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
-    return IMF_ERR_LAUNCH;
+  static bool smem_set[2][HOST_MAX_DEVICES] = {{false}};
+  if (!allow_smem((const void*)kern, smem, smem_set[qlist != nullptr])) return IMF_ERR_LAUNCH;
   kern<<<sp.ctas(), BW_THREADS, smem, st>>>(mq, mk, mv, mdo, mdq, maq, mad, prm);
   if (cudaGetLastError() != cudaSuccess) return IMF_ERR_LAUNCH;
   if (sp.n_split) {

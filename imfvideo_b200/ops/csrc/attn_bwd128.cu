@@ -575,9 +575,8 @@ int attn_bwd128_launch(const Bwd128Args& a) {
   prm.part = sp.n_split ? reinterpret_cast<float*>(end) : nullptr;
   prm.turn = (a.fixed_order && a.status != nullptr) ? turn : nullptr;
   const size_t smem = sizeof(Smem) + 1024;
-  if (cudaFuncSetAttribute(attn_bwd128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
-    return IMF_ERR_LAUNCH;
+  static bool smem_set[HOST_MAX_DEVICES] = {false};
+  if (!allow_smem((const void*)attn_bwd128_kernel, smem, smem_set)) return IMF_ERR_LAUNCH;
   attn_bwd128_kernel<<<sp.ctas(), THREADS, smem, st>>>(mq, mk, mv, mdo, mdq, prm);
   if (cudaGetLastError() != cudaSuccess) return IMF_ERR_LAUNCH;
   if (sp.n_split) {

@@ -599,9 +599,8 @@ static int launch_attn_fwd(const void* q, const void* k, const void* v, const vo
   }
   auto kern = attn_fwd_kernel<TANGENT, NTP>;
   const size_t smem = sizeof(AttSmem<TANGENT, NTP>) + 1024;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
-    return IMF_ERR_LAUNCH;
+  static bool smem_set[HOST_MAX_DEVICES] = {false};
+  if (!allow_smem((const void*)kern, smem, smem_set)) return IMF_ERR_LAUNCH;
   kern<<<G, C::THREADS, smem, stream>>>(mq, mk, mv, mdq, mdk, mdv, prm);
   if (cudaGetLastError() != cudaSuccess) return IMF_ERR_LAUNCH;
   if (G != prm.sh.n_items) {

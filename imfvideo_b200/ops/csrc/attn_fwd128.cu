@@ -627,9 +627,8 @@ static int launch(const Fwd128Args& a) {
   }
   auto kern = attn_fwd128_kernel<TANGENT>;
   const size_t smem = sizeof(Smem<TANGENT>) + 1024;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
-    return IMF_ERR_LAUNCH;
+  static bool smem_set[HOST_MAX_DEVICES] = {false};
+  if (!allow_smem((const void*)kern, smem, smem_set)) return IMF_ERR_LAUNCH;
   cudaStream_t stream = static_cast<cudaStream_t>(a.stream);
   kern<<<G, C::THREADS, smem, stream>>>(mq, mk, mv, mdq, mdk, mdv, prm);
   if (cudaGetLastError() != cudaSuccess) return IMF_ERR_LAUNCH;

@@ -910,8 +910,8 @@ extern "C" int imf_attn_sparse_fwd(const void* q8, const void* k8, const float* 
     const size_t smem = sizeof(SpSmem<T_, I_>);                                                 \
     int grid = (p.n_tiles + C_::NT - 1) / C_::NT;                                               \
     if (grid > sms * C_::CTAS_PER_SM) grid = sms * C_::CTAS_PER_SM;                             \
-    if (cudaFuncSetAttribute(attn_sparse_fwd_kernel<T_, I_>,                                    \
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) \
+    static bool smem_set[HOST_MAX_DEVICES] = {false};                                           \
+    if (!allow_smem((const void*)attn_sparse_fwd_kernel<T_, I_>, smem, smem_set))               \
       return IMF_ERR_LAUNCH;                                                                    \
     attn_sparse_fwd_kernel<T_, I_><<<grid, C_::THREADS, smem, st>>>(mq8, mk8, mq, mk, mv, mdq,  \
                                                                     mdk, mdv, p);               \

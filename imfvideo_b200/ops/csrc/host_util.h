@@ -65,4 +65,18 @@ inline int make_tmap(CUtensorMap* out, CUtensorMapDataType dt, int rank, void* b
   return IMF_OK;
 }
 
+// Allow a kernel its dynamic shared memory, once per device (`done`: a static array of the
+// caller's, one per kernel; the call costs the host more than the launch itself otherwise).
+constexpr int HOST_MAX_DEVICES = 64;
+inline bool allow_smem(const void* kern, size_t smem, bool (&done)[HOST_MAX_DEVICES]) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const bool known = dev >= 0 && dev < HOST_MAX_DEVICES;
+  if (known && done[dev]) return true;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return false;
+  if (known) done[dev] = true;
+  return true;
+}
+
 }  // namespace imf

@@ -42,6 +42,8 @@ def available() -> bool:
     if os.environ.get("IMF_B200_ALLOW_FALLBACK") == "1" and \
             os.environ.get("IMF_B200_FORCE_TORCH") == "1":
         return False
+    if _registered:              # device seen and library loaded: neither goes away again
+        return True
     if not torch.cuda.is_available():
         return False
     if lib() is None:

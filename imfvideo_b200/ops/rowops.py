@@ -42,7 +42,7 @@ def _p(t: Optional[torch.Tensor]) -> int:
 
 
 def _ptr_array(ptrs: Sequence[int]):
-    return (c_void_p * len(ptrs))(*[c_void_p(x) for x in ptrs])
+    return (c_void_p * len(ptrs))(*ptrs)
 
 
 def _ints(vals: Sequence[int]):
