@@ -50,8 +50,12 @@ constexpr int BW_T = 128;            // tile rows (both q and kv)
 constexpr int BW_THREADS = 512;
 constexpr int BW_QSTAGES = 2;
 
-// TMEM columns
-constexpr int BC_S = 0, BC_DP = 128, BC_P = 256, BC_DK = 320, BC_DV = 384, BC_DQ = 448;
+// TMEM columns.  P^T and dS^T (bf16) overwrite the scores they are made from: query columns
+// 0-63 of S^T become columns 0-31, query columns 64-127 become columns 64-95 (each half is read
+// and written by one warp group only); dP^T likewise.
+constexpr int BC_S = 0, BC_DP = 128, BC_K = 256, BC_V = 288, BC_DK = 320, BC_DV = 384, BC_DQ = 448;
+// columns of the bf16 A operand of k-step `ks` (16 query rows) in an overwritten score tile
+__device__ __forceinline__ constexpr int bw_step_col(int ks) { return (ks >> 2) * 64 + (ks & 3) * 8; }
 
 struct BwSmem {
   alignas(1024) uint8_t k[BW_T * 128];
@@ -65,7 +69,8 @@ struct BwSmem {
   alignas(1024) uint8_t augd[BW_QSTAGES][BW_T * 32]; // [q 128][16]: -delta as (hi, lo), zeros
   uint64_t kv_full;
   uint64_t q_full[BW_QSTAGES], q_empty[BW_QSTAGES];
-  uint64_t s_full, s_taken, p_ready, p_free;
+  uint64_t kv_tmem;                 // K and V have been copied to TMEM
+  uint64_t s_full, dp_full, p_ready, ds_ready;
   uint64_t ds_free[2];
   uint64_t dq_full, dq_free;
   uint64_t final_bar;
@@ -172,10 +177,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       mbar_init(&s.q_full[i], 1);
       mbar_init(&s.q_empty[i], 1);
     }
+    mbar_init(&s.kv_tmem, 8);      // one arrival per exp warp
     mbar_init(&s.s_full, 1);
-    mbar_init(&s.s_taken, 8);      // one arrival per exp warp
+    mbar_init(&s.dp_full, 1);
     mbar_init(&s.p_ready, 8);
-    mbar_init(&s.p_free, 1);
+    mbar_init(&s.ds_ready, 8);
     mbar_init(&s.ds_free[0], 1);
     mbar_init(&s.ds_free[1], 1);
     mbar_init(&s.dq_full, 1);
@@ -203,7 +209,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (warp == 13) {
       // ---------------------------------------------------- TMA producer --
-      if (elect_one()) {
+      if (n_q > 0 && elect_one()) {
         prefetch_tmap(&tm_q);
         prefetch_tmap(&tm_k);
         prefetch_tmap(&tm_v);
@@ -240,10 +246,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     } else if (warp == 12) {
       // ------------------------------------------------------ MMA issuer --
       if (elect_one()) {
-        constexpr uint32_t id_st = idesc_bf16(BW_T, BW_T, 0, 0);     // S^T, dP^T
-        constexpr uint32_t id_kn = idesc_bf16(BW_T, BW_HD, 0, 1);    // dV (TS), dK (SS, A K-major)
-        constexpr uint32_t id_mn = idesc_bf16(BW_T, BW_HD, 1, 1);    // dQ (A MN-major)
-        const uint32_t ka = smem_u32(s.k), va = smem_u32(s.v);
+        constexpr uint32_t id_st = idesc_bf16(BW_T, BW_T, 0, 0);     // S^T, dP^T (TS)
+        constexpr uint32_t id_kn = idesc_bf16(BW_T, BW_HD, 0, 1);    // dV, dK (TS)
+        constexpr uint32_t id_mn = idesc_bf16(BW_T, BW_HD, 1, 1);    // dQ (SS, A MN-major)
+        const uint32_t ka = smem_u32(s.k);
         const uint64_t ones_d = sdesc_kmajor_sw32(smem_u32(s.ones));
         constexpr uint32_t id_st64 = idesc_bf16(BW_T, 64, 0, 0);     // one 64-row query half
         // Block-sparse tiles: `f` has one bit per 64 x 64 quadrant (kv half * 2 + q half).  A
@@ -251,86 +257,79 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // and of the K dimension of dV / dK; a K/V half that no query half attends is left out
         // of the K dimension of dQ.  The math warps write zeros for dead quadrants, so the
         // skipped products would only have added zeros.  Dense: f = 15.
-        auto issue_s = [&](int st, uint32_t f) {
-          const uint32_t qa = smem_u32(s.q[st]), doa = smem_u32(s.d_o[st]);
+        // D = [K | ones] [Q | -lse2]^T (the exponent itself) or [V | ones] [dO | -delta]^T: K and V
+        // are A operands in TMEM, so only the query side is read from shared memory
+        auto issue_scores = [&](uint32_t d_col, uint32_t a_col, uint32_t b_tile, uint32_t aug, uint32_t f) {
           const uint32_t qh = ((f & 5u) ? 1u : 0u) | ((f & 10u) ? 2u : 0u);   // live query halves
-          if (qh == 3u) {
+          const uint32_t half = qh == 2u;                     // the live one, if only one is
+          const uint32_t bt = b_tile + half * (64 * 128), d = tmem + d_col + half * 64;
+          const uint32_t id = qh == 3u ? id_st : id_st64;
 #pragma unroll
-            for (int ks = 0; ks < BW_HD / 16; ++ks)
-              mma_ss(tmem + BC_S, sdesc_kmajor(ka + ks * 32), sdesc_kmajor(qa + ks * 32), id_st, ks != 0);
-            // + ones[kv] x (-lse2[q])  ->  the accumulator holds the exponent itself
-            mma_ss(tmem + BC_S, ones_d, sdesc_kmajor_sw32(smem_u32(s.augq[st])), id_st, 1);
-#pragma unroll
-            for (int ks = 0; ks < BW_HD / 16; ++ks)
-              mma_ss(tmem + BC_DP, sdesc_kmajor(va + ks * 32), sdesc_kmajor(doa + ks * 32), id_st, ks != 0);
-            // + ones[kv] x (-delta[q])  ->  dP - delta
-            mma_ss(tmem + BC_DP, ones_d, sdesc_kmajor_sw32(smem_u32(s.augd[st])), id_st, 1);
-          } else {
-            const uint32_t h = qh >> 1;                     // the live half: rows 64 h .. 64 h + 63
-            const uint32_t qo = h * (64 * 128), ao = h * (64 * 32), co = h * 64;
-#pragma unroll
-            for (int ks = 0; ks < BW_HD / 16; ++ks)
-              mma_ss(tmem + BC_S + co, sdesc_kmajor(ka + ks * 32), sdesc_kmajor(qa + qo + ks * 32),
-                     id_st64, ks != 0);
-            mma_ss(tmem + BC_S + co, ones_d, sdesc_kmajor_sw32(smem_u32(s.augq[st]) + ao), id_st64, 1);
-#pragma unroll
-            for (int ks = 0; ks < BW_HD / 16; ++ks)
-              mma_ss(tmem + BC_DP + co, sdesc_kmajor(va + ks * 32), sdesc_kmajor(doa + qo + ks * 32),
-                     id_st64, ks != 0);
-            mma_ss(tmem + BC_DP + co, ones_d, sdesc_kmajor_sw32(smem_u32(s.augd[st]) + ao), id_st64, 1);
-          }
+          for (int ks = 0; ks < BW_HD / 16; ++ks)
+            mma_ts(d, tmem + a_col + ks * 8, sdesc_kmajor(bt + ks * 32), id, ks != 0);
+          mma_ss(d, ones_d, sdesc_kmajor_sw32(aug + half * (64 * 32)), id, 1);
+        };
+        auto issue_s = [&](int st, uint32_t f) {
+          issue_scores(BC_S, BC_K, smem_u32(s.q[st]), smem_u32(s.augq[st]), f);
           tc_commit(&s.s_full);
+        };
+        auto issue_dp = [&](int st, uint32_t f) {
+          issue_scores(BC_DP, BC_V, smem_u32(s.d_o[st]), smem_u32(s.augd[st]), f);
+          tc_commit(&s.dp_full);
         };
         bool ok = n_q > 0 &&      // a K/V tile that no query tile attends has zero gradients
                   mbar_wait(&s.kv_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMA) &&
+                  mbar_wait(&s.kv_tmem, 0, abort_flag, p.status, STATUS_TIMEOUT_SOFTMAX) &&
                   mbar_wait(&s.q_full[0], 0, abort_flag, p.status, STATUS_TIMEOUT_TMA);
         if (ok) {
           tc_fence_after();
           issue_s(0, flags_at(0));
+          issue_dp(0, flags_at(0));
         }
         bool kv_started = false;     // dK / dV accumulators hold something
         for (int i = 0; i < n_q && ok; ++i) {
-          const int st = i % BW_QSTAGES;
+          const int st = i % BW_QSTAGES, st1 = (i + 1) % BW_QSTAGES;
           const uint32_t par = (uint32_t)(i & 1);
-          ok = mbar_wait(&s.s_taken, par, abort_flag, p.status, STATUS_TIMEOUT_SOFTMAX);
+          const uint32_t f = flags_at(i);
+          // k-steps of 16 query rows that belong to a live query half / of 16 K/V rows that
+          // belong to a live K/V half
+          const int q0 = (f & 5u) ? 0 : 4, q1 = (f & 10u) ? 8 : 4;
+          const int k0 = (f & 3u) ? 0 : 4, k1 = (f & 12u) ? 8 : 4;
+          const uint32_t qa = smem_u32(s.q[st]), doa = smem_u32(s.d_o[st]);
+          const uint32_t dsa = smem_u32(s.ds[i & 1]);
+          // dV += P^T dO, then the next scores over P^T, while the math warps work on dS^T
+          ok = mbar_wait(&s.p_ready, par, abort_flag, p.status, STATUS_TIMEOUT_SOFTMAX);
           if (!ok) break;
+          tc_fence_after();
+#pragma unroll
+          for (int ks = 0; ks < BW_T / 16; ++ks)
+            if (ks >= q0 && ks < q1)
+              mma_ts(tmem + BC_DV, tmem + BC_S + bw_step_col(ks),
+                     sdesc_mnmajor(doa + ks * 2048, BW_T * 128), id_kn, kv_started || ks != q0);
           if (i + 1 < n_q) {
-            const int st1 = (i + 1) % BW_QSTAGES;
             ok = mbar_wait(&s.q_full[st1], (uint32_t)(((i + 1) / BW_QSTAGES) & 1), abort_flag,
                            p.status, STATUS_TIMEOUT_TMA);
             if (!ok) break;
             tc_fence_after();
             issue_s(st1, flags_at(i + 1));
           }
-          ok = mbar_wait(&s.p_ready, par, abort_flag, p.status, STATUS_TIMEOUT_SOFTMAX);
+          // dK += dS^T Q, the next dP^T over dS^T, dQ_i = dS K, while the math warps take the
+          // exponentials of the next scores
+          ok = mbar_wait(&s.ds_ready, par, abort_flag, p.status, STATUS_TIMEOUT_SOFTMAX);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t qa = smem_u32(s.q[st]), doa = smem_u32(s.d_o[st]);
-          const uint32_t dsa = smem_u32(s.ds[i & 1]);
-          const uint32_t f = flags_at(i);
-          // k-steps of 16 query rows that belong to a live query half / of 16 K/V rows that
-          // belong to a live K/V half
-          const int q0 = (f & 5u) ? 0 : 4, q1 = (f & 10u) ? 8 : 4;
-          const int k0 = (f & 3u) ? 0 : 4, k1 = (f & 12u) ? 8 : 4;
-          // dV += P^T dO   (A = P^T in TMEM: 128 q as K -> 8 k-steps of 8 columns)
 #pragma unroll
           for (int ks = 0; ks < BW_T / 16; ++ks)
             if (ks >= q0 && ks < q1)
-              mma_ts(tmem + BC_DV, tmem + BC_P + ks * 8,
-                     sdesc_mnmajor(doa + ks * 2048, BW_T * 128), id_kn, kv_started || ks != q0);
-          tc_commit(&s.p_free);
-          // dK += dS^T Q   (A = dS^T from smem, K-major view: K = q)
-#pragma unroll
-          for (int ks = 0; ks < BW_T / 16; ++ks)
-            if (ks >= q0 && ks < q1)
-              mma_ss(tmem + BC_DK, sdesc_kmajor(dsa + (ks / 4) * (BW_T * 128) + (ks % 4) * 32),
+              mma_ts(tmem + BC_DK, tmem + BC_DP + bw_step_col(ks),
                      sdesc_mnmajor(qa + ks * 2048, BW_T * 128), id_kn, kv_started || ks != q0);
           kv_started = true;
           // the query-side stage (Q, dO, bands) has had its last reader: hand it back to the
           // TMA producer now, not after the dQ GEMM -- with two stages, the load of tile i+2
-          // starts here and its latency sets the pace of the whole pipeline
+          // starts here
           tc_commit(&s.q_empty[st]);
-          // dQ_i = dS K    (A = dS^T from smem, MN-major view: M = q, K = kv)
+          if (i + 1 < n_q) issue_dp(st1, flags_at(i + 1));
+          // A = dS^T from smem, MN-major view: M = q, K = kv
           if (i > 0) {
             ok = mbar_wait(&s.dq_free, (uint32_t)((i - 1) & 1), abort_flag, p.status,
                            STATUS_TIMEOUT_SOFTMAX);
@@ -429,55 +428,92 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const int row = wl * 32 + lane;     // kv row of this thread (TMEM lane)
     const uint32_t tb = tmem_addr(tmem, wl * 32, 0);
     bool ok = true;
+    if (n_q > 0) {                      // warps 0-3 copy K, warps 4-7 copy V to TMEM
+      ok = __all_sync(0xffffffffu, mbar_wait(&s.kv_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMA));
+      if (ok) {
+        const uint8_t* src = (wg == 0 ? s.k : s.v) + row * 128;
+        uint32_t r[32];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const uint4 u = *reinterpret_cast<const uint4*>(src + ((c ^ (row & 7)) << 4));
+          r[4 * c] = u.x; r[4 * c + 1] = u.y; r[4 * c + 2] = u.z; r[4 * c + 3] = u.w;
+        }
+        tmem_st32(tb + (wg == 0 ? BC_K : BC_V), r);
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s.kv_tmem);
+      }
+    }
     for (int i = 0; i < n_q && ok; ++i) {
       const uint32_t par = (uint32_t)(i & 1);
+      // block-sparse: this thread's 64 columns are one (kv half, q half) quadrant, this warp's
+      // 32 rows and 64 columns lie in it
+      const bool live = !SPARSE || ((flags_at(i) >> ((row >> 6) * 2 + wg)) & 1);
+      // P^T = exp2(S scale log2e - lse2), the exponents straight from the tensor core
       ok = __all_sync(0xffffffffu,
                       mbar_wait(&s.s_full, par, abort_flag, p.status, STATUS_TIMEOUT_MMA));
       if (!ok) break;
       tc_fence_after();
-      uint32_t sv[64], dp[64];
-      tmem_ld32(tb + BC_S + wg * 64, sv);
-      tmem_ld32(tb + BC_S + wg * 64 + 32, sv + 32);
-      tmem_ld32(tb + BC_DP + wg * 64, dp);
-      tmem_ld32(tb + BC_DP + wg * 64 + 32, dp + 32);
-      tc_wait_ld();
+      uint32_t sv[64];                  // the exponents, then P^T
+      if (live) {
+        tmem_ld32(tb + BC_S + wg * 64, sv);
+        tc_wait_ld();
+        tmem_ld32(tb + BC_S + wg * 64 + 32, sv + 32);
+      }
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh) {
+        uint32_t pk[16];
+#pragma unroll
+        for (int c = 0; c < 32; c += 2) {
+          const int cg = hh * 32 + c;
+          if (live) {
+            const float p0 = ex2(__uint_as_float(sv[cg])), p1 = ex2(__uint_as_float(sv[cg + 1]));
+            pk[c / 2] = pack_bf16(p0, p1);
+            sv[cg] = __float_as_uint(p0);
+            sv[cg + 1] = __float_as_uint(p1);
+          } else {
+            pk[c / 2] = 0u;
+          }
+        }
+        if (hh == 0 && live) tc_wait_ld();
+        tmem_st16(tb + BC_S + wg * 64 + hh * 16, pk);
+      }
+      tc_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&s.s_taken);
-      // P^T goes to TMEM (A operand of the dV GEMM): dV of tile i-1 must have read it;
-      // dS^T goes to smem buffer i&1: the GEMMs of tile i-2 must have read it
-      if (i > 0) {
-        ok = __all_sync(0xffffffffu, mbar_wait(&s.p_free, (uint32_t)((i - 1) & 1), abort_flag,
-                                               p.status, STATUS_TIMEOUT_MMA));
-        if (!ok) break;
-      }
-      if (i >= 2) {
+      if (lane == 0) mbar_arrive(&s.p_ready);
+      // dS^T = P^T .* (dP^T - delta), the bracket straight from the tensor core: to TMEM for dK and
+      // to smem buffer i&1 for dQ (the dQ GEMM of tile i-2 must have read it)
+      ok = __all_sync(0xffffffffu,
+                      mbar_wait(&s.dp_full, par, abort_flag, p.status, STATUS_TIMEOUT_MMA));
+      if (ok && i >= 2)
         ok = __all_sync(0xffffffffu,
                         mbar_wait(&s.ds_free[i & 1], (uint32_t)(((i / 2) - 1) & 1), abort_flag,
                                   p.status, STATUS_TIMEOUT_MMA));
-        if (!ok) break;
-      }
+      if (!ok) break;
+      tc_fence_after();
       uint8_t* dsb = s.ds[i & 1] + wg * (BW_T * 128) + row * 128;
-      // block-sparse: this thread's 64 columns are one (kv half, q half) quadrant
-      const bool live = !SPARSE || ((flags_at(i) >> ((row >> 6) * 2 + wg)) & 1);
+      uint32_t dp[2][32];
+      if (live) {
+        tmem_ld32(tb + BC_DP + wg * 64, dp[0]);
+        tc_wait_ld();
+        tmem_ld32(tb + BC_DP + wg * 64 + 32, dp[1]);
+      }
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
-        uint32_t pk[16], dk_[16];
-        if (live) {        // warp-uniform: a warp's 32 rows and 64 columns lie in one quadrant
+        uint32_t dk_[16];
 #pragma unroll
-          for (int c = 0; c < 32; c += 2) {
-            const int cg = hh * 32 + c;
-            // sv = S scale log2e - lse2 and dp = dP - delta, straight from the tensor core
-            const float p0 = ex2(__uint_as_float(sv[cg]));
-            const float p1 = ex2(__uint_as_float(sv[cg + 1]));
-            pk[c / 2] = pack_bf16(p0, p1);
-            dk_[c / 2] = pack_bf16(p0 * __uint_as_float(dp[cg]), p1 * __uint_as_float(dp[cg + 1]));
+        for (int c = 0; c < 32; c += 2) {
+          if (live) {
+            const f32x2 d = mul2(pair2(sv[hh * 32 + c], sv[hh * 32 + c + 1]), pair2(dp[hh][c], dp[hh][c + 1]));
+            dk_[c / 2] = pack_bf16(lo2(d), hi2(d));
+          } else {
+            dk_[c / 2] = 0u;
           }
-        } else {           // block-sparse: this quadrant is not attended
-#pragma unroll
-          for (int c = 0; c < 16; ++c) pk[c] = dk_[c] = 0u;
         }
-        tmem_st16(tb + BC_P + wg * 32 + hh * 16, pk);
+        if (hh == 0 && live) tc_wait_ld();       // columns 16-31 are written over next
+        tmem_st16(tb + BC_DP + wg * 64 + hh * 16, dk_);
 #pragma unroll
         for (int cc = 0; cc < 4; ++cc) {
           const int chunk = hh * 4 + cc;
@@ -489,7 +525,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       fence_proxy_async_smem();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&s.p_ready);
+      if (lane == 0) mbar_arrive(&s.ds_ready);
     }
     // ---- epilogue: WG0 stores dK (scaled), WG1 stores dV ----
     if (ok && n_q > 0) ok = mbar_wait(&s.final_bar, 0, abort_flag, p.status, STATUS_TIMEOUT_MMA);
