@@ -13,9 +13,9 @@
 //
 // CTA = one 128-row K/V tile of one (batch, head); it walks over all 128-row
 // Q tiles.  Everything is computed TRANSPOSED (K/V rows on the TMEM lanes), so
-// P^T can stay in TMEM as the A operand of the dV GEMM, and dK/dV accumulate
-// in TMEM for the whole walk.  dS^T goes through shared memory once and feeds
-// both the dK GEMM (K-major view) and the dQ GEMM (MN-major view).  dQ tiles
+// P^T and dS^T are the A operands of the dV and dK GEMMs from TMEM, and dK/dV
+// accumulate in TMEM for the whole walk.  dS^T also goes through shared memory
+// once, for the dQ GEMM (MN-major view).  dQ tiles
 // are added to an fp32 accumulator in global memory by TMA (reduce-add),
 // converted to bf16 by a small epilogue kernel.  On request the adds to one
 // query tile happen in a FIXED order (a turn counter per query tile), so the
@@ -36,8 +36,18 @@
 //
 // Warps 0-3 / 4-7: exp / dS math for columns 0-63 / 64-127 of the S^T tile;
 // warps 8-11: dQ tile TMEM -> global reduction; warp 12: tcgen05.mma issuer;
-// warp 13: TMA producer.  S^T/dP^T of tile i+1 are issued as soon as tile i
-// has been pulled into registers, so the tensor core overlaps the exp math.
+// warp 13: TMA producer.  S^T of tile i+1 is issued as soon as S^T of tile i has
+// been pulled into registers, dV while the math warps work on dS^T, and dK, dQ
+// and dP^T of tile i+1 while they take the next exponentials.
+//
+// What bounds it (B 1, H 4, L 29,140: 2.15 ms, 2,900 clocks per tile): the exponential
+// unit needs 1,024 of them and the tensor core 1,540, but the math warps do one after
+// the other what is left between the barriers, each of which costs 150 to 300 clocks
+// while shared memory moves 296 KB per tile (2,312 clocks at 128 B).  96 KB of that is
+// the dQ tile on its way out: without it the kernel takes 1.91 ms; adding it to global
+// memory from registers instead takes 2.29 ms.  Other arrangements of TMEM measured: K
+// and V as TMEM operands with P^T over S^T 2.21 ms (the next S^T waits for dV), the two
+// warp groups half a tile apart 3.24 ms.
 #include "attn_bwd128.h"
 #include "attn_bwd_split.h"
 #include "common.cuh"
@@ -48,13 +58,13 @@ namespace imf {
 constexpr int BW_HD = 64;
 constexpr int BW_T = 128;            // tile rows (both q and kv)
 constexpr int BW_THREADS = 512;
-constexpr int BW_QSTAGES = 2;
+constexpr int BW_QSTAGES = 3;
 
-// TMEM columns.  P^T and dS^T (bf16) overwrite the scores they are made from: query columns
-// 0-63 of S^T become columns 0-31, query columns 64-127 become columns 64-95 (each half is read
-// and written by one warp group only); dP^T likewise.
-constexpr int BC_S = 0, BC_DP = 128, BC_K = 256, BC_V = 288, BC_DK = 320, BC_DV = 384, BC_DQ = 448;
-// columns of the bf16 A operand of k-step `ks` (16 query rows) in an overwritten score tile
+// TMEM columns.  dS^T (bf16) overwrites the dP^T it is made from: query columns 0-63 become columns
+// 0-31, query columns 64-127 become columns 64-95 (each half is read and written by one warp group
+// only).
+constexpr int BC_S = 0, BC_DP = 128, BC_P = 256, BC_DK = 320, BC_DV = 384, BC_DQ = 448;
+// column of the bf16 A operand of k-step `ks` (16 query rows) in the overwritten tile
 __device__ __forceinline__ constexpr int bw_step_col(int ks) { return (ks >> 2) * 64 + (ks & 3) * 8; }
 
 struct BwSmem {
@@ -62,16 +72,14 @@ struct BwSmem {
   alignas(1024) uint8_t v[BW_T * 128];
   alignas(1024) uint8_t q[BW_QSTAGES][BW_T * 128];
   alignas(1024) uint8_t d_o[BW_QSTAGES][BW_T * 128];
-  alignas(1024) uint8_t ds[2][2 * BW_T * 128];       // dS^T: [kv 128][q 128] as two 64-col panels
+  alignas(1024) uint8_t ds[2 * BW_T * 128];          // dS^T: [kv 128][q 128] as two 64-col panels
   alignas(1024) float dq_stage[BW_T * BW_HD];        // dQ tile staged for the TMA reduce-add
   alignas(1024) uint8_t ones[BW_T * 32];             // [128][16] bf16 1.0, 32-byte rows (SWIZZLE_32B)
   alignas(1024) uint8_t augq[BW_QSTAGES][BW_T * 32]; // [q 128][16]: -lse2 as (hi, lo), zeros
   alignas(1024) uint8_t augd[BW_QSTAGES][BW_T * 32]; // [q 128][16]: -delta as (hi, lo), zeros
   uint64_t kv_full;
   uint64_t q_full[BW_QSTAGES], q_empty[BW_QSTAGES];
-  uint64_t kv_tmem;                 // K and V have been copied to TMEM
-  uint64_t s_full, dp_full, p_ready, ds_ready;
-  uint64_t ds_free[2];
+  uint64_t s_full, s_taken, dp_full, p_ready, p_free, ds_ready;
   uint64_t dq_full, dq_free;
   uint64_t final_bar;
   uint32_t tmem_base;
@@ -177,13 +185,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       mbar_init(&s.q_full[i], 1);
       mbar_init(&s.q_empty[i], 1);
     }
-    mbar_init(&s.kv_tmem, 8);      // one arrival per exp warp
     mbar_init(&s.s_full, 1);
+    mbar_init(&s.s_taken, 8);      // one arrival per exp warp
+    mbar_init(&s.p_free, 1);
     mbar_init(&s.dp_full, 1);
     mbar_init(&s.p_ready, 8);
     mbar_init(&s.ds_ready, 8);
-    mbar_init(&s.ds_free[0], 1);
-    mbar_init(&s.ds_free[1], 1);
     mbar_init(&s.dq_full, 1);
     mbar_init(&s.dq_free, 4);
     mbar_init(&s.final_bar, 1);
@@ -206,7 +213,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   volatile int* abort_flag = &s.abort_flag;
 
   if (warp >= 12) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
     if (warp == 13) {
       // ---------------------------------------------------- TMA producer --
       if (n_q > 0 && elect_one()) {
@@ -246,10 +253,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     } else if (warp == 12) {
       // ------------------------------------------------------ MMA issuer --
       if (elect_one()) {
-        constexpr uint32_t id_st = idesc_bf16(BW_T, BW_T, 0, 0);     // S^T, dP^T (TS)
+        constexpr uint32_t id_st = idesc_bf16(BW_T, BW_T, 0, 0);     // S^T, dP^T (SS)
         constexpr uint32_t id_kn = idesc_bf16(BW_T, BW_HD, 0, 1);    // dV, dK (TS)
         constexpr uint32_t id_mn = idesc_bf16(BW_T, BW_HD, 1, 1);    // dQ (SS, A MN-major)
-        const uint32_t ka = smem_u32(s.k);
+        const uint32_t ka = smem_u32(s.k), va = smem_u32(s.v), dsa = smem_u32(s.ds);
         const uint64_t ones_d = sdesc_kmajor_sw32(smem_u32(s.ones));
         constexpr uint32_t id_st64 = idesc_bf16(BW_T, 64, 0, 0);     // one 64-row query half
         // Block-sparse tiles: `f` has one bit per 64 x 64 quadrant (kv half * 2 + q half).  A
@@ -257,29 +264,27 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // and of the K dimension of dV / dK; a K/V half that no query half attends is left out
         // of the K dimension of dQ.  The math warps write zeros for dead quadrants, so the
         // skipped products would only have added zeros.  Dense: f = 15.
-        // D = [K | ones] [Q | -lse2]^T (the exponent itself) or [V | ones] [dO | -delta]^T: K and V
-        // are A operands in TMEM, so only the query side is read from shared memory
-        auto issue_scores = [&](uint32_t d_col, uint32_t a_col, uint32_t b_tile, uint32_t aug, uint32_t f) {
+        // D = [K | ones] [Q | -lse2]^T (the exponent itself) or [V | ones] [dO | -delta]^T
+        auto issue_scores = [&](uint32_t d_col, uint32_t a_tile, uint32_t b_tile, uint32_t aug, uint32_t f) {
           const uint32_t qh = ((f & 5u) ? 1u : 0u) | ((f & 10u) ? 2u : 0u);   // live query halves
           const uint32_t half = qh == 2u;                     // the live one, if only one is
           const uint32_t bt = b_tile + half * (64 * 128), d = tmem + d_col + half * 64;
           const uint32_t id = qh == 3u ? id_st : id_st64;
 #pragma unroll
           for (int ks = 0; ks < BW_HD / 16; ++ks)
-            mma_ts(d, tmem + a_col + ks * 8, sdesc_kmajor(bt + ks * 32), id, ks != 0);
+            mma_ss(d, sdesc_kmajor(a_tile + ks * 32), sdesc_kmajor(bt + ks * 32), id, ks != 0);
           mma_ss(d, ones_d, sdesc_kmajor_sw32(aug + half * (64 * 32)), id, 1);
         };
         auto issue_s = [&](int st, uint32_t f) {
-          issue_scores(BC_S, BC_K, smem_u32(s.q[st]), smem_u32(s.augq[st]), f);
+          issue_scores(BC_S, ka, smem_u32(s.q[st]), smem_u32(s.augq[st]), f);
           tc_commit(&s.s_full);
         };
         auto issue_dp = [&](int st, uint32_t f) {
-          issue_scores(BC_DP, BC_V, smem_u32(s.d_o[st]), smem_u32(s.augd[st]), f);
+          issue_scores(BC_DP, va, smem_u32(s.d_o[st]), smem_u32(s.augd[st]), f);
           tc_commit(&s.dp_full);
         };
         bool ok = n_q > 0 &&      // a K/V tile that no query tile attends has zero gradients
                   mbar_wait(&s.kv_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMA) &&
-                  mbar_wait(&s.kv_tmem, 0, abort_flag, p.status, STATUS_TIMEOUT_SOFTMAX) &&
                   mbar_wait(&s.q_full[0], 0, abort_flag, p.status, STATUS_TIMEOUT_TMA);
         if (ok) {
           tc_fence_after();
@@ -287,33 +292,37 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           issue_dp(0, flags_at(0));
         }
         bool kv_started = false;     // dK / dV accumulators hold something
+        int st = 0;                  // stage of tile i
         for (int i = 0; i < n_q && ok; ++i) {
-          const int st = i % BW_QSTAGES, st1 = (i + 1) % BW_QSTAGES;
+          const int st1 = st + 1 == BW_QSTAGES ? 0 : st + 1;
           const uint32_t par = (uint32_t)(i & 1);
-          const uint32_t f = flags_at(i);
+          const uint32_t f = flags_at(i), f1 = i + 1 < n_q ? flags_at(i + 1) : 0u;
           // k-steps of 16 query rows that belong to a live query half / of 16 K/V rows that
           // belong to a live K/V half
           const int q0 = (f & 5u) ? 0 : 4, q1 = (f & 10u) ? 8 : 4;
           const int k0 = (f & 3u) ? 0 : 4, k1 = (f & 12u) ? 8 : 4;
           const uint32_t qa = smem_u32(s.q[st]), doa = smem_u32(s.d_o[st]);
-          const uint32_t dsa = smem_u32(s.ds[i & 1]);
-          // dV += P^T dO, then the next scores over P^T, while the math warps work on dS^T
+          // the next S^T as soon as this one is in registers: it waits for the math warps when
+          // they come back for it
+          if (i + 1 < n_q) {
+            ok = mbar_wait(&s.q_full[st1], (uint32_t)(((i + 1) / BW_QSTAGES) & 1), abort_flag,
+                           p.status, STATUS_TIMEOUT_TMA) &&
+                 mbar_wait(&s.s_taken, par, abort_flag, p.status, STATUS_TIMEOUT_SOFTMAX);
+            if (!ok) break;
+            tc_fence_after();
+            issue_s(st1, f1);
+          }
+          // dV += P^T dO, while the math warps work on dS^T
           ok = mbar_wait(&s.p_ready, par, abort_flag, p.status, STATUS_TIMEOUT_SOFTMAX);
           if (!ok) break;
           tc_fence_after();
 #pragma unroll
           for (int ks = 0; ks < BW_T / 16; ++ks)
             if (ks >= q0 && ks < q1)
-              mma_ts(tmem + BC_DV, tmem + BC_S + bw_step_col(ks),
-                     sdesc_mnmajor(doa + ks * 2048, BW_T * 128), id_kn, kv_started || ks != q0);
-          if (i + 1 < n_q) {
-            ok = mbar_wait(&s.q_full[st1], (uint32_t)(((i + 1) / BW_QSTAGES) & 1), abort_flag,
-                           p.status, STATUS_TIMEOUT_TMA);
-            if (!ok) break;
-            tc_fence_after();
-            issue_s(st1, flags_at(i + 1));
-          }
-          // dK += dS^T Q, the next dP^T over dS^T, dQ_i = dS K, while the math warps take the
+              mma_ts(tmem + BC_DV, tmem + BC_P + ks * 8, sdesc_mnmajor(doa + ks * 2048, BW_T * 128),
+                     id_kn, kv_started || ks != q0);
+          tc_commit(&s.p_free);
+          // dK += dS^T Q, dQ_i = dS K, the next dP^T over dS^T, while the math warps take the
           // exponentials of the next scores
           ok = mbar_wait(&s.ds_ready, par, abort_flag, p.status, STATUS_TIMEOUT_SOFTMAX);
           if (!ok) break;
@@ -324,11 +333,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               mma_ts(tmem + BC_DK, tmem + BC_DP + bw_step_col(ks),
                      sdesc_mnmajor(qa + ks * 2048, BW_T * 128), id_kn, kv_started || ks != q0);
           kv_started = true;
-          // the query-side stage (Q, dO, bands) has had its last reader: hand it back to the
-          // TMA producer now, not after the dQ GEMM -- with two stages, the load of tile i+2
-          // starts here
-          tc_commit(&s.q_empty[st]);
-          if (i + 1 < n_q) issue_dp(st1, flags_at(i + 1));
+          tc_commit(&s.q_empty[st]);           // the stage has had its last reader
           // A = dS^T from smem, MN-major view: M = q, K = kv
           if (i > 0) {
             ok = mbar_wait(&s.dq_free, (uint32_t)((i - 1) & 1), abort_flag, p.status,
@@ -342,14 +347,16 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               mma_ss(tmem + BC_DQ, sdesc_mnmajor(dsa + ks * 2048, BW_T * 128),
                      sdesc_mnmajor(ka + ks * 2048, BW_T * 128), id_mn, ks != k0);
           tc_commit(&s.dq_full);
-          tc_commit(&s.ds_free[i & 1]);
+          // behind dQ, so that dp_full also says that dS^T in shared memory has been read
+          if (i + 1 < n_q) issue_dp(st1, f1);
+          st = st1;
         }
         if (ok) tc_commit(&s.final_bar);
       }
     }
   } else if (warp >= 8) {
     // ------------------------------------------ dQ tile -> global reduction --
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
     const int wl = warp & 3;
     const uint32_t tb = tmem_addr(tmem, wl * 32, BC_DQ);
     bool ok = true;
@@ -428,39 +435,29 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const int row = wl * 32 + lane;     // kv row of this thread (TMEM lane)
     const uint32_t tb = tmem_addr(tmem, wl * 32, 0);
     bool ok = true;
-    if (n_q > 0) {                      // warps 0-3 copy K, warps 4-7 copy V to TMEM
-      ok = __all_sync(0xffffffffu, mbar_wait(&s.kv_full, 0, abort_flag, p.status, STATUS_TIMEOUT_TMA));
-      if (ok) {
-        const uint8_t* src = (wg == 0 ? s.k : s.v) + row * 128;
-        uint32_t r[32];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const uint4 u = *reinterpret_cast<const uint4*>(src + ((c ^ (row & 7)) << 4));
-          r[4 * c] = u.x; r[4 * c + 1] = u.y; r[4 * c + 2] = u.z; r[4 * c + 3] = u.w;
-        }
-        tmem_st32(tb + (wg == 0 ? BC_K : BC_V), r);
-        tc_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&s.kv_tmem);
-      }
-    }
     for (int i = 0; i < n_q && ok; ++i) {
       const uint32_t par = (uint32_t)(i & 1);
       // block-sparse: this thread's 64 columns are one (kv half, q half) quadrant, this warp's
       // 32 rows and 64 columns lie in it
       const bool live = !SPARSE || ((flags_at(i) >> ((row >> 6) * 2 + wg)) & 1);
       // P^T = exp2(S scale log2e - lse2), the exponents straight from the tensor core
-      ok = __all_sync(0xffffffffu,
-                      mbar_wait(&s.s_full, par, abort_flag, p.status, STATUS_TIMEOUT_MMA));
+      // and the dV GEMM of the previous tile has read P^T (probed first: long done as a rule, and
+      // the two probes' latencies overlap)
+      const bool p_ok = i == 0 || mbar_test(&s.p_free, par ^ 1);
+      ok = mbar_wait(&s.s_full, par, abort_flag, p.status, STATUS_TIMEOUT_MMA) &&
+           (p_ok || mbar_wait(&s.p_free, par ^ 1, abort_flag, p.status, STATUS_TIMEOUT_MMA));
+      ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
       uint32_t sv[64];                  // the exponents, then P^T
       if (live) {
         tmem_ld32(tb + BC_S + wg * 64, sv);
-        tc_wait_ld();
         tmem_ld32(tb + BC_S + wg * 64 + 32, sv + 32);
+        tc_wait_ld();
+        tc_fence_before();
       }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s.s_taken);
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
         uint32_t pk[16];
@@ -476,24 +473,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             pk[c / 2] = 0u;
           }
         }
-        if (hh == 0 && live) tc_wait_ld();
-        tmem_st16(tb + BC_S + wg * 64 + hh * 16, pk);
+        tmem_st16(tb + BC_P + wg * 32 + hh * 16, pk);
       }
       tc_wait_st();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&s.p_ready);
       // dS^T = P^T .* (dP^T - delta), the bracket straight from the tensor core: to TMEM for dK and
-      // to smem buffer i&1 for dQ (the dQ GEMM of tile i-2 must have read it)
+      // to smem for dQ (dP^T was issued behind the dQ GEMM of the previous tile)
       ok = __all_sync(0xffffffffu,
                       mbar_wait(&s.dp_full, par, abort_flag, p.status, STATUS_TIMEOUT_MMA));
-      if (ok && i >= 2)
-        ok = __all_sync(0xffffffffu,
-                        mbar_wait(&s.ds_free[i & 1], (uint32_t)(((i / 2) - 1) & 1), abort_flag,
-                                  p.status, STATUS_TIMEOUT_MMA));
       if (!ok) break;
       tc_fence_after();
-      uint8_t* dsb = s.ds[i & 1] + wg * (BW_T * 128) + row * 128;
+      uint8_t* dsb = s.ds + wg * (BW_T * 128) + row * 128;
       uint32_t dp[2][32];
       if (live) {
         tmem_ld32(tb + BC_DP + wg * 64, dp[0]);
