@@ -129,8 +129,7 @@ class Router(nn.Module):
             topk = max(1, min(nb, int(k_frac * nb)))
             pq, pk = ((self.proj_q.weight, self.proj_k.weight) if self.learnable
                       else (None, None))
-            lut = SP.route_topk(SP.pool_blocks(q, self.bq), SP.pool_blocks(k, self.bk), topk,
-                                pq, pk)
+            lut = SP.route_topk(*SP.pool_blocks_qk(q, self.bq, k, self.bk), topk, pq, pk)
             return None, lut, topk, None
         pc = self.scores(q, k)
         nb = pc.shape[-1]
@@ -155,7 +154,7 @@ def route_tiles(q: Tensor, k: Tensor, topk_frac: float, Np: int, E: int, prefix_
     if _router_kernels_ok(q, k):
         from ..ops import sparse as SP
 
-        lut = SP.route_topk(SP.pool_blocks(q, E), SP.pool_blocks(k, E, Np), T, proj_q, proj_k,
+        lut = SP.route_topk(*SP.pool_blocks_qk(q, E, k, E, Np), T, proj_q, proj_k,
                             n_tail=n_tail, tail0=Np)
         return lut, T
     qb = block_mean(q, E)                                   # (B,H,Mb,D) incl. prefix tail blocks
@@ -480,23 +479,31 @@ class SparseCore:
     def __init__(self, mod, qblk: int, bk: int, n_comp: Optional[int], int8: bool):
         self.mod, self.qblk, self.bk, self.n_comp, self.int8 = mod, qblk, bk, n_comp, int8
 
-    def _sel_and_alpha(self, qh, kh):
+    def _select(self, qh, kh):
         m = self.mod
-        L = qh.shape[2]
         if isinstance(m, SLA2CubeQATAttentionImpl):
-            sel, _ = m.route(qh, kh)
-            a_rows = torch.sigmoid(m.alpha_logit)[:, m.a_index]
-        else:
-            with torch.no_grad():
-                _, sel, _, _ = m.sla2.router(qh, kh, m.sla2.topk, need_mask=False)
-            a_rows = torch.sigmoid(m.sla2.alpha_logit).repeat_interleave(m.bq, dim=-1)[:, :L]
-        return sel, a_rows
+            return m.route(qh, kh)[0]
+        with torch.no_grad():
+            return m.sla2.router(qh, kh, m.sla2.topk, need_mask=False)[1]
+
+    def _a_rows(self, L):
+        """(H, L) mixing ratio per row, differentiable."""
+        m = self.mod
+        if isinstance(m, SLA2CubeQATAttentionImpl):
+            return torch.sigmoid(m.alpha_logit)[:, m.a_index]
+        return torch.sigmoid(m.sla2.alpha_logit).repeat_interleave(m.bq, dim=-1)[:, :L]
+
+    def _alpha(self):
+        """The mixing logits, (H, query blocks): row r of both attention forms takes block
+        r // qblk (a cube's tail blocks come after its tiles)."""
+        m = self.mod
+        return m.alpha_logit if isinstance(m, SLA2CubeQATAttentionImpl) else m.sla2.alpha_logit
 
     def fwd(self, q, k, v, dq, dk, dv, need_bwd: bool):
         from ..ops import sparse as SP
 
         qh, kh, vh = (x.permute(0, 2, 1, 3) for x in (q, k, v))
-        sel, a_rows = self._sel_and_alpha(qh.detach(), kh.detach())
+        sel = self._select(qh.detach(), kh.detach())
         lut, flags, cnt, fm = SP.route_tables(sel, self.qblk, q.shape[1])
         # inference form (no reverse mode to follow, e.g. the sampler and the guidance passes):
         # no log-sum-exp, no saved state; the same INT8 block-sparse kernel and the same
@@ -508,12 +515,13 @@ class SparseCore:
 
         if LA.AVAILABLE:
             with torch.no_grad():
-                o, do, C = LA.forward(q, k, v, dq, dk, dv, o_s, do_s, sel, a_rows, self.qblk,
-                                      self.bk, self.n_comp)
+                o, do, C = LA.forward(q, k, v, dq, dk, dv, o_s, do_s, sel, None, self.qblk, self.bk,
+                                      self.n_comp, alpha=self._alpha())
                 if need_bwd and isinstance(self.mod, SLA2CubeQATAttentionImpl):
                     self.mod.logit_max_log2 = (lse.amax(dim=(0, 2)) * 1.4426950408889634).float()
             return o, do, (sel, lut, flags, o_s, lse, C if need_bwd else None)
         f = lambda a, b, c: linear_branch(a, b, c, sel, self.qblk, self.bk, self.n_comp)
+        a_rows = self._a_rows(q.shape[1])
         with torch.no_grad():
             if dq is not None:
                 o_l, do_l = torch.func.jvp(f, (qh.float(), kh.float(), vh.float()),
@@ -547,8 +555,7 @@ class SparseCore:
         if C is not None:
             return self._bwd_kernels(q, k, v, saved, go, gv_out, alpha_param, cube)
         with torch.enable_grad():
-            a_rows = (torch.sigmoid(alpha_param)[:, m.a_index] if cube else
-                      torch.sigmoid(alpha_param).repeat_interleave(m.bq, dim=-1)[:, :L])
+            a_rows = self._a_rows(L)
             ql, kl, vl = (x.detach().permute(0, 2, 1, 3).float().requires_grad_(True)
                           for x in (q, k, v))
             o_l = linear_branch(ql, kl, vl, sel, self.qblk, self.bk, self.n_comp)
@@ -588,11 +595,8 @@ def _sparse_core_bwd_kernels(self, q, k, v, saved, go, gv_out, alpha_param, cube
     m = self.mod
     B, L, H, D = q.shape
     with torch.no_grad():
-        a_rows = (torch.sigmoid(alpha_param)[:, m.a_index] if cube else
-                  torch.sigmoid(alpha_param).repeat_interleave(m.bq, dim=-1)[:, :L])
-        gq_l, gnum, gden, ga_row, g_os = LA.backward_rows(q, o_s, go, C, a_rows, self.qblk)
-        Mb = -(-L // self.qblk)
-        ga = F.pad(ga_row.sum(0), (0, Mb * self.qblk - L)).view(H, Mb, self.qblk).sum(-1)
+        gq_l, gnum, gden, ga, g_os = LA.backward_rows(q, o_s, go, C, None, self.qblk, alpha=alpha_param)
+        ga = ga[0] if B == 1 else ga.sum(0)
         if ga.shape[1] < alpha_param.shape[1]:
             ga = F.pad(ga, (0, alpha_param.shape[1] - ga.shape[1]))
         ga = ga.to(alpha_param.dtype)

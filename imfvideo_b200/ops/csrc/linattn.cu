@@ -22,6 +22,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "host_util.h"
+
 namespace imf {
 
 constexpr int LD = 64;             // head dim
@@ -317,10 +319,15 @@ struct ApplyArgs {
   RowPtr q, dq, os, dos;
   const float* C;          // [(b, h)][Mb][LSTATE] complement states
   const float* dC;
-  const float* a_rows;     // (H, L) mixing ratio per row
+  const float* a_rows;     // (H, L) mixing ratio per row, or null:
+  const float* alpha;      // (H, alpha_ld) logits per query block, ratio = sigmoid
   RowPtr o, dout;          // bf16 outputs
-  int L, H, Mb, qblk;
+  int L, H, Mb, qblk, alpha_ld;
 };
+
+__device__ __forceinline__ float sigmoid_at(const float* logits, int64_t i) {
+  return 1.f / (1.f + expf(-logits[i]));
+}
 
 template <bool TANGENT>
 __global__ void __launch_bounds__(256) lin_apply_kernel(const ApplyArgs a) {
@@ -336,6 +343,7 @@ __global__ void __launch_bounds__(256) lin_apply_kernel(const ApplyArgs a) {
   const int64_t sidx = (((int64_t)b * a.H + h) * a.Mb + m) * LSTATE;
   load_state(C, a.C + sidx, tid);
   if (TANGENT) load_state(dC, a.dC + sidx, tid);
+  const float al_blk = a.alpha ? sigmoid_at(a.alpha, (int64_t)h * a.alpha_ld + m) : 0.f;
   __syncthreads();
   const float z0 = C[(2 * lane) * LP + 64], z1 = C[(2 * lane + 1) * LP + 64];
   const float dz0 = TANGENT ? dC[(2 * lane) * LP + 64] : 0.f;
@@ -389,7 +397,7 @@ __global__ void __launch_bounds__(256) lin_apply_kernel(const ApplyArgs a) {
       const int row = m * a.qblk + ch + r0 + i;
       if (row >= a.L) continue;
       const float inv = 1.f / Den[r0 + i];
-      const float al = a.a_rows[(int64_t)h * a.L + row], bl = 1.f - al;
+      const float al = a.alpha ? al_blk : a.a_rows[(int64_t)h * a.L + row], bl = 1.f - al;
       float s[4], l[4];
       ld_bf16x4(row_at(a.os, b, row, h) + c0, s);
 #pragma unroll
@@ -421,13 +429,15 @@ __global__ void __launch_bounds__(256) lin_apply_kernel(const ApplyArgs a) {
 struct BwdRowsArgs {
   RowPtr q, os, go;
   const float* C;
-  const float* a_rows;
+  const float* a_rows;     // as in ApplyArgs
+  const float* alpha;
   float* gq;               // (B, L, H, 64) fp32 contiguous
   float* gnum;             // (B, L, H, 64) fp32 contiguous
   float* gden;             // (B, H, L)
-  float* ga_row;           // (B, H, L)
+  float* ga_row;           // (B, H, L) with a_rows
+  float* ga_blk;           // (B, H, Mb) with alpha: the same summed over the block's rows
   RowPtr gos;              // bf16 out
-  int L, H, Mb, qblk;
+  int L, H, Mb, qblk, alpha_ld;
 };
 
 __global__ void __launch_bounds__(256) lin_bwd_rows_kernel(const BwdRowsArgs a) {
@@ -437,10 +447,12 @@ __global__ void __launch_bounds__(256) lin_bwd_rows_kernel(const BwdRowsArgs a) 
   float* P = Ct + 64 * LP;            // phi rows
   float* G = P + 64 * LP;             // g_num rows
   float* S = G;                       // result tile of the products (G is dead at both times)
-  __shared__ float Den[64], GD[64];
+  __shared__ float Den[64], GD[64], GA[64];
   const int m = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   load_state(C, a.C + (((int64_t)b * a.H + h) * a.Mb + m) * LSTATE, tid);
+  const float al_blk = a.alpha ? sigmoid_at(a.alpha, (int64_t)h * a.alpha_ld + m) : 0.f;
+  float ga_sum = 0.f;                 // warp 0
   __syncthreads();
   transpose_state(Ct, C, tid);
   const float z0 = C[(2 * lane) * LP + 64], z1 = C[(2 * lane + 1) * LP + 64];
@@ -482,7 +494,7 @@ __global__ void __launch_bounds__(256) lin_bwd_rows_kernel(const BwdRowsArgs a) 
       float gn[4] = {0.f, 0.f, 0.f, 0.f};
       float uo = 0.f, ga = 0.f, al = 0.f;
       if (live) {
-        al = a.a_rows[(int64_t)h * a.L + row];
+        al = a.alpha ? al_blk : a.a_rows[(int64_t)h * a.L + row];
         float g[4], s[4];
         ld_bf16x4(row_at(a.go, b, row, h) + c0, g);
         ld_bf16x4(row_at(a.os, b, row, h) + c0, s);
@@ -504,14 +516,16 @@ __global__ void __launch_bounds__(256) lin_bwd_rows_kernel(const BwdRowsArgs a) 
       if (tx == 0) {
         const float g_den = -uo * inv;
         GD[r0 + i] = g_den;
+        GA[r0 + i] = live ? al * (1.f - al) * ga : 0.f;
         if (live) {
           const int64_t so = ((int64_t)b * a.H + h) * a.L + row;
           a.gden[so] = g_den;
-          a.ga_row[so] = al * (1.f - al) * ga;
+          if (a.ga_row) a.ga_row[so] = GA[r0 + i];
         }
       }
     }
     __syncthreads();
+    if (a.ga_blk && warp == 0) ga_sum += warp_sum(GA[lane] + GA[lane + 32]);
     float gp[4][4] = {};
     {
       float fr[4][4] = {};
@@ -537,6 +551,7 @@ __global__ void __launch_bounds__(256) lin_bwd_rows_kernel(const BwdRowsArgs a) 
                         ps[2] * (gp[i][2] - dot), ps[3] * (gp[i][3] - dot));
     }
   }
+  if (a.ga_blk && tid == 0) a.ga_blk[((int64_t)b * a.H + h) * a.Mb + m] = ga_sum;
 }
 
 // --------------------------------------------------------------------------
@@ -695,14 +710,6 @@ static RowPtr row_ptr(const void* p, const int64_t* st) {
   return r;
 }
 
-template <typename K>
-static int set_smem(K kern, size_t bytes) {
-  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) ==
-                 cudaSuccess
-             ? 0
-             : -3;
-}
-
 }  // namespace imf
 
 using namespace imf;
@@ -726,7 +733,8 @@ extern "C" int imf_comp_mask(const int* sel, void* cm, int BH, int Mb, int Nb, i
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
-// strides: x(3), dx(3), y(3), dy(3) element strides (batch, row, head).
+// strides: x(3), dx(3), y(3), dy(3) element strides (batch, row, head).  Blocks without rows below
+// `lim` (the padding up to nblk_pad among them) get zero states.
 extern "C" int imf_lin_states(const void* x, const void* dx, const void* y, const void* dy,
                               const float* w, void* out, void* dout, int B, int L, int H, int bs,
                               int nblk, int nblk_pad, int lim, int y_fp32, const int64_t* strides,
@@ -742,10 +750,11 @@ extern "C" int imf_lin_states(const void* x, const void* dx, const void* y, cons
   a.dout = static_cast<__nv_bfloat16*>(dout);
   a.L = L; a.H = H; a.bs = bs; a.nblk_pad = nblk_pad; a.lim = lim < L ? lim : L; a.y_fp32 = y_fp32;
   a.tangent = dx != nullptr;
-  const dim3 grid(nblk, H, B);
+  const dim3 grid(nblk_pad, H, B);
   const size_t tile = (size_t)64 * LP * sizeof(float);      // X, Y (+ dX, dY with a tangent)
   if (dx) {
-    if (set_smem(lin_states_kernel<true>, 4 * tile)) return -3;
+    static bool done[HOST_MAX_DEVICES] = {false};
+    if (!allow_smem((const void*)lin_states_kernel<true>, 4 * tile, done)) return -3;
     lin_states_kernel<true><<<grid, 256, 4 * tile, (cudaStream_t)stream>>>(a);
   } else {
     lin_states_kernel<false><<<grid, 256, 2 * tile, (cudaStream_t)stream>>>(a);
@@ -755,10 +764,11 @@ extern "C" int imf_lin_states(const void* x, const void* dx, const void* y, cons
 
 // strides: q(3), dq(3), os(3), dos(3), o(3), dout(3).
 extern "C" int imf_lin_apply(const void* q, const void* dq, const void* os, const void* dos,
-                             const float* C, const float* dC, const float* a_rows, void* o,
-                             void* dout, int B, int L, int H, int Mb, int qblk,
-                             const int64_t* strides, void* stream) {
-  if (qblk % 64 || B <= 0) return -1;
+                             const float* C, const float* dC, const float* a_rows,
+                             const float* alpha, int alpha_ld, void* o, void* dout, int B, int L,
+                             int H, int Mb, int qblk, const int64_t* strides, void* stream) {
+  if (qblk % 64 || B <= 0 || (a_rows == nullptr) == (alpha == nullptr) || (alpha && alpha_ld < Mb))
+    return -1;
   const void* ptrs[6] = {q, dq, os, dos, o, dout};
   if (!rows_vec4_ok(ptrs, 6, strides)) return -2;
   ApplyArgs a;
@@ -768,12 +778,13 @@ extern "C" int imf_lin_apply(const void* q, const void* dq, const void* os, cons
   a.dos = row_ptr(dos, strides + 9);
   a.o = row_ptr(o, strides + 12);
   a.dout = row_ptr(dout, strides + 15);
-  a.C = C; a.dC = dC; a.a_rows = a_rows;
+  a.C = C; a.dC = dC; a.a_rows = a_rows; a.alpha = alpha; a.alpha_ld = alpha_ld;
   a.L = L; a.H = H; a.Mb = Mb; a.qblk = qblk;
   const dim3 grid(Mb, H, B);
   const size_t base = (size_t)(LSTATE + 64 * LP) * sizeof(float);
   if (dq) {
-    if (set_smem(lin_apply_kernel<true>, 2 * base)) return -3;
+    static bool done[HOST_MAX_DEVICES] = {false};
+    if (!allow_smem((const void*)lin_apply_kernel<true>, 2 * base, done)) return -3;
     lin_apply_kernel<true><<<grid, 256, 2 * base, (cudaStream_t)stream>>>(a);
   } else {
     lin_apply_kernel<false><<<grid, 256, base, (cudaStream_t)stream>>>(a);
@@ -783,10 +794,11 @@ extern "C" int imf_lin_apply(const void* q, const void* dq, const void* os, cons
 
 // strides: q(3), os(3), go(3), gos(3).  gq / gnum: (B, L, H, 64) fp32 contiguous.
 extern "C" int imf_lin_bwd_rows(const void* q, const void* os, const void* go, const float* C,
-                                const float* a_rows, float* gq, float* gnum, float* gden,
-                                float* ga_row, void* gos, int B, int L, int H, int Mb, int qblk,
-                                const int64_t* strides, void* stream) {
-  if (qblk % 64 || B <= 0) return -1;
+                                const float* a_rows, const float* alpha, int alpha_ld, float* gq,
+                                float* gnum, float* gden, float* ga, void* gos, int B, int L, int H,
+                                int Mb, int qblk, const int64_t* strides, void* stream) {
+  if (qblk % 64 || B <= 0 || (a_rows == nullptr) == (alpha == nullptr) || (alpha && alpha_ld < Mb))
+    return -1;
   const void* ptrs[4] = {q, os, go, gos};
   if (!rows_vec4_ok(ptrs, 4, strides)) return -2;
   BwdRowsArgs a;
@@ -794,10 +806,12 @@ extern "C" int imf_lin_bwd_rows(const void* q, const void* os, const void* go, c
   a.os = row_ptr(os, strides + 3);
   a.go = row_ptr(go, strides + 6);
   a.gos = row_ptr(gos, strides + 9);
-  a.C = C; a.a_rows = a_rows; a.gq = gq; a.gnum = gnum; a.gden = gden; a.ga_row = ga_row;
+  a.C = C; a.a_rows = a_rows; a.gq = gq; a.gnum = gnum; a.gden = gden;
+  a.alpha = alpha; a.alpha_ld = alpha_ld; a.ga_row = alpha ? nullptr : ga; a.ga_blk = alpha ? ga : nullptr;
   a.L = L; a.H = H; a.Mb = Mb; a.qblk = qblk;
   const size_t smem = (size_t)(LSTATE + 3 * 64 * LP) * sizeof(float);
-  if (set_smem(lin_bwd_rows_kernel, smem)) return -3;
+  static bool done[HOST_MAX_DEVICES] = {false};
+  if (!allow_smem((const void*)lin_bwd_rows_kernel, smem, done)) return -3;
   lin_bwd_rows_kernel<<<dim3(Mb, H, B), 256, smem, (cudaStream_t)stream>>>(a);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
@@ -818,7 +832,8 @@ extern "C" int imf_lin_bwd_kv(const void* k, const void* v, const void* gks, con
   a.gv = row_ptr(gv, strides + 15);
   a.gS = gS; a.L = L; a.H = H; a.Nb = Nb; a.lim = lim < L ? lim : L;
   const size_t smem = (size_t)(LSTATE + 3 * 64 * LP) * sizeof(float);
-  if (set_smem(lin_bwd_kv_kernel, smem)) return -3;
+  static bool done[HOST_MAX_DEVICES] = {false};
+  if (!allow_smem((const void*)lin_bwd_kv_kernel, smem, done)) return -3;
   lin_bwd_kv_kernel<<<dim3(Nb, H, B), 256, smem, (cudaStream_t)stream>>>(a);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }

@@ -212,11 +212,21 @@ kv_pair_lists_kernel(const uint8_t* __restrict__ fm, int* __restrict__ qlist,
 // out (B, H, nb, 64) fp32, mean over the valid rows of each block.  Fixed
 // summation order (rows of a warp in sequence, then the warps in sequence).
 // --------------------------------------------------------------------------
-__global__ void __launch_bounds__(RT_THREADS)
-pool_blocks_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, int64_t sb,
-                   int64_t sl, int64_t sh, int L, int block, int nb) {
+struct PoolArgs {
+  const __nv_bfloat16* x;
+  float* out;
+  int64_t sb, sl, sh;
+  int L, block, nb;
+};
+// one or two tensors (q and k of an attention call) in one launch: grid.x = p0.nb + p1.nb
+__global__ void __launch_bounds__(RT_THREADS) pool_blocks_kernel(const PoolArgs p0, const PoolArgs p1) {
   __shared__ float2 part[RT_THREADS / 32][32];
-  const int n = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const bool second = (int)blockIdx.x >= p0.nb;
+  const __nv_bfloat16* x = second ? p1.x : p0.x;
+  float* out = second ? p1.out : p0.out;
+  const int64_t sb = second ? p1.sb : p0.sb, sl = second ? p1.sl : p0.sl, sh = second ? p1.sh : p0.sh;
+  const int L = second ? p1.L : p0.L, block = second ? p1.block : p0.block, nb = second ? p1.nb : p0.nb;
+  const int n = blockIdx.x - (second ? p0.nb : 0), h = blockIdx.y, b = blockIdx.z;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r0 = n * block, r1 = min(L, r0 + block);
   const __nv_bfloat16* base = x + b * sb + h * sh + 2 * lane;
@@ -412,13 +422,23 @@ route_topk_kernel(const float* __restrict__ qb, const float* __restrict__ kb,
 
 using namespace imf;
 
-extern "C" int imf_pool_blocks(const void* x, float* out, int B, int L, int H, int block, int nb,
-                               int64_t sb, int64_t sl, int64_t sh, void* stream) {
-  if (B <= 0 || H <= 0 || L <= 0 || block <= 0 || nb <= 0 || (int64_t)(nb - 1) * block >= L)
-    return -1;
-  if ((reinterpret_cast<uintptr_t>(x) & 3) || ((sb | sl | sh) & 1)) return -2;
-  pool_blocks_kernel<<<dim3(nb, H, B), RT_THREADS, 0, (cudaStream_t)stream>>>(
-      static_cast<const __nv_bfloat16*>(x), out, sb, sl, sh, L, block, nb);
+static int pool_args(PoolArgs& a, const void* x, float* out, int L, int block, int nb, const int64_t* st) {
+  if (L <= 0 || block <= 0 || nb <= 0 || (int64_t)(nb - 1) * block >= L) return -1;
+  if ((reinterpret_cast<uintptr_t>(x) & 3) || ((st[0] | st[1] | st[2]) & 1)) return -2;
+  a = PoolArgs{static_cast<const __nv_bfloat16*>(x), out, st[0], st[1], st[2], L, block, nb};
+  return 0;
+}
+
+// `strides`: (batch, row, head) of x, then of x2.  x2 may be null (one tensor).
+extern "C" int imf_pool_blocks(const void* x, float* out, int L, int block, int nb, const void* x2,
+                               float* out2, int L2, int block2, int nb2, int B, int H,
+                               const int64_t* strides, void* stream) {
+  if (B <= 0 || H <= 0) return -1;
+  PoolArgs a, a2 = {};
+  int rc = pool_args(a, x, out, L, block, nb, strides);
+  if (rc == 0 && x2) rc = pool_args(a2, x2, out2, L2, block2, nb2, strides + 3);
+  if (rc) return rc;
+  pool_blocks_kernel<<<dim3(a.nb + a2.nb, H, B), RT_THREADS, 0, (cudaStream_t)stream>>>(a, a2);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 

@@ -29,9 +29,9 @@ if AVAILABLE:
     _lib.imf_lin_states.restype = ci
     _lib.imf_lin_states.argtypes = [vp] * 7 + [ci] * 8 + [vp, vp]
     _lib.imf_lin_apply.restype = ci
-    _lib.imf_lin_apply.argtypes = [vp] * 9 + [ci] * 5 + [vp, vp]
+    _lib.imf_lin_apply.argtypes = [vp] * 8 + [ci] + [vp] * 2 + [ci] * 5 + [vp, vp]
     _lib.imf_lin_bwd_rows.restype = ci
-    _lib.imf_lin_bwd_rows.argtypes = [vp] * 10 + [ci] * 5 + [vp, vp]
+    _lib.imf_lin_bwd_rows.argtypes = [vp] * 6 + [ci] + [vp] * 5 + [ci] * 5 + [vp, vp]
     _lib.imf_lin_bwd_kv.restype = ci
     _lib.imf_lin_bwd_kv.argtypes = [vp] * 7 + [ci] * 5 + [vp, vp]
     if K._has("imf_comp_mask"):
@@ -91,9 +91,8 @@ def states(x, dx, y, dy, w, bs: int, lim: int) -> Tuple[torch.Tensor, Optional[t
     assert D == 64 and x.dtype == torch.bfloat16
     nblk = -(-L // bs)
     nbp = _pad4(nblk)
-    mk = torch.zeros if nbp != nblk else torch.empty
-    out = mk(B * H, 2 * nbp, LSTATE, dtype=torch.bfloat16, device=x.device)
-    dout = mk(B * H, 2 * nbp, LSTATE, dtype=torch.bfloat16, device=x.device) if dx is not None else None
+    out = torch.empty(B * H, 2 * nbp, LSTATE, dtype=torch.bfloat16, device=x.device)
+    dout = torch.empty_like(out) if dx is not None else None
     y_fp32 = y.dtype == torch.float32
     assert y_fp32 or y.dtype == torch.bfloat16
     if w is not None:
@@ -106,9 +105,19 @@ def states(x, dx, y, dy, w, bs: int, lim: int) -> Tuple[torch.Tensor, Optional[t
     return out, dout
 
 
+def _mixing(a_rows, alpha, H: int, L: int, Mb: int):
+    """(a_rows, alpha, alpha_ld) for the launchers: the mixing ratio per row, (H, L), or logits per
+    query block, (H, at least Mb), whose sigmoid the kernels take."""
+    assert (a_rows is None) != (alpha is None)
+    t = (a_rows if alpha is None else alpha).detach().float().contiguous()
+    assert t.shape[0] == H and (t.shape[1] == L if alpha is None else t.shape[1] >= Mb)
+    return (t, None, 0) if alpha is None else (None, t, t.shape[1])
+
+
 def forward(q, k, v, dq, dk, dv, o_s, do_s, sel, a_rows, qblk: int, bk: int,
-            n_comp: Optional[int]):
-    """o = a o_s + (1 - a) o_l (and its tangent).  Returns (o, do, C) with C the
+            n_comp: Optional[int], alpha: Optional[torch.Tensor] = None):
+    """o = a o_s + (1 - a) o_l (and its tangent), a = ``a_rows`` (H, L) or, where that is None,
+    sigmoid(``alpha``) (H, query blocks).  Returns (o, do, C) with C the
     ``(B*H, Mb, LSTATE)`` fp32 complement states (kept for reverse mode)."""
     B, L, H, D = q.shape
     Mb, Nb = -(-L // qblk), -(-L // bk)
@@ -118,35 +127,37 @@ def forward(q, k, v, dq, dk, dv, o_s, do_s, sel, a_rows, qblk: int, bk: int,
     cm2 = comp_mask(sel, Mb, Nb)
     C = K.gemm_batched(cm2, S2, b_mn=True, out_dtype=torch.float32)
     dC = K.gemm_batched(cm2, dS2, b_mn=True, out_dtype=torch.float32) if tangent else None
-    a_rows = a_rows.detach().float().contiguous()
+    a_rows, alpha, ald = _mixing(a_rows, alpha, H, L, Mb)
     o = torch.empty(B, L, H, D, dtype=torch.bfloat16, device=q.device)
     do = torch.empty_like(o) if tangent else None
     rc = _lib.imf_lin_apply(K._ptr(q), K._ptr(dq), K._ptr(o_s), K._ptr(do_s), K._ptr(C),
-                            K._ptr(dC), K._ptr(a_rows), K._ptr(o), K._ptr(do), B, L, H, Mb, qblk,
-                            _strides(q, dq, o_s, do_s, o, do), K._stream())
+                            K._ptr(dC), K._ptr(a_rows), K._ptr(alpha), ald, K._ptr(o), K._ptr(do), B,
+                            L, H, Mb, qblk, _strides(q, dq, o_s, do_s, o, do), K._stream())
     K._check(rc, "imf_lin_apply")
     K.LAUNCHES.count += 1
     return o, do, C
 
 
-def backward_rows(q, o_s, go, C, a_rows, qblk: int):
-    """Row side of reverse mode.  Returns (gq_l fp32, gnum fp32, gden, ga_row, g_os bf16)."""
+def backward_rows(q, o_s, go, C, a_rows, qblk: int, alpha: Optional[torch.Tensor] = None):
+    """Row side of reverse mode.  Returns (gq_l fp32, gnum fp32, gden, ga, g_os bf16); ga is the
+    gradient of the mixing logit of each row (B, H, L) with ``a_rows``, of each query block
+    (B, H, Mb) with ``alpha`` (see ``forward``)."""
     B, L, H, D = q.shape
     Mb = -(-L // qblk)
     dev = q.device
     gq = torch.empty(B, L, H, D, dtype=torch.float32, device=dev)
     gnum = torch.empty(B, L, H, D, dtype=torch.float32, device=dev)
     gden = torch.empty(B, H, L, dtype=torch.float32, device=dev)
-    ga_row = torch.empty(B, H, L, dtype=torch.float32, device=dev)
+    a_rows, alpha, ald = _mixing(a_rows, alpha, H, L, Mb)
+    ga = torch.empty(B, H, L if alpha is None else Mb, dtype=torch.float32, device=dev)
     g_os = torch.empty(B, L, H, D, dtype=torch.bfloat16, device=dev)
-    a_rows = a_rows.detach().float().contiguous()
     rc = _lib.imf_lin_bwd_rows(K._ptr(q), K._ptr(o_s), K._ptr(go), K._ptr(C), K._ptr(a_rows),
-                               K._ptr(gq), K._ptr(gnum), K._ptr(gden), K._ptr(ga_row),
+                               K._ptr(alpha), ald, K._ptr(gq), K._ptr(gnum), K._ptr(gden), K._ptr(ga),
                                K._ptr(g_os), B, L, H, Mb, qblk, _strides(q, o_s, go, g_os),
                                K._stream())
     K._check(rc, "imf_lin_bwd_rows")
     K.LAUNCHES.count += 1
-    return gq, gnum, gden, ga_row, g_os
+    return gq, gnum, gden, ga, g_os
 
 
 def backward_kv(q, k, v, gnum, gden, sel, gk_s, gv_s, qblk: int, bk: int, n_comp: Optional[int],

@@ -40,23 +40,41 @@ if K._has("imf_build_tile_lut"):
 ROUTER_KERNELS = K._has("imf_route_topk")
 if ROUTER_KERNELS:
     _lib.imf_pool_blocks.restype = ci
-    _lib.imf_pool_blocks.argtypes = [vp, vp] + [ci] * 5 + [c64] * 3 + [vp]
+    _lib.imf_pool_blocks.argtypes = [vp, vp, ci, ci, ci] * 2 + [ci, ci, vp, vp]
     _lib.imf_route_topk.restype = ci
     _lib.imf_route_topk.argtypes = [vp] * 6 + [ci] * 8 + [cf, vp]
+
+
+def _pool(items):
+    """One launch for one or two (x, block, nb): see ``pool_blocks``."""
+    args, strides, outs = [], [], []
+    for x, block, nb in items:
+        B, H, L, D = x.shape
+        assert D == 64 and x.dtype == torch.bfloat16 and x.stride(3) == 1
+        nb = -(-L // block) if nb is None else nb
+        outs.append(torch.empty(B, H, nb, D, dtype=torch.float32, device=x.device))
+        args += [x.data_ptr(), outs[-1].data_ptr(), min(L, nb * block), block, nb]
+        sb, sh, sl, _ = x.stride()
+        strides += [sb, sl, sh]
+    if len(items) == 1:
+        args += [None, None, 0, 0, 0]
+    B, H = items[0][0].shape[:2]
+    K._check(_lib.imf_pool_blocks(*args, B, H, (c64 * len(strides))(*strides), K._stream()),
+             "imf_pool_blocks")
+    K.LAUNCHES.count += 1
+    return outs
 
 
 def pool_blocks(x: torch.Tensor, block: int, nb: Optional[int] = None) -> torch.Tensor:
     """Means of the first ``nb`` blocks of ``block`` rows (ragged last block: mean of its
     valid rows).  x: (B, H, L, 64) bf16 view with a contiguous last dim -> (B, H, nb, 64) fp32."""
-    B, H, L, D = x.shape
-    assert D == 64 and x.dtype == torch.bfloat16 and x.stride(3) == 1
-    nb = -(-L // block) if nb is None else nb
-    out = torch.empty(B, H, nb, D, dtype=torch.float32, device=x.device)
-    K._check(_lib.imf_pool_blocks(K._ptr(x), K._ptr(out), B, min(L, nb * block), H, block, nb,
-                                  x.stride(0), x.stride(2), x.stride(1), K._stream()),
-             "imf_pool_blocks")
-    K.LAUNCHES.count += 1
-    return out
+    return _pool([(x, block, nb)])[0]
+
+
+def pool_blocks_qk(q: torch.Tensor, bq: int, k: torch.Tensor, bk: int, nk: Optional[int] = None):
+    """``pool_blocks(q, bq), pool_blocks(k, bk, nk)`` in one launch."""
+    assert q.shape[:2] == k.shape[:2]
+    return _pool([(q, bq, None), (k, bk, nk)])
 
 
 def route_topk(qb: torch.Tensor, kb: torch.Tensor, T: int, proj_q: Optional[torch.Tensor] = None,

@@ -302,6 +302,39 @@ def test_linear_branch_kernels_match_formulas():
     assert rel(gv, gv_r.permute(0, 2, 1, 3)) < 6e-3
 
 
+@pytest.mark.parametrize("B,L,qblk,extra", [(1, 583, 64, 0), (2, 640, 128, 2), (1, 130, 128, 0)])
+def test_linear_branch_mixing_logits_per_block(SP, B, L, qblk, extra):
+    """Mixing logits per query block (sigmoid and the row sums of their gradient in the kernels)
+    against the ratio per row: the same arithmetic but for one fp32 sigmoid (2^-22) and the order
+    of a sum of at most 128 rows; states of a padded block count start from unwritten memory."""
+    from imfvideo_b200.ops import linattn as LA
+
+    torch.manual_seed(L)
+    H = 3
+    mk = lambda: torch.randn(B, L, H, 64, device="cuda").bfloat16()
+    q, k, v, o_s, do_s, dq, dk, dv, go = (mk() for _ in range(9))
+    Mb, Nb = -(-L // qblk), -(-L // 64)
+    sel = torch.rand(B, H, Mb, Nb, device="cuda").argsort(-1)[..., :max(1, Nb // 4)].int().contiguous()
+    alpha = torch.randn(H, Mb + extra, device="cuda")
+    rows = torch.sigmoid(alpha).repeat_interleave(qblk, dim=-1)[:, :L]
+    torch.empty(1 << 24, device="cuda").fill_(float("nan"))     # what the allocator hands out next
+    a = LA.forward(q, k, v, dq, dk, dv, o_s, do_s, sel, None, qblk, 64, None, alpha=alpha)
+    b = LA.forward(q, k, v, dq, dk, dv, o_s, do_s, sel, rows, qblk, 64, None)
+    for x, y in zip(a, b):
+        assert torch.isfinite(x).all() and _rel(x, y) < 1e-3      # bf16 results: ties at most
+    ga = LA.backward_rows(q, o_s, go, a[2], None, qblk, alpha=alpha)
+    gr = LA.backward_rows(q, o_s, go, a[2], rows, qblk)
+    for x, y in ((ga[0], gr[0]), (ga[1], gr[1]), (ga[2], gr[2]), (ga[4], gr[4])):
+        assert _rel(x, y) < 1e-3
+    want = torch.nn.functional.pad(gr[3], (0, Mb * qblk - L)).view(B, H, Mb, qblk).double().sum(-1)
+    assert ga[3].shape == want.shape
+    assert (ga[3] - want).abs().max() <= 128 * 2 ** -22 * gr[3].abs().max() * 128
+    q2, k2 = (x.permute(0, 2, 1, 3) for x in (q, k))
+    for nk in (None, max(1, Nb - 1)):
+        got = SP.pool_blocks_qk(q2, qblk, k2, 64, nk)
+        assert torch.equal(got[0], SP.pool_blocks(q2, qblk)) and torch.equal(got[1], SP.pool_blocks(k2, 64, nk))
+
+
 @pytest.mark.parametrize("qblk", [64, 128])
 def test_device_routing_tables_match_torch_builders(SP, qblk):
     torch.manual_seed(5)
