@@ -136,9 +136,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
     for (int t = 0; t < C::NT; ++t) {
       mbar_init(&s.s_full[t], 1);
-      mbar_init(&s.p_full[t], ATT_TILE_M);
+      mbar_init(&s.p_full[t], 4);      // one arrival per softmax warp
       mbar_init(&s.o_done[t], 1);
-      mbar_init(&s.o_free[t], ATT_TILE_M);
+      mbar_init(&s.o_free[t], 4);
     }
     s.abort_flag = 0;
     fence_barrier_init();
@@ -248,7 +248,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           for (int t = 0; t < C::NT; ++t) issue_qk(t, (int)(kv_it % C::STAGES), &s.s_full[t]);
           if (n_j == 1) tc_commit(&s.q_empty);
           for (int jj = 0; jj < n_j && ok; ++jj, ++kv_it, ++it) {
-            const int st = (int)(kv_it % C::STAGES);
+            const int st = (int)(kv_it % C::STAGES), st1 = (int)((kv_it + 1) % C::STAGES);
+            // the next K/V tile, loaded long ago: seen now, not between P V and the next Q K^T (a
+            // wait costs some 200 clocks even when there is nothing to wait for)
+            if (jj + 1 < n_j) {
+              ok = mbar_wait(&s.kv_full[st1], (uint32_t)(((kv_it + 1) / C::STAGES) & 1), abort_flag,
+                             p.status, STATUS_TIMEOUT_TMA);
+              if (!ok) break;
+            }
 #pragma unroll
             for (int t = 0; t < C::NT; ++t) {
               if (!ok) break;
@@ -262,14 +269,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               issue_pv(t, st, jj == 0);
               if (t == C::NT - 1) tc_commit(&s.kv_empty[st]);
               if (jj + 1 < n_j) {
-                const long nk = kv_it + 1;
-                const int st1 = (int)(nk % C::STAGES);
-                if (t == 0) {
-                  ok = mbar_wait(&s.kv_full[st1], (uint32_t)((nk / C::STAGES) & 1), abort_flag,
-                                 p.status, STATUS_TIMEOUT_TMA);
-                  if (!ok) break;
-                  tc_fence_after();
-                }
                 issue_qk(t, st1, &s.s_full[t]);
                 if (t == C::NT - 1 && jj + 2 == n_j) tc_commit(&s.q_empty);   // last Q read of the item
               }
@@ -466,7 +465,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         tc_wait_st();
         tc_fence_before();
-        mbar_arrive(&s.p_full[t]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s.p_full[t]);
       }
       // ---- epilogue of this segment ----
       if (ok)
@@ -537,7 +537,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         stats[2 * C::ITEM_M + row_in_item] = mu_tot;
       }
       tc_fence_before();
-      mbar_arrive(&s.o_free[t]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s.o_free[t]);
     }
     tc_fence_before();
   }

@@ -131,11 +131,11 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     for (int t = 0; t < C::NT; ++t) {
       for (int b = 0; b < C::SBUF; ++b) {
         mbar_init(&s.s_full[t][b], 1);
-        mbar_init(&s.p_full[t][b], C::ROW_THREADS);
+        mbar_init(&s.p_full[t][b], C::ROW_THREADS / 32);
       }
       mbar_init(&s.o_done[t], 1);
       mbar_init(&s.o_final[t], 1);
-      mbar_init(&s.o_free[t], C::ROW_THREADS);
+      mbar_init(&s.o_free[t], C::ROW_THREADS / 32);
     }
     mbar_init(&s.xbar, C::SOFT_WARPS);
     s.abort_flag = 0;
@@ -309,6 +309,11 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
               const int st = (int)(kv_it % C::STAGES);
               ok = mbar_wait(&s.v_full[st], (uint32_t)((kv_it / C::STAGES) & 1), abort_flag, p.status,
                              STATUS_TIMEOUT_TMA);
+              // the next K tile, loaded long ago: seen now, not between P V and the next Q K^T
+              const int st1 = (int)((kv_it + 1) % C::STAGES);
+              if (ok && jj + 1 < n_j)
+                ok = mbar_wait(&s.k_full[st1], (uint32_t)(((kv_it + 1) / C::STAGES) & 1), abort_flag,
+                               p.status, STATUS_TIMEOUT_TMA);
 #pragma unroll
               for (int t = 0; t < C::NT; ++t) {
                 if (!ok) break;
@@ -322,14 +327,6 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 issue_pv(t, 0, st, jj == 0, jj + 1 == n_j);
                 if (t == C::NT - 1) tc_commit(&s.v_empty[st]);
                 if (jj + 1 < n_j) {
-                  const long nk = kv_it + 1;
-                  const int st1 = (int)(nk % C::STAGES);
-                  if (t == 0) {
-                    ok = mbar_wait(&s.k_full[st1], (uint32_t)((nk / C::STAGES) & 1), abort_flag,
-                                   p.status, STATUS_TIMEOUT_TMA);
-                    if (!ok) break;
-                    tc_fence_after();
-                  }
                   const uint32_t tb = tmem + t * C::TILE_COLS;
                   const uint32_t qa = smem_u32(s.q[0][t]), ka = smem_u32(s.k[st1][0]);
 #pragma unroll
@@ -472,7 +469,8 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         }
         tc_wait_st();
         tc_fence_before();
-        mbar_arrive(&s.p_full[t][buf]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s.p_full[t][buf]);
       }
       // ---- epilogue of this segment ----
       if (ok)
@@ -561,7 +559,8 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         }
       }
       tc_fence_before();
-      mbar_arrive(&s.o_free[t]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s.o_free[t]);
     }
     tc_fence_before();
   }
