@@ -213,7 +213,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
       // The additive source (bf16) is read 32 columns ahead of its use, the first ones while the
       // tile's products still run: a read waits for L2, and with one after the other in line the
       // epilogue took longer than the tile's products (24 x 1,024 x 1,024, five times X X^T and
-      // b A + c A A: 445 -> 425 us).
+      // b A + c A A: 445 -> 425 us, and 376 us once it was added without a test per element).
       uint32_t cv[16], cv_next[16];
       bool have_cin = false, have_next = false;
       auto read_cin = [&](int c) {
@@ -266,6 +266,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
               for (int i = 0; i < 16; ++i)
                 o[i] = pack_bf16(__uint_as_float(r[2 * i]) * alpha,
                                  __uint_as_float(r[2 * i + 1]) * alpha);
+            } else if (have_cin && bias == nullptr) {      // additive source in registers
+#pragma unroll
+              for (int i = 0; i < 16; ++i)
+                o[i] = pack_bf16(fmaf(beta, bf16_lo(cv[i]), __uint_as_float(r[2 * i]) * alpha),
+                                 fmaf(beta, bf16_hi(cv[i]), __uint_as_float(r[2 * i + 1]) * alpha));
             } else
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
@@ -288,11 +293,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CU
               // mirror image of an off-diagonal tile: element (row, col) also goes to (col, row);
               // for a fixed column the 32 lanes write 32 consecutive bf16 of one row of C
               uint16_t* Ct = reinterpret_cast<uint16_t*>(C);
+              uint16_t* dst = Ct + (int64_t)(n0 + c) * ldc + row;
+              if (n0 + c + 32 <= N) {
 #pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                const int col = n0 + c + 2 * i;
-                if (col < N) Ct[(int64_t)col * ldc + row] = (uint16_t)(o[i] & 0xffffu);
-                if (col + 1 < N) Ct[(int64_t)(col + 1) * ldc + row] = (uint16_t)(o[i] >> 16);
+                for (int i = 0; i < 16; ++i) {
+                  dst[0] = (uint16_t)(o[i] & 0xffffu);
+                  dst[ldc] = (uint16_t)(o[i] >> 16);
+                  dst += 2 * ldc;
+                }
+              } else {
+                for (int i = 0; i < 16; ++i, dst += 2 * ldc) {
+                  const int col = n0 + c + 2 * i;
+                  if (col < N) dst[0] = (uint16_t)(o[i] & 0xffffu);
+                  if (col + 1 < N) dst[ldc] = (uint16_t)(o[i] >> 16);
+                }
               }
             }
             uint8_t* panel = s.c + (c / PANEL_COLS) * (GEMM_BM * 128) + r_in * 128;
@@ -605,6 +619,14 @@ extern "C" int imf_splitk_reduce(const float* partial, int splits, int M, int N,
   return cudaGetLastError() == cudaSuccess ? imf::IMF_OK : imf::IMF_ERR_LAUNCH;
 }
 
+namespace imf {
+// Batched bf16 products from this K on run one CTA per SM with a ring of six stages, shorter ones
+// two CTAs per SM with two stages each, whose second epilogue then counts for more (five
+// Newton-Schulz steps, products only: 24 x 1,024 x 1,024 609 against 727 us; 28 x 1,024 x 528,
+// half of it at K = 528, 439 against 435 us).
+constexpr int BATCHED_DEEP_K = 768;
+}  // namespace imf
+
 // Batched form with an additive source: C[z] = alpha * op(A[z]) op(B[z])^T + beta * Cin[z].
 // sa/sb/sc: batch strides in elements (multiples of 8 for A, B).  Used by the
 // Newton-Schulz iteration (X X^T, b A + c A A, a X + B X as three launches).
@@ -617,20 +639,20 @@ extern "C" int imf_gemm_bf16_batched(const void* A, const void* B, void* C, cons
   if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return IMF_ERR_ARG;
   if ((lda & 7) || (ldb & 7) || (batch > 1 && ((sa & 7) || (sb & 7)))) return IMF_ERR_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-#define IMF_GEMM_CASE(AM, BM_, OT)                                                              \
-  return launch_gemm<128, IMF_GEMM_STAGES(OT), AM, BM_, OT>(                                    \
-      A, B, C, nullptr, M, N, K, lda, ldb, ldc, 0, alpha, 0, status, st, batch, sa, sb, sc, Cin, beta)
-  if (out_fp32) {
-    if (!a_mn && !b_mn) IMF_GEMM_CASE(false, false, float);
-    if (!a_mn && b_mn) IMF_GEMM_CASE(false, true, float);
-    if (a_mn && !b_mn) IMF_GEMM_CASE(true, false, float);
-    IMF_GEMM_CASE(true, true, float);
-  } else {
-    if (!a_mn && !b_mn) IMF_GEMM_CASE(false, false, __nv_bfloat16);
-    if (!a_mn && b_mn) IMF_GEMM_CASE(false, true, __nv_bfloat16);
-    if (a_mn && !b_mn) IMF_GEMM_CASE(true, false, __nv_bfloat16);
-    IMF_GEMM_CASE(true, true, __nv_bfloat16);
+#define IMF_GEMM_CASE(ST, AM, BM_, OT)                                                            \
+  return launch_gemm<128, ST, AM, BM_, OT>(A, B, C, nullptr, M, N, K, lda, ldb, ldc, 0, alpha, 0, \
+                                           status, st, batch, sa, sb, sc, Cin, beta)
+#define IMF_GEMM_MAJORS(ST, OT)                             \
+  {                                                         \
+    if (!a_mn && !b_mn) IMF_GEMM_CASE(ST, false, false, OT); \
+    if (!a_mn && b_mn) IMF_GEMM_CASE(ST, false, true, OT);  \
+    if (a_mn && !b_mn) IMF_GEMM_CASE(ST, true, false, OT);  \
+    IMF_GEMM_CASE(ST, true, true, OT);                      \
   }
+  if (out_fp32) IMF_GEMM_MAJORS(4, float);
+  if (K >= BATCHED_DEEP_K) IMF_GEMM_MAJORS(6, __nv_bfloat16);
+  IMF_GEMM_MAJORS(2, __nv_bfloat16);
+#undef IMF_GEMM_MAJORS
 #undef IMF_GEMM_CASE
 }
 
@@ -646,13 +668,17 @@ extern "C" int imf_gemm_bf16_batched_sym(const void* A, const void* B, void* C, 
   if ((lda & 7) || (ldb & 7) || (batch > 1 && ((sa & 7) || (sb & 7)))) return IMF_ERR_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   using OT = __nv_bfloat16;
-  if (mn)      // both operands MN-major ([K, M]): X^T X
-    return launch_gemm<128, IMF_GEMM_STAGES(OT), true, true, OT>(
-        A, B, C, nullptr, M, M, K, lda, ldb, ldc, 0, alpha, 0, status, st, batch, sa, sb, sc, Cin,
-        beta, 1, nullptr, 1);
-  return launch_gemm<128, IMF_GEMM_STAGES(OT), false, false, OT>(
-      A, B, C, nullptr, M, M, K, lda, ldb, ldc, 0, alpha, 0, status, st, batch, sa, sb, sc, Cin,
-      beta, 1, nullptr, 1);
+#define IMF_GEMM_SYM(ST, MN)                                                                       \
+  return launch_gemm<128, ST, MN, MN, OT>(A, B, C, nullptr, M, M, K, lda, ldb, ldc, 0, alpha, 0,   \
+                                          status, st, batch, sa, sb, sc, Cin, beta, 1, nullptr, 1)
+  const bool deep = K >= BATCHED_DEEP_K;
+  if (mn) {    // both operands MN-major ([K, M]): X^T X
+    if (deep) IMF_GEMM_SYM(6, true);
+    IMF_GEMM_SYM(2, true);
+  }
+  if (deep) IMF_GEMM_SYM(6, false);
+  IMF_GEMM_SYM(2, false);
+#undef IMF_GEMM_SYM
 }
 
 // ---------------------------------------------------------------------------

@@ -321,6 +321,26 @@ def test_attention_backward_hd128(K, B, L, H):
     K.check_status()
 
 
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("M,N,Kd", [(264, 200, 800), (128, 328, 768), (136, 40, 760)])
+def test_gemm_batched_additive_source(K, a_mn, b_mn, M, N, Kd):
+    """Batched products around the K from which the deep ring is taken, with an additive source
+    whose last 32-column group is whole, ragged or short; one rounding to bf16 of an fp32 sum."""
+    torch.manual_seed(M + N)
+    A = torch.randn(3, M, Kd, device="cuda").bfloat16()
+    B = torch.randn(3, N, Kd, device="cuda").bfloat16()
+    cin = (torch.randn(3, M, N, device="cuda") * 20).bfloat16()
+    op = lambda t, mn: t.transpose(1, 2).contiguous() if mn else t
+    out = K.gemm_batched(op(A, a_mn), op(B, b_mn), a_mn=a_mn, b_mn=b_mn, cin=cin, alpha=0.5, beta=-2.0)
+    ref = 0.5 * A.float() @ B.float().transpose(1, 2) - 2.0 * cin.float()
+    assert _rel(out, ref) < 2.5e-3              # rms of a bf16 rounding: 2^-9 / sqrt(3) at most
+    if a_mn == b_mn and M % 8 == 0:
+        full = K.gemm_batched(op(A, a_mn), op(A, a_mn), a_mn=a_mn, b_mn=a_mn)
+        sym = K.gemm_batched(op(A, a_mn), op(A, a_mn), a_mn=a_mn, b_mn=a_mn, sym=True)
+        assert torch.equal(sym.triu(), full.triu()) and torch.equal(sym, sym.transpose(1, 2))
+    K.check_status()
+
+
 @pytest.mark.parametrize("k,n,m", [(3, 128, 256), (2, 256, 128), (2, 256, 682), (2, 682, 256),
                                    (4, 1, 256), (1, 448, 128), (1, 520, 1024)])
 def test_newton_schulz_kernel(K, k, n, m):
