@@ -508,8 +508,12 @@ class SparseCore:
         # inference form (no reverse mode to follow, e.g. the sampler and the guidance passes):
         # no log-sum-exp, no saved state; the same INT8 block-sparse kernel and the same
         # per-key-block states with the alpha mix fused into the apply kernel
+        # reverse mode differentiates the same quantised operands: kept, not made again (25 us of
+        # 29,140 tokens x 4 heads; three bf16 tensors of the size of q)
+        quant = SP.quantize_qkv(q, k, v, self.qblk, want_fq=need_bwd) if self.int8 else None
+        fq = tuple(x[2] for x in quant) if quant and need_bwd else (None, None, None)
         o_s, do_s, lse = SP.sparse_fwd(q, k, v, dq, dk, dv, lut, flags, self.qblk, self.int8,
-                                       quant_p=self.int8, need_lse=need_bwd, cnt=cnt)
+                                       quant_p=self.int8, need_lse=need_bwd, cnt=cnt, quant=quant)
         flags = fm          # reverse mode needs the (K/V tile, query tile) maps, not the per-tile flags
         from ..ops import linattn as LA
 
@@ -519,7 +523,7 @@ class SparseCore:
                                       self.n_comp, alpha=self._alpha())
                 if need_bwd and isinstance(self.mod, SLA2CubeQATAttentionImpl):
                     self.mod.logit_max_log2 = (lse.amax(dim=(0, 2)) * 1.4426950408889634).float()
-            return o, do, (sel, lut, flags, o_s, lse, C if need_bwd else None)
+            return o, do, (sel, lut, flags, o_s, lse, C if need_bwd else None) + fq
         f = lambda a, b, c: linear_branch(a, b, c, sel, self.qblk, self.bk, self.n_comp)
         a_rows = self._a_rows(q.shape[1])
         with torch.no_grad():
@@ -537,7 +541,7 @@ class SparseCore:
                 do = (a * do_s.float() + (1 - a) * do_l.permute(0, 2, 1, 3)).to(q.dtype).contiguous()
             if need_bwd and isinstance(self.mod, SLA2CubeQATAttentionImpl):
                 self.mod.logit_max_log2 = (lse.amax(dim=(0, 2)) * 1.4426950408889634).float()
-        return o, do, (sel, lut, flags, o_s, lse, None)
+        return o, do, (sel, lut, flags, o_s, lse, None) + fq
 
     def bwd(self, q, k, v, o, saved, go, gv_out=None):
         """o = a o_s + (1 - a) o_l: the sparse branch goes through the block-sparse
@@ -547,7 +551,7 @@ class SparseCore:
         from ..ops import kernels as K
         from ..ops import sparse as SP
 
-        sel, lut, flags, o_s, lse, C = saved
+        sel, lut, flags, o_s, lse, C, *fq = saved
         m = self.mod
         cube = isinstance(m, SLA2CubeQATAttentionImpl)
         alpha_param = m.alpha_logit if cube else m.sla2.alpha_logit
@@ -566,11 +570,7 @@ class SparseCore:
         alpha_param.grad = ga if alpha_param.grad is None else alpha_param.grad + ga
         with torch.no_grad():
             g_os = (a.detach() * gof).to(q.dtype).contiguous()
-            qq, kk, vv = q, k, v
-            if self.int8:
-                _, _, qq = SP.quantize_blocks(K._tma_ok(q), self.qblk, want_q=False, want_fq=True)
-                _, _, kk = SP.quantize_blocks(K._tma_ok(k), 64, want_q=False, want_fq=True)
-                _, _, vv = SP.quantize_blocks(K._tma_ok(v), 64, want_q=False, want_fq=True)
+            qq, kk, vv = fq if self.int8 else (q, k, v)
             gq_s, gk_s, gv_s = K.attn_bwd(qq, kk, vv, o_s, lse, g_os,
                                           **SP.bwd_lists(flags))   # `flags`: the maps (see fwd)
             back = lambda t: t.permute(0, 2, 1, 3)
@@ -591,7 +591,7 @@ def _sparse_core_bwd_kernels(self, q, k, v, saved, go, gv_out, alpha_param, cube
     from ..ops import linattn as LA
     from ..ops import sparse as SP
 
-    sel, lut, flags, o_s, lse, C = saved
+    sel, lut, flags, o_s, lse, C, *fq = saved
     m = self.mod
     B, L, H, D = q.shape
     with torch.no_grad():
@@ -601,14 +601,7 @@ def _sparse_core_bwd_kernels(self, q, k, v, saved, go, gv_out, alpha_param, cube
             ga = F.pad(ga, (0, alpha_param.shape[1] - ga.shape[1]))
         ga = ga.to(alpha_param.dtype)
         alpha_param.grad = ga if alpha_param.grad is None else alpha_param.grad + ga
-        qq, kk, vv = q, k, v
-        if self.int8 and self.qblk == 64:
-            (_, _, qq), (_, _, kk), (_, _, vv) = SP.quantize_blocks_many(
-                [(q, False, True), (k, False, True), (v, False, True)])
-        elif self.int8:
-            _, _, qq = SP.quantize_blocks(K._tma_ok(q), self.qblk, want_q=False, want_fq=True)
-            _, _, kk = SP.quantize_blocks(K._tma_ok(k), 64, want_q=False, want_fq=True)
-            _, _, vv = SP.quantize_blocks(K._tma_ok(v), 64, want_q=False, want_fq=True)
+        qq, kk, vv = fq if self.int8 else (q, k, v)
         # the linear branch's query gradient rides into the block-sparse backward's dQ epilogue
         gq, gk_s, gv_s = K.attn_bwd(qq, kk, vv, o_s, lse, g_os, dq_add=gq_l,
                                     **SP.bwd_lists(flags))         # `flags`: the maps (see fwd)

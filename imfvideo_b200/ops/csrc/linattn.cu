@@ -75,7 +75,7 @@ __device__ __forceinline__ void softmax_row_jvp(float2 phi, float2 dx, float2& d
 // mantissa bits) and fp32 accumulation: the eight warps form a 4 x 2 grid, each with a
 // 16 x 32 piece of the result (four 16 x 8 accumulator fragments).  The results go through a
 // shared-memory tile S so that every thread ends up with the 4 x 4 block
-//     acc[i][j] += sum_k A[r0 + i][k] * Bm[k][c0 + j]        (A_T: A[k][r0 + i])
+//     acc[i][j] += sum_k A[r0 + i][k] * Bm[k][c0 + j]        (A_T: A[k][r0 + i]; B_T: Bm[c0 + j][k])
 // of the 16 x 16 thread grid that the row-wise epilogues of the callers are written for.
 // Fragment layout (g = lane / 4, t = lane % 4): A (row g | g + 8, col t | t + 4),
 // B (k t | t + 4, n g), C (row g | g + 8, col 2 t | 2 t + 1).  Must be called by all 256
@@ -98,8 +98,10 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4],
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// d[n][.] += (A or A^T)[rows mr .. mr + 15][:] * Bm[:][cols nc + 8 n .. + 7], n = 0 .. 3
-template <bool A_T>
+// d[n][.] += (A or A^T)[rows mr .. mr + 15][:] * (Bm or Bm^T)[:][cols nc + 8 n .. + 7], n = 0 .. 3.
+// At pitch 68 the transposed B fragment reads banks 4 g + t, one each: a transposed operand needs
+// no copy of its own.
+template <bool A_T, bool B_T = false>
 __device__ __forceinline__ void warp_mm_tf32(const float* __restrict__ A,
                                              const float* __restrict__ Bm, int mr, int nc,
                                              int g, int t, float (&d)[4][4]) {
@@ -120,8 +122,9 @@ __device__ __forceinline__ void warp_mm_tf32(const float* __restrict__ A,
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
       uint32_t b[2];
-      b[0] = to_tf32(Bm[(k + t) * LP + nc + n * 8 + g]);
-      b[1] = to_tf32(Bm[(k + t + 4) * LP + nc + n * 8 + g]);
+      b[0] = to_tf32(B_T ? Bm[(nc + n * 8 + g) * LP + k + t] : Bm[(k + t) * LP + nc + n * 8 + g]);
+      b[1] = to_tf32(B_T ? Bm[(nc + n * 8 + g) * LP + k + t + 4]
+                         : Bm[(k + t + 4) * LP + nc + n * 8 + g]);
       mma_tf32(d[n], a, b);
     }
   }
@@ -169,8 +172,9 @@ struct StatesArgs {
   int L, H, bs, nblk_pad, lim, y_fp32, tangent;
 };
 
+// (resident CTAs: 29,140 tokens x 4 heads are 1,824 CTAs, 58 us with three to an SM, 56 with four)
 template <bool TANGENT>
-__global__ void __launch_bounds__(256) lin_states_kernel(const StatesArgs a) {
+__global__ void __launch_bounds__(256, TANGENT ? 2 : 4) lin_states_kernel(const StatesArgs a) {
   extern __shared__ __align__(16) float sm[];
   float* X = sm;                     // [64][LP]  phi rows
   float* Y = X + 64 * LP;            // [64][LP]  y rows | w
@@ -287,12 +291,6 @@ __device__ __forceinline__ void load_state(float* dst, const float* src, int tid
     *reinterpret_cast<float4*>(dst + i) = *reinterpret_cast<const float4*>(src + i);
 }
 
-// dst[e][d] = src[d][e] for d, e < 64 (both pitch LP, both in shared memory)
-__device__ __forceinline__ void transpose_state(float* dst, const float* src, int tid) {
-  const int d = tid & 63;
-  for (int e = tid >> 6; e < 64; e += 4) dst[e * LP + d] = src[d * LP + e];
-}
-
 __device__ __forceinline__ __nv_bfloat16* row_at(const RowPtr& t, int b, int row, int h) {
   return static_cast<__nv_bfloat16*>(const_cast<void*>(t.p)) + b * t.sb + (int64_t)row * t.sl +
          h * t.sh;
@@ -329,8 +327,9 @@ __device__ __forceinline__ float sigmoid_at(const float* logits, int64_t i) {
   return 1.f / (1.f + expf(-logits[i]));
 }
 
+// (resident CTAs: 49 us with four to an SM, 45 with five)
 template <bool TANGENT>
-__global__ void __launch_bounds__(256) lin_apply_kernel(const ApplyArgs a) {
+__global__ void __launch_bounds__(256, TANGENT ? 3 : 5) lin_apply_kernel(const ApplyArgs a) {
   extern __shared__ __align__(16) float sm[];
   float* C = sm;                      // [64][LP]: H | z
   float* P = C + LSTATE;              // phi rows [64][LP]
@@ -443,8 +442,7 @@ struct BwdRowsArgs {
 __global__ void __launch_bounds__(256) lin_bwd_rows_kernel(const BwdRowsArgs a) {
   extern __shared__ __align__(16) float sm[];
   float* C = sm;                      // [64 d][LP]: H | z
-  float* Ct = C + LSTATE;             // [64 e][LP]: H^T
-  float* P = Ct + 64 * LP;            // phi rows
+  float* P = C + LSTATE;              // phi rows
   float* G = P + 64 * LP;             // g_num rows
   float* S = G;                       // result tile of the products (G is dead at both times)
   __shared__ float Den[64], GD[64], GA[64];
@@ -454,7 +452,6 @@ __global__ void __launch_bounds__(256) lin_bwd_rows_kernel(const BwdRowsArgs a) 
   const float al_blk = a.alpha ? sigmoid_at(a.alpha, (int64_t)h * a.alpha_ld + m) : 0.f;
   float ga_sum = 0.f;                 // warp 0
   __syncthreads();
-  transpose_state(Ct, C, tid);
   const float z0 = C[(2 * lane) * LP + 64], z1 = C[(2 * lane + 1) * LP + 64];
   const int r0 = (tid >> 4) * 4, c0 = (tid & 15) * 4, tx = tid & 15;
   float zc[4];
@@ -477,7 +474,7 @@ __global__ void __launch_bounds__(256) lin_bwd_rows_kernel(const BwdRowsArgs a) 
       const float den = warp_sum(fmaf(phi.x, z0, phi.y * z1));
       if (lane == 0) Den[rr] = den + LIN_EPS;
     }
-    __syncthreads();                  // also orders the writes of Ct before its first use
+    __syncthreads();
     float num[4][4] = {};
     const MmaPos mp(tid);
     {
@@ -529,7 +526,7 @@ __global__ void __launch_bounds__(256) lin_bwd_rows_kernel(const BwdRowsArgs a) 
     float gp[4][4] = {};
     {
       float fr[4][4] = {};
-      warp_mm_tf32<false>(G, Ct, mp.mr, mp.nc, mp.g, mp.t, fr);       // columns are d here
+      warp_mm_tf32<false, true>(G, C, mp.mr, mp.nc, mp.g, mp.t, fr);      // g_num H^T: columns are d
       frags_to_blocks(fr, S, mp.mr, mp.nc, mp.g, mp.t, r0, c0, gp);
     }
 #pragma unroll
@@ -568,8 +565,7 @@ struct BwdKvArgs {
 __global__ void __launch_bounds__(256) lin_bwd_kv_kernel(const BwdKvArgs a) {
   extern __shared__ __align__(16) float sm[];
   float* C = sm;                      // [64 d][LP]: gH | gz
-  float* Ct = C + LSTATE;             // [64 e][LP]: gH^T
-  float* P = Ct + 64 * LP;            // phi(k) rows
+  float* P = C + LSTATE;              // phi(k) rows
   float* V = P + 64 * LP;             // v rows
   float* S = V;                       // result tile of the products (V is dead by then)
   const int n = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
@@ -596,15 +592,13 @@ __global__ void __launch_bounds__(256) lin_bwd_kv_kernel(const BwdKvArgs a) {
     }
   }
   __syncthreads();
-  transpose_state(Ct, C, tid);
   const int r0 = (tid >> 4) * 4, c0 = (tid & 15) * 4;
   float gv[4][4] = {}, gp[4][4] = {};
   {
     const MmaPos mp(tid);
     float f1[4][4] = {}, f2[4][4] = {};
-    __syncthreads();                  // Ct is complete
     warp_mm_tf32<false>(P, C, mp.mr, mp.nc, mp.g, mp.t, f1);     // g_v, columns e
-    warp_mm_tf32<false>(V, Ct, mp.mr, mp.nc, mp.g, mp.t, f2);    // g_phi, columns d
+    warp_mm_tf32<false, true>(V, C, mp.mr, mp.nc, mp.g, mp.t, f2);     // g_phi = V gH^T, columns d
     frags_to_blocks(f1, S, mp.mr, mp.nc, mp.g, mp.t, r0, c0, gv);
     frags_to_blocks(f2, S, mp.mr, mp.nc, mp.g, mp.t, r0, c0, gp);
   }
@@ -809,7 +803,7 @@ extern "C" int imf_lin_bwd_rows(const void* q, const void* os, const void* go, c
   a.C = C; a.a_rows = a_rows; a.gq = gq; a.gnum = gnum; a.gden = gden;
   a.alpha = alpha; a.alpha_ld = alpha_ld; a.ga_row = alpha ? nullptr : ga; a.ga_blk = alpha ? ga : nullptr;
   a.L = L; a.H = H; a.Mb = Mb; a.qblk = qblk;
-  const size_t smem = (size_t)(LSTATE + 3 * 64 * LP) * sizeof(float);
+  const size_t smem = (size_t)(LSTATE + 2 * 64 * LP) * sizeof(float);
   static bool done[HOST_MAX_DEVICES] = {false};
   if (!allow_smem((const void*)lin_bwd_rows_kernel, smem, done)) return -3;
   lin_bwd_rows_kernel<<<dim3(Mb, H, B), 256, smem, (cudaStream_t)stream>>>(a);
@@ -831,7 +825,7 @@ extern "C" int imf_lin_bwd_kv(const void* k, const void* v, const void* gks, con
   a.gk = row_ptr(gk, strides + 12);
   a.gv = row_ptr(gv, strides + 15);
   a.gS = gS; a.L = L; a.H = H; a.Nb = Nb; a.lim = lim < L ? lim : L;
-  const size_t smem = (size_t)(LSTATE + 3 * 64 * LP) * sizeof(float);
+  const size_t smem = (size_t)(LSTATE + 2 * 64 * LP) * sizeof(float);
   static bool done[HOST_MAX_DEVICES] = {false};
   if (!allow_smem((const void*)lin_bwd_kv_kernel, smem, done)) return -3;
   lin_bwd_kv_kernel<<<dim3(Nb, H, B), 256, smem, (cudaStream_t)stream>>>(a);

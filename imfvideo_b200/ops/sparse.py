@@ -220,6 +220,17 @@ def quantize_blocks_many(items, block: int = 64):
     return outs
 
 
+def quantize_qkv(q, k, v, qblk: int, want_fq: bool = False):
+    """[(int8 | None, scales, de-quantised | None)] of q, k, v on the grid of the sparse branch
+    (query blocks of ``qblk`` rows, key blocks of 64): q and k as int8 and, for reverse mode
+    (``want_fq``), de-quantised too; v de-quantised."""
+    if qblk == 64:
+        return quantize_blocks_many([(q, True, want_fq), (k, True, want_fq), (v, False, True)])
+    return [quantize_blocks(K._tma_ok(q), qblk, want_fq=want_fq),
+            quantize_blocks(K._tma_ok(k), 64, want_fq=want_fq),
+            quantize_blocks(K._tma_ok(v), 64, want_q=False, want_fq=True)]
+
+
 def build_tile_lut(sel: torch.Tensor, qblk: int) -> Tuple[torch.Tensor, torch.Tensor]:
     """Per-128-row query tile list of 64-key blocks from the per-routing-block
     selection ``sel`` (B, H, Mb, T).  qblk 128: one routing block per tile.
@@ -255,21 +266,17 @@ def build_tile_lut(sel: torch.Tensor, qblk: int) -> Tuple[torch.Tensor, torch.Te
 
 def sparse_fwd(q, k, v, dq, dk, dv, lut, flags, qblk: int, int8: bool, quant_p: bool,
                need_lse: bool = True, scale: Optional[float] = None,
-               cnt: Optional[torch.Tensor] = None):
+               cnt: Optional[torch.Tensor] = None, quant=None):
     """Block-sparse softmax branch: (o_s, do_s | None, lse | None).
-    q, k, v (+ tangents): (B, L, H, 64) bf16, token order = routing order."""
+    q, k, v (+ tangents): (B, L, H, 64) bf16, token order = routing order.  ``quant``: what
+    ``quantize_qkv(q, k, v, qblk)`` returned, if the caller has it."""
     B, L, H, D = q.shape
     scale = 1.0 / math.sqrt(D) if scale is None else scale
     tang = dq is not None
     q8 = k8 = qs = ks = None
     vv = K._tma_ok(v)
-    if int8 and qblk == 64:
-        (q8, qs, _), (k8, ks, _), (_, _, vv) = quantize_blocks_many(
-            [(q, True, False), (k, True, False), (vv, False, True)])
-    elif int8:
-        q8, qs, _ = quantize_blocks(K._tma_ok(q), qblk)
-        k8, ks, _ = quantize_blocks(K._tma_ok(k), 64)
-        _, _, vv = quantize_blocks(vv, 64, want_q=False, want_fq=True)
+    if int8:
+        (q8, qs, _), (k8, ks, _), (_, _, vv) = quant or quantize_qkv(q, k, v, qblk)
     ts = [K._tma_ok(q), K._tma_ok(k), vv]
     if tang:
         ts += [K._tma_ok(dq), K._tma_ok(dk), K._tma_ok(dv)]
