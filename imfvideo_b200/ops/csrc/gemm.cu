@@ -567,14 +567,31 @@ extern "C" int imf_gemm_fp8(const void* A, const void* B, void* C, const float* 
 // slices are summed in a fixed order by imf_splitk_reduce, so the result does not depend on
 // which CTA finishes first.  `splits` must satisfy ceil(nkb / ceil(nkb / splits)) == splits for
 // nkb = ceil(K / 64) (imf_gemm_splitk_count returns such a value).
-extern "C" int imf_gemm_splitk_count(int M, int N, int K, int target_tiles) {
-  const int tiles_mn = ((M + 127) / 128) * ((N + 127) / 128);
+//
+// Slices for a persistent grid of `ctas` CTAs (one per SM: the fp32 staging tile leaves room for no
+// second one): the count with the least waves x (k-blocks per slice + what a tile costs besides)
+// + the writing and adding up of the slices.  A k-block of 128 x 128 x 64 lands every 0.27 us; a
+// tile's fill and epilogue take about six of them (an unsplit product adds to its destination in
+// the epilogue, some twenty); the partials move at some 5 TB/s.  (Always filling two waves made 308
+// tiles of 22, three waves on 148 SMs, and wrote twice the partials: the nine weight gradients of a
+// block, d 256, 29,140 tokens, 153 us against 133.)
+extern "C" int imf_gemm_splitk_count(int M, int N, int K, int ctas) {
+  const long tiles = (long)((M + 127) / 128) * ((N + 127) / 128);
   const int nkb = (K + imf::GEMM_BK - 1) / imf::GEMM_BK;
-  int want = (target_tiles + tiles_mn - 1) / tiles_mn;
-  if (want > nkb / 4) want = nkb / 4;          // at least four k-blocks per slice
-  if (want < 1) want = 1;
-  const int per = (nkb + want - 1) / want;
-  return (nkb + per - 1) / per;
+  if (ctas < 1) ctas = 1;
+  int best = 1;
+  double best_cost = 1e30;
+  const long most = 2 * ctas / tiles + 2;
+  for (int want = 1; want <= nkb / 4 && want <= most; ++want) {         // at least four k-blocks per slice
+    const int per = (nkb + want - 1) / want, s = (nkb + per - 1) / per;
+    const double waves = (double)((tiles * s + ctas - 1) / ctas);
+    const double cost = waves * (per + 6) + (s > 1 ? 8.0 + 8.0 * s * M * N / 5e12 / 0.27e-6 : 20.0);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = s;
+    }
+  }
+  return best;
 }
 
 extern "C" int imf_gemm_bf16_splitk(const void* A, const void* B, float* partial, int M, int N,
@@ -597,15 +614,45 @@ extern "C" int imf_gemm_bf16_splitk(const void* A, const void* B, float* partial
 }
 
 namespace imf {
-__global__ void splitk_reduce_kernel(const float* __restrict__ partial, int splits, long plane,
-                                     int N, float* __restrict__ out, int64_t ldo, float alpha,
-                                     int accumulate) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= plane) return;
-  float acc = 0.f;
-  for (int z = 0; z < splits; ++z) acc += partial[z * plane + i];     // fixed order
+// VEC values per thread (4: N, ldo and the addresses are multiples of 16 bytes).  The planes are
+// dealt to the four groups of a CTA in contiguous runs, whose sums are added in order, and a group
+// reads four planes at a time: a sum over all planes in one thread is a chain of memory latencies
+// (7 us for 33 planes of 256 x 256).
+constexpr int REDUCE_GROUPS = 4, REDUCE_LANES = 64;
+template <int VEC>
+__global__ void __launch_bounds__(REDUCE_GROUPS * REDUCE_LANES)
+splitk_reduce_kernel(const float* __restrict__ partial, int splits, long plane, int N,
+                     float* __restrict__ out, int64_t ldo, float alpha, int accumulate) {
+  __shared__ float sums[REDUCE_GROUPS][REDUCE_LANES * VEC];
+  const int lane = threadIdx.x % REDUCE_LANES, grp = threadIdx.x / REDUCE_LANES;
+  const long i = ((long)blockIdx.x * REDUCE_LANES + lane) * VEC;
+  float acc[VEC];
+#pragma unroll
+  for (int j = 0; j < VEC; ++j) acc[j] = 0.f;
+  if (i < plane) {
+    const int z0 = grp * splits / REDUCE_GROUPS, z1 = (grp + 1) * splits / REDUCE_GROUPS;
+#pragma unroll 4
+    for (int z = z0; z < z1; ++z) {
+      if constexpr (VEC == 4) {
+        const float4 v = *reinterpret_cast<const float4*>(partial + z * plane + i);
+        acc[0] += v.x; acc[1] += v.y; acc[2] += v.z; acc[3] += v.w;
+      } else {
+        acc[0] += partial[z * plane + i];
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < VEC; ++j) sums[grp][j * REDUCE_LANES + lane] = acc[j];
+  __syncthreads();
+  if (grp != 0 || i >= plane) return;
   float* dst = out + (i / N) * ldo + (i % N);
-  *dst = accumulate ? *dst + alpha * acc : alpha * acc;
+#pragma unroll
+  for (int j = 0; j < VEC; ++j) {
+    float v = acc[j];
+#pragma unroll
+    for (int g = 1; g < REDUCE_GROUPS; ++g) v += sums[g][j * REDUCE_LANES + lane];
+    dst[j] = accumulate ? dst[j] + alpha * v : alpha * v;
+  }
 }
 }  // namespace imf
 
@@ -614,8 +661,16 @@ extern "C" int imf_splitk_reduce(const float* partial, int splits, int M, int N,
                                  int64_t ldo, float alpha, int accumulate, void* stream) {
   if (splits < 1 || M <= 0 || N <= 0) return imf::IMF_ERR_ARG;
   const long plane = (long)M * N;
-  imf::splitk_reduce_kernel<<<(unsigned)((plane + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-      partial, splits, plane, N, out, ldo, alpha, accumulate);
+  cudaStream_t st = (cudaStream_t)stream;
+  const bool vec = N % 4 == 0 && ldo % 4 == 0 &&
+                   ((reinterpret_cast<uintptr_t>(partial) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  const long threads = vec ? plane / 4 : plane;
+  const unsigned blocks = (unsigned)((threads + imf::REDUCE_LANES - 1) / imf::REDUCE_LANES);
+  constexpr int T = imf::REDUCE_GROUPS * imf::REDUCE_LANES;
+  if (vec)
+    imf::splitk_reduce_kernel<4><<<blocks, T, 0, st>>>(partial, splits, plane, N, out, ldo, alpha, accumulate);
+  else
+    imf::splitk_reduce_kernel<1><<<blocks, T, 0, st>>>(partial, splits, plane, N, out, ldo, alpha, accumulate);
   return cudaGetLastError() == cudaSuccess ? imf::IMF_OK : imf::IMF_ERR_LAUNCH;
 }
 

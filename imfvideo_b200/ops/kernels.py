@@ -183,7 +183,7 @@ def linear_fp8(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = 
     return gemm_fp8(a8, sa, b8, sb, bias=bias).view(*x.shape[:-1], w.shape[0])
 
 
-SPLITK_TARGET_TILES = 296      # two CTAs per SM on 148 SMs
+SPLITK_CTAS = 148              # SMs: the split-K products run one CTA on each
 
 
 def gemm_wgrad(dy: torch.Tensor, x: torch.Tensor, out: Optional[torch.Tensor] = None,
@@ -205,7 +205,7 @@ def gemm_wgrad(dy: torch.Tensor, x: torch.Tensor, out: Optional[torch.Tensor] = 
         out = torch.empty(M, N, dtype=torch.float32, device=dy.device)
         accumulate = False
     assert out.dtype == torch.float32 and out.shape == (M, N) and out.stride(1) == 1
-    splits = int(_lib.imf_gemm_splitk_count(M, N, rows, SPLITK_TARGET_TILES))
+    splits = int(_lib.imf_gemm_splitk_count(M, N, rows, SPLITK_CTAS))
     st = _ptr(status_word(dy.device))
     if splits < 2:
         _check(_lib.imf_gemm_bf16(_ptr(dy), _ptr(x), _ptr(out), None, M, N, rows, dy.stride(0),
