@@ -721,7 +721,7 @@ __global__ void attn_bwd_combine_kernel(const BwParams p, int n_split, float sca
   *reinterpret_cast<uint2*>(dst + c) = o;
 }
 
-// A CTA's start, pipeline fill and epilogue cost about 2.5 of its 1.8 us query steps.
+// A CTA's start, pipeline fill and epilogue cost about 2.5 of its 1.5 us query steps.
 static BwdSplit bwd64_split(int B, int L, int H) {
   const int n_t = (L + BW_T - 1) / BW_T;
   return bwd_split((long)n_t * H * B, n_t, bwd_sm_count(), 2.5f);

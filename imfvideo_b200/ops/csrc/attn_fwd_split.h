@@ -2,9 +2,9 @@
 // kernels.
 //
 // The flattened (item, K/V tile) iteration space is cut into G equal contiguous shares, one per
-// CTA of a persistent grid, so the SMs finish together whatever the number of items (304 items
-// on 148 SMs, B 1, H 4, L 29,140, would otherwise be 2.05 waves).  A share boundary inside an
-// item leaves partial results (un-normalised accumulators, running maximum, sums), which a small
+// CTA of a persistent grid, so the SMs finish together whatever the number of items (228 items
+// on 148 SMs, B 1, H 4, L 29,140, would otherwise be two waves, the second half empty).  A share
+// boundary inside an item leaves partial results (un-normalised accumulators, running maximum, sums), which a small
 // second kernel merges.  With more items than SMs an item is cut at most once; with fewer (short
 // sequences) an item's K/V tiles are spread over several CTAs.
 #pragma once

@@ -65,8 +65,8 @@ inline int make_tmap(CUtensorMap* out, CUtensorMapDataType dt, int rank, void* b
   return IMF_OK;
 }
 
-// Allow a kernel its dynamic shared memory, once per device (`done`: a static array of the
-// caller's, one per kernel; the call costs the host more than the launch itself otherwise).
+// Allow a kernel its dynamic shared memory, once per device instead of once per launch (`done`: a
+// static array of the caller's, one per kernel).
 constexpr int HOST_MAX_DEVICES = 64;
 inline bool allow_smem(const void* kern, size_t smem, bool (&done)[HOST_MAX_DEVICES]) {
   int dev = 0;
