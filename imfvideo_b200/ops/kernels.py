@@ -574,12 +574,13 @@ def newton_schulz(G: torch.Tensor, coeffs, steps: int = 5, eps: float = 1e-7,
         nrm = Gf.flatten(1).norm(dim=1).view(k, 1, 1) + eps
         X.zero_()
         X[:, :, :m] = (Gf / nrm).to(torch.bfloat16)
-    if out is None and mp == m:
+    if out is None and mp == m and steps > 0:
         out = torch.empty(k, n, m, dtype=torch.bfloat16, device=G.device)   # not a workspace view
     if mp != m:
         Y.zero_()        # the pad columns of the other iterate stay zero through a X + B X
-    direct = (out is not None and mp == m and out.dtype == torch.bfloat16 and out.is_contiguous()
-              and out.shape == (k, n, m))
+    # the last product stores into `out`; with no steps the normalised X is copied
+    direct = (steps > 0 and out is not None and mp == m and out.dtype == torch.bfloat16
+              and out.is_contiguous() and out.shape == (k, n, m))
     # upper tiles + mirror pays from four tiles along the Gram side on (measured: 24 x 1024 x
     # 1024 1.10 -> 0.93 ms, 30 x 1536 x 1536 3.93 -> 2.93 ms, but 64 x 256 x 256 0.25 -> 0.28 ms)
     sym = g >= 512 and os.environ.get("IMF_NS_SYM", "1") != "0"     # IMF_NS_SYM=0: full products

@@ -360,6 +360,23 @@ def test_newton_schulz_kernel(K, k, n, m):
     K.check_status()
 
 
+@pytest.mark.parametrize("n,m", [(128, 256), (256, 128), (256, 682)])
+@pytest.mark.parametrize("given", [False, True])
+def test_newton_schulz_without_steps(K, n, m, given):
+    """No iteration: the normalised matrices, as on the torch path (one rounding to bf16, 2^-9, of
+    G over a norm there taken in bf16), not memory that no product has written."""
+    from imfvideo_b200.optim.moonlight import zeropower_via_newtonschulz5
+
+    G = torch.randn(2, n, m, device="cuda")
+    torch.empty(2, n, m, device="cuda").fill_(float("nan"))       # what the allocator hands out next
+    out = torch.full((2, n, m), float("nan"), device="cuda").bfloat16() if given else None
+    X = zeropower_via_newtonschulz5(G, steps=0, out=out)
+    want = G / G.flatten(1).norm(dim=1).view(2, 1, 1)
+    assert (X is out) == given and X.dtype == torch.bfloat16
+    assert _rel(X, want) < 2.0 ** -8
+    K.check_status()
+
+
 def test_batched_gemm_with_additive_source(K):
     torch.manual_seed(0)
     a = torch.randn(3, 200, 136, device="cuda").bfloat16()
