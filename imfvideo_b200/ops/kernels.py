@@ -213,7 +213,7 @@ def gemm_wgrad(dy: torch.Tensor, x: torch.Tensor, out: Optional[torch.Tensor] = 
                                   st, _stream()), "imf_gemm_bf16 (weight gradient)")
         LAUNCHES.count += 1
         return out
-    part = _scratch_buf(dy.device, splits * M * N * 4, "wgrad")
+    part = _workspace(dy.device, splits * M * N * 4)
     _check(_lib.imf_gemm_bf16_splitk(_ptr(dy), _ptr(x), _ptr(part), M, N, rows, dy.stride(0),
                                      x.stride(0), 1, 1, splits, st, _stream()),
            "imf_gemm_bf16_splitk")
@@ -236,20 +236,11 @@ if _has("imf_attn_fwd"):
 
 ATTN_HEAD_DIMS = (64, 128)
 
-_scratch: Dict[Tuple[int, str], torch.Tensor] = {}
 
-
-def _scratch_buf(device: torch.device, nbytes: int, tag: str) -> Optional[torch.Tensor]:
-    """Per-device grow-only scratch (split-item partials of the persistent
-    attention kernels); reused by every call on the same stream order."""
-    if nbytes <= 0:
-        return None
-    key = (device.index or 0, tag)
-    buf = _scratch.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(nbytes, dtype=torch.uint8, device=device)
-        _scratch[key] = buf
-    return buf
+def _workspace(device: torch.device, nbytes: int) -> Optional[torch.Tensor]:
+    """Scratch of one call, from the allocator of the calling stream: calls on several streams or
+    threads may overlap, so it is neither kept nor shared."""
+    return torch.empty(nbytes, dtype=torch.uint8, device=device) if nbytes > 0 else None
 
 
 def _tma_ok(t: torch.Tensor) -> torch.Tensor:
@@ -283,8 +274,7 @@ def attn_fwd(q, k, v, dq=None, dk=None, dv=None, scale: Optional[float] = None,
     do = torch.empty_like(o) if tang else None
     lse = torch.empty(B, H, L, dtype=torch.float32, device=dev) if need_lse else None
     nscr = _lib.imf_attn_fwd_scratch_bytes_hd(B, L, H, int(tang), hd)
-    # of the allocator, not shared: calls on several streams may overlap
-    scr = torch.empty(nscr, dtype=torch.uint8, device=dev) if nscr else None
+    scr = _workspace(dev, nscr)
     ps = [t.data_ptr() for t in ts] + ([] if tang else [None] * 3)
     rc = _lib.imf_attn_fwd(*ps, o.data_ptr(), _ptr(do), _ptr(lse), B, L, H, hd, arr, L * H * hd, H * hd,
                            hd, float(scale), _ptr(scr), nscr, status_word(dev).data_ptr(), _stream())
@@ -347,7 +337,7 @@ def attn_bwd(q, k, v, o, lse, go, scale: Optional[float] = None,
         raise ValueError("dv output needs 16-byte aligned rows")
     i3 = lambda t: (c_int64 * 3)(*t.stride()[:3])
     nscr = _lib.imf_attn_bwd_scratch_bytes_hd(B, L, H, hd)
-    scr = _scratch_buf(q.device, nscr, "attn_bwd")
+    scr = _workspace(q.device, nscr)
     rc = _lib.imf_attn_bwd(*[t.data_ptr() for t in ts[:3]], _ptr(o), _ptr(ts[3]), _ptr(lse), _ptr(dq),
                            _ptr(dk), _ptr(dv), B, L, H, hd, arr, i3(o), i3(dk), i3(dv), float(scale),
                            _ptr(scr), nscr, _ptr(qlist), _ptr(qflags), _ptr(qrank),

@@ -268,6 +268,38 @@ def test_attention_backward_split_tiles(K, B, L, H, hd):
     K.check_status()
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+def test_calls_on_two_streams(K, hd):
+    """Forward (shares of few items), backward (split tiles) and split-K weight gradients issued on
+    two streams in turn, with sizes and values of their own: what they compute one after the other.
+    Equal bits but for dQ, whose fp32 additions land in arrival order (bf16 result: 2^-9)."""
+    g = torch.Generator(device="cuda").manual_seed(hd)
+    mk = lambda *shape: torch.randn(*shape, device="cuda", generator=g).bfloat16()
+    sides = [([mk(1, L, H, hd) for _ in range(7)], mk(L, 256), mk(L, 136)) for L, H in ((2068, 4), (1300, 6))]
+
+    def call(side):
+        (q, k, v, go, *t), dy, x = side
+        o, _, lse = K.attn_fwd(q, k, v)
+        o2, do, _ = K.attn_fwd(q, k, v, *t)
+        return (o, lse, o2, do, *K.attn_bwd(q, k, v, o, lse, go)[1:], K.gemm_wgrad(dy, x),
+                K.attn_bwd(q, k, v, o, lse, go)[0])
+
+    want = [call(side) for side in sides]
+    streams = [torch.cuda.Stream() for _ in sides]
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(6):
+        for i, st in enumerate(streams):
+            with torch.cuda.stream(st):
+                got[i].append(call(sides[i]))
+    torch.cuda.synchronize()
+    K.check_status()
+    for i in range(2):
+        for res in got[i]:
+            assert all(torch.equal(a, b) for a, b in zip(res[:-1], want[i][:-1]))
+            assert _rel(res[-1], want[i][-1]) < 2e-3
+
+
 @pytest.mark.parametrize("B,L,H", [(1, 128, 1), (1, 300, 2), (2, 1000, 3), (1, 2049, 2)])
 def test_attention_backward(K, B, L, H):
     from imfvideo_b200.ops import reference as ref
