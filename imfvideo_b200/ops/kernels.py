@@ -520,21 +520,14 @@ if _has("imf_ns_prepare"):
     _lib.imf_ns_prepare.argtypes = [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
                                     c_float, c_void_p]
 
-_ns_ws: Dict[Tuple[int, int, int, int], Tuple[torch.Tensor, ...]] = {}
-
 
 def _ns_workspace(dev: torch.device, k: int, n: int, mp: int, g: int):
-    """X, Y (k, n, mp), A, B (k, g, g) bf16 and the norm partials, allocated once per shape
-    batch and reused by every later step (the optimizer calls with the same shapes)."""
-    key = (dev.index or 0, k, n, mp)
-    ws = _ns_ws.get(key)
-    if ws is None:
-        bf = dict(dtype=torch.bfloat16, device=dev)
-        ws = (torch.zeros(k, n, mp, **bf), torch.zeros(k, n, mp, **bf),
-              torch.empty(k, g, g, **bf), torch.empty(k, g, g, **bf),
-              torch.empty(k * 32, dtype=torch.float64, device=dev))
-        _ns_ws[key] = ws
-    return ws
+    """X, Y (k, n, mp), A, B (k, g, g) bf16 and the norm partials of one call, from the allocator
+    of the calling stream (calls on several streams or threads may overlap)."""
+    bf = dict(dtype=torch.bfloat16, device=dev)
+    return (torch.empty(k, n, mp, **bf), torch.empty(k, n, mp, **bf),
+            torch.empty(k, g, g, **bf), torch.empty(k, g, g, **bf),
+            torch.empty(k * 32, dtype=torch.float64, device=dev))
 
 
 def newton_schulz(G: torch.Tensor, coeffs, steps: int = 5, eps: float = 1e-7,
@@ -544,9 +537,8 @@ def newton_schulz(G: torch.Tensor, coeffs, steps: int = 5, eps: float = 1e-7,
     tiles on and above the diagonal are computed, the epilogue mirrors them),
     X <- a X + B X (or X B), three launches for the whole batch.  The Gram
     side is chosen by operand major flags, so no transposed copy is made.
-    Normalisation, cast and padding are one two-launch kernel; the iterates live in
-    a workspace kept between calls; with ``out`` (bf16 (k, n, m), m a multiple of 8)
-    the last iteration writes the result there."""
+    Normalisation, cast and padding are one two-launch kernel; with ``out`` (bf16
+    (k, n, m), m a multiple of 8) the last iteration writes the result there."""
     a_, b_, c_ = coeffs
     k, n, m = G.shape
     if min(n, m) < 8 or (n > m and m % 8):
@@ -564,8 +556,6 @@ def newton_schulz(G: torch.Tensor, coeffs, steps: int = 5, eps: float = 1e-7,
         nrm = Gf.flatten(1).norm(dim=1).view(k, 1, 1) + eps
         X.zero_()
         X[:, :, :m] = (Gf / nrm).to(torch.bfloat16)
-    if out is None and mp == m and steps > 0:
-        out = torch.empty(k, n, m, dtype=torch.bfloat16, device=G.device)   # not a workspace view
     if mp != m:
         Y.zero_()        # the pad columns of the other iterate stay zero through a X + B X
     # the last product stores into `out`; with no steps the normalised X is copied
@@ -591,7 +581,7 @@ def newton_schulz(G: torch.Tensor, coeffs, steps: int = 5, eps: float = 1e-7,
     if out is not None:
         out.copy_(res)
         return out
-    return res.clone()      # the workspace is reused by the next call
+    return res.contiguous()
 
 
 if _has("imf_gemm_bf16_batched"):

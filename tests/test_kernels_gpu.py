@@ -270,19 +270,21 @@ def test_attention_backward_split_tiles(K, B, L, H, hd):
 
 @pytest.mark.parametrize("hd", [64, 128])
 def test_calls_on_two_streams(K, hd):
-    """Forward (shares of few items), backward (split tiles) and split-K weight gradients issued on
-    two streams in turn, with sizes and values of their own: what they compute one after the other.
-    Equal bits but for dQ, whose fp32 additions land in arrival order (bf16 result: 2^-9)."""
+    """Forward (shares of few items), backward (split tiles), split-K weight gradients and
+    Newton-Schulz (same shape, other values) issued on two streams in turn: what they compute one
+    after the other.  Equal bits but for dQ, whose fp32 additions land in arrival order (bf16
+    result: 2^-9)."""
     g = torch.Generator(device="cuda").manual_seed(hd)
     mk = lambda *shape: torch.randn(*shape, device="cuda", generator=g).bfloat16()
-    sides = [([mk(1, L, H, hd) for _ in range(7)], mk(L, 256), mk(L, 136)) for L, H in ((2068, 4), (1300, 6))]
+    sides = [([mk(1, L, H, hd) for _ in range(7)], mk(L, 256), mk(L, 136), mk(4, 256, 2 * hd))
+             for L, H in ((2068, 4), (1300, 6))]
 
     def call(side):
-        (q, k, v, go, *t), dy, x = side
+        (q, k, v, go, *t), dy, x, G = side
         o, _, lse = K.attn_fwd(q, k, v)
         o2, do, _ = K.attn_fwd(q, k, v, *t)
         return (o, lse, o2, do, *K.attn_bwd(q, k, v, o, lse, go)[1:], K.gemm_wgrad(dy, x),
-                K.attn_bwd(q, k, v, o, lse, go)[0])
+                K.newton_schulz(G, (3.4445, -4.7750, 2.0315)), K.attn_bwd(q, k, v, o, lse, go)[0])
 
     want = [call(side) for side in sides]
     streams = [torch.cuda.Stream() for _ in sides]
