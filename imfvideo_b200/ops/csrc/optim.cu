@@ -294,7 +294,7 @@ ns_scale_kernel(const float* __restrict__ g, __nv_bfloat16* __restrict__ x, int 
   const float* src = g + (long)z * n * m;
   __nv_bfloat16* dst = x + (long)z * n * mp;
   const long total = (long)n * mp;
-  if (m == mp && (reinterpret_cast<uintptr_t>(g) & 15) == 0) {   // mp is a multiple of eight
+  if (m == mp && mp % 8 == 0 && ((reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(x)) & 15) == 0) {
     // nothing to pad: 32 bytes in, 16 bytes out per thread, no division (24 x 1,024 x 1,024:
     // 71 us with a value per thread and its row and column by 64-bit division)
     for (long i = (long)blockIdx.x * 256 + threadIdx.x; i < total / 8; i += (long)gridDim.x * 256) {

@@ -411,6 +411,25 @@ def test_newton_schulz_without_steps(K, n, m, given):
     K.check_status()
 
 
+@pytest.mark.parametrize("n,m,mp,shift", [(3, 13, 13, 0), (5, 12, 12, 0), (5, 16, 16, 0), (5, 16, 16, 1),
+                                          (5, 16, 16, 2), (4, 13, 16, 0), (33, 24, 24, 0)])
+def test_newton_schulz_prepare_forms(K, n, m, mp, shift):
+    """The normalise-and-cast launcher takes any row length and address: widths that are no multiple
+    of eight, and a source (shift 1) or destination (shift 2) off a 16-byte boundary, go value by
+    value.  One rounding to bf16 (2^-9) of an fp32 quotient."""
+    k = 3
+    src = torch.randn(k * n * m + 1, device="cuda")[int(shift == 1):][:k * n * m].view(k, n, m)
+    dst = torch.full((k * n * mp + 2,), 7.0, device="cuda").bfloat16()
+    x = dst[int(shift == 2):][:k * n * mp].view(k, n, mp)
+    part = torch.empty(k * 32, dtype=torch.float64, device="cuda")
+    rc = K._lib.imf_ns_prepare(K._ptr(src), K._ptr(x), k, n, m, mp, K._ptr(part), 1e-7, K._stream())
+    assert rc == 0
+    want = src / src.flatten(1).norm(dim=1).view(k, 1, 1)
+    assert _rel(x[..., :m], want) < 2.0 ** -9 and bool((x[..., m:] == 0).all())
+    rest = torch.cat([dst[:int(shift == 2)], dst[int(shift == 2) + k * n * mp:]])
+    assert bool((rest == 7.0).all())
+
+
 def test_batched_gemm_with_additive_source(K):
     torch.manual_seed(0)
     a = torch.randn(3, 200, 136, device="cuda").bfloat16()
