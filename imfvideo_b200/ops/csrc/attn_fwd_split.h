@@ -81,7 +81,8 @@ __device__ __forceinline__ void combine_split_items(const P& p, int G) {
   const int q_row = qb * ITEM_M + r;
   if (q_row >= p.L) return;
   const float* x = p.scratch + (size_t)(2 * c + 1) * REC + r;     // then records 2c + 2, 2c + 4, ...
-  float m = -INFINITY, l = 0.f, mu = 0.f;
+  // the first part's own maximum, not -inf: with a scale of zero or below, -inf has no finite weight
+  float m = x[STATS], l = 0.f, mu = 0.f;
   float o[COMBINE_COLS], d[COMBINE_COLS];
 #pragma unroll
   for (int i = 0; i < COMBINE_COLS; ++i) o[i] = d[i] = 0.f;

@@ -208,6 +208,27 @@ def test_attention_forward_shares(K, hd, B, L, H, grow):
     K.check_status()
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("B,L,H", [(1, 532, 4), (1, 7000, 10)])
+@pytest.mark.parametrize("scale", [0.0, -0.1])
+def test_attention_forward_scale_of_zero_and_below(K, hd, B, L, H, scale):
+    """Split items (few, and more than SMs) with every weight equal, and with the sign of the scores
+    turned over.  The rounding of P and of the result to bf16, 2^-9 each, bounds the error; the
+    tangent is a difference of two such sums."""
+    from imfvideo_b200.ops import reference as ref
+
+    g = torch.Generator(device="cuda").manual_seed(L + hd)
+    q, k, v, dq, dk, dv = (torch.randn(B, L, H, hd, device="cuda", generator=g).bfloat16() for _ in range(6))
+    f = lambda t: t.float()
+    ro, rdo = ref.attention_jvp(*map(f, (q, k, v, dq, dk, dv)), scale=scale)
+    rl = ref.attention_lse(f(q), f(k), scale=scale)
+    o, _, lse = K.attn_fwd(q, k, v, scale=scale)
+    o2, do, lse2 = K.attn_fwd(q, k, v, dq, dk, dv, scale=scale)
+    assert _rel(o, ro) < 6e-3 and _rel(o2, ro) < 6e-3 and _rel(do, rdo) < 1.2e-2
+    assert (lse - rl).abs().max() < 1e-3 and (lse2 - rl).abs().max() < 1e-3
+    K.check_status()
+
+
 def test_attention_strided_views_and_run_twice(K):
     """v as a slice of a wider kv tensor (as in MLA); two runs are bit-equal."""
     torch.manual_seed(0)
