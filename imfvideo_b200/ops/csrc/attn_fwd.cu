@@ -576,12 +576,9 @@ static int launch_attn_fwd(const void* q, const void* k, const void* v, const vo
   prm.sh.n_items = prm.n_qblk * H * B;
   prm.sh.n_kv = (L + C::BN - 1) / C::BN;
   prm.sh.total = (long)prm.sh.n_items * prm.sh.n_kv;
-  const int G = fwd_grid(prm.sh.n_items, prm.sh.n_kv);
-  if (G != prm.sh.n_items) {
-    if (prm.scratch == nullptr ||
-        scratch_bytes < (size_t)G * 2 * att_part_floats<TANGENT, NTP>() * sizeof(float))
-      return IMF_ERR_ARG;
-  }
+  const int G = fwd_grid(prm.sh.n_items, prm.sh.n_kv, prm.scratch, scratch_bytes / sizeof(float),
+                         att_part_floats<TANGENT, NTP>());
+  if (G == 0) return IMF_ERR_ARG;
   // strides: [q_sb,q_sl,q_sh, k_sb,k_sl,k_sh, v_sb,v_sl,v_sh, dq.., dk.., dv..]
   if ((rc = make_qkv_map(&mq, q, B, L, H, strides[0], strides[1], strides[2], ATT_TILE_M))) return rc;
   if ((rc = make_qkv_map(&mk, k, B, L, H, strides[3], strides[4], strides[5], C::BN))) return rc;
@@ -627,9 +624,14 @@ static int primal_nt(int L) {
   return rows4 * 9L <= rows3 * 10L ? 4 : 3;
 }
 
+static long primal_items(int B, int L, int H) {
+  const int item_m = primal_nt(L) * ATT_TILE_M;
+  return (long)((L + item_m - 1) / item_m) * H * B;
+}
+
 }  // namespace imf
 
-// Bytes of scratch the forward needs for (B, L, H): 0 when no item is split.
+// Bytes of scratch the forward takes for (B, L, H): 0 when no item is split.
 extern "C" long imf_attn_fwd_scratch_bytes(int B, int L, int H, int tangent) {
   using namespace imf;
   return (long)(tangent ? att_scratch_bytes<true, 2>(B, L, H)
@@ -647,7 +649,8 @@ extern "C" long imf_attn_fwd_scratch_bytes_hd(int B, int L, int H, int tangent, 
 // bf16, head_dim 64 or 128; `strides` holds (batch, row, head) element strides for q, k, v and,
 // when tangents are given, dq, dk, dv.  o/dout contiguous-in-last-dim with
 // strides (o_sb, o_sl, o_sh).  lse: (B, H, L) fp32 or null.  scratch: device
-// buffer of at least imf_attn_fwd_scratch_bytes() bytes (may be null if 0).
+// buffer of imf_attn_fwd_scratch_bytes_hd() bytes.  With less (or null), problems of
+// fewer work items than SMs run with one CTA per item, others are refused.
 extern "C" int imf_attn_fwd(const void* q, const void* k, const void* v, const void* dq,
                             const void* dk, const void* dv, void* o, void* dout, float* lse,
                             int B, int L, int H, int head_dim, const int64_t* strides,
@@ -724,7 +727,10 @@ extern "C" int imf_attn_fwd_noalloc(const void* q, const void* k, const void* v,
     scratch_of_device[dev] = static_cast<float*>(ptr);
   }
   if (head_dim != ATT_HD) return IMF_ERR_ARG;     // the built-in scratch is sized for head_dim 64
-  const long need = imf_attn_fwd_scratch_bytes(B, L, H, 0);
+  // problems of no more items than SMs leave the array alone (one CTA per item), so that short calls
+  // on several streams share nothing
+  const bool shares = B > 0 && L > 0 && H > 0 && primal_items(B, L, H) > fwd_sm_count();
+  const long need = shares ? imf_attn_fwd_scratch_bytes(B, L, H, 0) : 0;
   if (need > (long)(NOALLOC_FLOATS * sizeof(float))) {
     fprintf(stderr,
             "imf_attn_fwd_noalloc: problem needs %ld bytes of partial-result scratch, the "
@@ -733,6 +739,6 @@ extern "C" int imf_attn_fwd_noalloc(const void* q, const void* k, const void* v,
     return IMF_ERR_TOO_LARGE;
   }
   return imf_attn_fwd(q, k, v, nullptr, nullptr, nullptr, o, nullptr, lse, B, L, H, head_dim,
-                      strides, o_sb, o_sl, o_sh, scale, scratch_of_device[dev],
-                      (long)(NOALLOC_FLOATS * sizeof(float)), status, stream);
+                      strides, o_sb, o_sl, o_sh, scale, shares ? scratch_of_device[dev] : nullptr,
+                      shares ? (long)(NOALLOC_FLOATS * sizeof(float)) : 0, status, stream);
 }

@@ -603,12 +603,9 @@ static int launch(const Fwd128Args& a) {
   prm.sh.n_items = prm.n_qblk * a.H * a.B;
   prm.sh.n_kv = (a.L + BN - 1) / BN;
   prm.sh.total = (long)prm.sh.n_items * prm.sh.n_kv;
-  const int G = fwd_grid(prm.sh.n_items, prm.sh.n_kv);
-  if (G != prm.sh.n_items) {
-    if (prm.scratch == nullptr ||
-        (size_t)a.scratch_bytes < (size_t)G * 2 * part_floats<TANGENT>() * sizeof(float))
-      return IMF_ERR_ARG;
-  }
+  const int G = fwd_grid(prm.sh.n_items, prm.sh.n_kv, prm.scratch,
+                         (size_t)a.scratch_bytes / sizeof(float), part_floats<TANGENT>());
+  if (G == 0) return IMF_ERR_ARG;
   CUtensorMap mq, mk, mv, mdq, mdk, mdv;
   int rc;
   const int64_t* st = a.strides;

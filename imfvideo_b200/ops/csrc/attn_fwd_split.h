@@ -141,4 +141,13 @@ inline int fwd_grid(long n_items, int n_kv) {
   return (int)g;
 }
 
+// The same for a launch whose caller gave `have` floats of scratch, at two records of `rec` floats
+// per CTA.  Fewer items than SMs need none: one CTA takes each of them then, longer but as correct.
+// 0: the scratch is too small for a problem that cannot do without.
+inline int fwd_grid(long n_items, int n_kv, const float* scratch, size_t have, size_t rec) {
+  const int g = fwd_grid(n_items, n_kv);
+  if (g == n_items || (scratch != nullptr && have >= (size_t)g * 2 * rec)) return g;
+  return n_items <= fwd_sm_count() ? (int)n_items : 0;
+}
+
 }  // namespace imf

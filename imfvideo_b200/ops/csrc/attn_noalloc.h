@@ -9,28 +9,33 @@
 //
 // The regular entry point (imf_attn_fwd) expects the caller to provide a
 // scratch buffer for the partial results of work items that are split between
-// two thread blocks.  Here that scratch lives in a file-scope __device__ array
+// thread blocks.  Here that scratch lives in a file-scope __device__ array
 // inside the library, so the caller passes inputs and outputs only.
 //
 // Limits and rules:
 //  * primal forward only (no tangent), head_dim 64, bf16, same layouts as
 //    imf_attn_fwd;
-//  * the built-in scratch holds the partials of at most
-//    IMF_ATTN_NOALLOC_MAX_CTAS (160) thread blocks = 43,909,120 bytes; every
-//    GPU that loads the library keeps that much reserved until the process
-//    exits.  A device with more SMs than that, for a problem that needs one
-//    partial slot per SM, is rejected with IMF_ERR_TOO_LARGE (-4);
+//  * a work item is 384 or 512 query rows of one (batch, head).  A problem of no
+//    more items than the GPU has SMs runs with one thread block per item and
+//    does not use the built-in scratch (the regular entry point spreads such
+//    items over several thread blocks, which takes scratch and less time);
+//  * with more items the grid is one thread block per SM, and items are split
+//    between two of them.  The built-in scratch holds the partials (two records
+//    a thread block) of at most IMF_ATTN_NOALLOC_MAX_CTAS (160) thread blocks =
+//    43,909,120 bytes; every GPU that loads the library keeps that much reserved
+//    until the process exits.  On a device with more SMs than that such a
+//    problem is rejected with IMF_ERR_TOO_LARGE (-4);
 //  * the first call on each device looks up the device address of the array
 //    (cudaGetSymbolAddress, with that device current).  Make that first call
 //    outside of any stream capture.  First calls made at the same time from
 //    several host threads are safe: each of them looks up and stores the same
 //    address for that device;
-//  * all calls on a device share the one array and it keeps the previous
-//    call's contents.  Nothing in it needs to start at zero: every slot that a
-//    launch reads was written earlier in the same launch sequence.  Two calls
-//    whose kernels can overlap on the GPU (different streams without an
-//    ordering between them) race on the array and give wrong results; order
-//    them on one stream or with events;
+//  * all calls with more items than SMs share the one array of their device and
+//    it keeps the previous call's contents.  Nothing in it needs to start at
+//    zero: every slot that a launch reads was written earlier in the same launch
+//    sequence.  Two such calls whose kernels can overlap on the GPU (different
+//    streams without an ordering between them) race on the array and give wrong
+//    results; order them on one stream or with events;
 //  * no cudaMalloc / cudaFree / allocating library routine is called.
 #pragma once
 #include <stdint.h>

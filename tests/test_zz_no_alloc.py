@@ -93,3 +93,80 @@ def test_noalloc_entry_rejects_oversize_request():
     big = torch.zeros(1, 384 * (sms + 1), 1, 64, dtype=torch.bfloat16, device="cuda")
     rc, _, _ = _call_noalloc(lib, big, big, big, status)
     assert rc == -4
+
+
+@pytest.mark.parametrize("sizes", [((1, 532, 4), (1, 130, 2)), ((2, 2068, 4), (1, 3000, 12))])
+def test_short_calls_share_no_scratch(sizes):
+    """Problems of fewer work items than SMs leave the built-in array alone: two calls on two
+    streams at once give the bits of a call by itself.  Against the regular entry point, which
+    spreads such items over several thread blocks, the results differ by the order of fp32 sums
+    (rounded to bf16: 2^-9)."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from imfvideo_b200.ops import cuda as cu
+
+    assert cu.available()
+    from imfvideo_b200.ops import kernels as K
+
+    lib = ctypes.CDLL(cu.LIB_PATH)
+    status = K.status_word(torch.device("cuda", 0))
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    xs, alone = [], []
+    for seed, (B, L, H) in enumerate(sizes):
+        assert B * H * math.ceil(L / 384) < sms
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        xs.append([torch.randn(B, L, H, 64, device="cuda", generator=g).bfloat16() for _ in range(3)])
+        rc, o, lse = _call_noalloc(lib, *xs[-1], status)
+        assert rc == 0
+        alone.append((o, lse))
+        ref_o, _, ref_lse = K.attn_fwd(*xs[-1])
+        assert ((o.float() - ref_o.float()).norm() / ref_o.float().norm()) < 4e-3
+        assert (lse - ref_lse).abs().max() < 1e-4
+    streams = [torch.cuda.Stream() for _ in sizes]
+    torch.cuda.synchronize()
+    got = []
+    for _ in range(20):
+        for i, st in enumerate(streams):
+            with torch.cuda.stream(st):
+                got.append((i, *_call_noalloc(lib, *xs[i], status)))
+    torch.cuda.synchronize()
+    K.check_status()
+    for i, rc, o, lse in got:
+        assert rc == 0 and torch.equal(o, alone[i][0]) and torch.equal(lse, alone[i][1])
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("tangent", [False, True])
+def test_regular_entry_without_scratch(hd, tangent):
+    """The regular C entry takes a null (or too small) scratch where items are fewer than SMs, and
+    refuses it where they are more."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from imfvideo_b200.ops import cuda as cu
+
+    assert cu.available()
+    from imfvideo_b200.ops import kernels as K
+
+    def call(L, H, nbytes):
+        x = [torch.randn(1, L, H, hd, device="cuda", generator=g).bfloat16() for _ in range(6 if tangent else 3)]
+        o, do = torch.empty_like(x[0]), torch.empty_like(x[0]) if tangent else None
+        lse = torch.empty(1, H, L, device="cuda")
+        scr = torch.empty(nbytes, dtype=torch.uint8, device="cuda") if nbytes else None
+        rc = K._lib.imf_attn_fwd(*[t.data_ptr() for t in x], *([] if tangent else [None] * 3), o.data_ptr(),
+                                 K._ptr(do), lse.data_ptr(), 1, L, H, hd, K._bls_array(x, 18), L * H * hd,
+                                 H * hd, hd, 0.1, K._ptr(scr), nbytes,
+                                 K.status_word(torch.device("cuda", 0)).data_ptr(), K._stream())
+        return rc, x, o, do, lse
+
+    g = torch.Generator(device="cuda").manual_seed(hd)
+    for nbytes in (0, 4096):
+        assert K._lib.imf_attn_fwd_scratch_bytes_hd(1, 1100, 4, int(tangent), hd) > nbytes
+        rc, x, o, do, lse = call(1100, 4, nbytes)
+        assert rc == 0
+        want = K.attn_fwd(*x, scale=0.1)
+        for a, b in zip((o, do), want):
+            if a is not None:                      # order of fp32 sums, rounded to bf16 (2^-9)
+                assert ((a.float() - b.float()).norm() / b.float().norm()) < 6e-3
+        assert (lse - want[2]).abs().max() < 1e-4
+        assert call(4000, 40, nbytes)[0] == -1
+    K.check_status()
