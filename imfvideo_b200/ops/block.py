@@ -183,6 +183,9 @@ class _BlockFn(torch.autograd.Function):
         # 6. attention core
         o, do, core_saved = core.fwd(q[0], k[0], v0, q[1] if has_t else None,
                                      k[1] if has_t else None, v1, need_bwd)
+        for x in (o, do) if has_t else (o,):       # native code reads their bare pointers
+            assert x is not None and x.dtype == BF16 and x.numel() == rows * hv and x.is_contiguous() \
+                and x.device == dev
         # 7.-11. output gate, output projection, residual + remix + norm2, MLP, residual
         if g.gate:
             og = new(T, rows, hv)

@@ -191,6 +191,86 @@ def test_fused_block_matches_generic_composition(kernels, bs, wide):
     assert set(g_f) >= set(g_g)
 
 
+def _one_block(gate=True, impl=None, L=300, d=256, H=4):
+    """A block with nothing at its initial zero or one, its rope tables and inputs with tangent."""
+    from imfvideo_b200.models import flash_jvp_attention
+    from imfvideo_b200.models.imf_dit_video import TransformerBlock
+
+    torch.manual_seed(0)
+    blk = TransformerBlock(d, H, 128, 128, 48, 16, 64, weight_init_constant=0.5, norm_eps=1e-5,
+                           attn_impl=impl or flash_jvp_attention, mla_use_output_gate=gate).cuda()
+    with torch.no_grad():
+        for p in blk.parameters():
+            p.add_(torch.randn_like(p) * 0.03)
+        for p in (blk.attn_scale, blk.mlp_scale):
+            p.add_(0.5)
+    ang = torch.rand(L, 8, device="cuda") * 6.28
+    x = torch.randn(2, L, d, device="cuda")
+    return blk, ang.cos(), ang.sin(), x, torch.randn_like(x), torch.randn_like(x)
+
+
+@pytest.mark.parametrize("gate", [True, False])
+@pytest.mark.parametrize("tangent", [True, False])
+def test_fused_block_with_and_without_output_gate(kernels, gate, tangent):
+    """One block node against the op-by-op path, whose GEMMs and attention round to bf16 (2^-9) at
+    the same places; without the gate the attention's output goes straight into the projection."""
+    from imfvideo_b200.ops import cuda as cu
+    from imfvideo_b200.ops.dual import Dual
+
+    blk, cos, sin, x, dx, go = _one_block(gate)
+    assert blk.fused_ok(x, torch.bfloat16)
+
+    def run():
+        blk.zero_grad()
+        xx = x.clone().requires_grad_()
+        out = blk(Dual(xx, dx if tangent else None), cos, sin, torch.bfloat16)
+        out.p.backward(go)
+        return out.p, out.t, xx.grad, {n: p.grad.clone() for n, p in blk.named_parameters() if p.grad is not None}
+
+    of, tf, xf, gf = run()
+    kernels.check_status()
+    cu.disable("block")
+    try:
+        og, tg, xg, gg = run()
+    finally:
+        cu.enable("block")
+    rel = lambda a, b: ((a.float() - b.float()).norm() / (b.float().norm() + 1e-12)).item()
+    assert rel(of, og) < 2e-2 and rel(xf, xg) < 3e-2 and set(gf) >= set(gg)
+    assert (tf is None) == (tg is None) == (not tangent)
+    assert not tangent or rel(tf, tg) < 3e-2
+    bad = [(n, rel(gf[n], gg[n])) for n in gg if rel(gf[n], gg[n]) > 6e-2]
+    assert not bad, bad
+
+
+@pytest.mark.parametrize("gate", [True, False])
+@pytest.mark.parametrize("change", ["permuted", "fp32", "short", "no tangent"])
+def test_fused_block_refuses_what_its_core_must_not_return(kernels, gate, change):
+    """The native launches after the attention core read its outputs as contiguous bf16 rows."""
+    from imfvideo_b200.ops.block import DenseCore
+    from imfvideo_b200.ops.dual import Dual
+
+    class Core(DenseCore):
+        def fwd(self, *args):
+            o, do, saved = super().fwd(*args)
+            if change == "permuted":
+                o = o.transpose(1, 2).contiguous().transpose(1, 2)
+            elif change == "fp32":
+                do = do.float()
+            elif change == "short":
+                do = do[:, :-1].contiguous()
+            else:
+                do = None
+            return o, do, saved
+
+    class Impl:
+        fused_core = Core()
+
+    blk, cos, sin, x, dx, _ = _one_block(gate, Impl())
+    with pytest.raises(AssertionError), torch.no_grad():
+        blk(Dual(x, dx), cos, sin, torch.bfloat16)
+    kernels.check_status()
+
+
 def test_weight_gradients_written_straight_into_existing_grad_buffers(kernels):
     """With fp32 ``.grad`` buffers already attached (the optimizer engine's arena views), the
     block node accumulates dY^T X into them itself and hands autograd nothing for the
