@@ -479,11 +479,15 @@ extern "C" int imf_build_kv_lists(const uint8_t* fm, const uint16_t* rk, int* ql
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
-// Block ids are 16 bits with the sign bit of an entry left alone, and the staging fits 48 KB.
+// The staging (6 bytes per query tile) and the scan's static array share the 48 KB a launch gets
+// without asking; block ids then fit 16 bits with the sign bit of an entry left alone.  Maps of
+// imf_build_tile_lut have at most 2,048 query tiles.
+constexpr int KV_PAIR_MAX_TILES = (48 * 1024 - 256) / 6;
+
 extern "C" int imf_build_kv_pair_lists(const uint8_t* fm, int* qlist, uint8_t* qflags, int B, int H,
                                        int n_kvt, int n_mt, void* stream) {
   if (B <= 0 || H <= 0 || n_kvt <= 0 || n_mt <= 0) return -1;
-  if (n_mt > 8192) return -4;
+  if (n_mt > KV_PAIR_MAX_TILES) return -4;
   kv_pair_lists_kernel<<<dim3(n_kvt, H, B), RT_THREADS, 6 * n_mt, (cudaStream_t)stream>>>(
       fm, qlist, qflags, n_mt);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;

@@ -164,9 +164,8 @@ def kv_pair_lists(maps: torch.Tensor):
 
 def bwd_lists(maps: torch.Tensor):
     """Arguments of ``kernels.attn_bwd`` that describe the routing: block pairs, or whole query
-    tiles with their ranks where the order of dQ additions is fixed (it is kept per tile) or the
-    block ids do not fit an entry."""
-    if K.DETERMINISTIC or maps.shape[-1] > 8192:
+    tiles with their ranks where the order of dQ additions is fixed (it is kept per tile)."""
+    if K.DETERMINISTIC:
         qlist, qflags, qrank = kv_lists(maps, want_rank=True)
         return dict(qlist=qlist, qflags=qflags, qrank=qrank)
     qlist, qflags = kv_pair_lists(maps)

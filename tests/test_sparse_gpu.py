@@ -228,6 +228,28 @@ def test_sparse_backward_block_pairs(SP, qblk, L, T):
     kernels.check_status()
 
 
+@pytest.mark.parametrize("n_mt", [1, 255, 2048, 8149])
+def test_block_pair_lists_of_long_rows(SP, n_mt):
+    """Every length of a row of maps up to what the kernel's staging holds; one more is refused."""
+    g = torch.Generator(device="cuda").manual_seed(n_mt)
+    fm = torch.randint(0, 16, (1, 1, 2, n_mt), device="cuda", generator=g).to(torch.uint8)
+    ql, qf = (t.cpu() for t in SP.kv_pair_lists(fm))
+    for t in range(2):
+        f = fm[0, 0, t].cpu().long()
+        halves = torch.stack([f & 5, (f >> 1) & 5], 1).view(-1)        # of blocks 0, 1, 2, ...
+        ids = halves.nonzero().view(-1)
+        n = -(-len(ids) // 2)
+        assert bool((ql[0, 0, t, n:] == -1).all()) and bool((qf[0, 0, t, n:] == 0).all())
+        e, k = ql[0, 0, t, :n].long(), qf[0, 0, t, :n].long()
+        got = torch.stack([e & 0xffff, e >> 16], 1).view(-1)
+        flags = torch.stack([k & 5, (k >> 1) & 5], 1).view(-1)
+        if len(ids) % 2:
+            assert got[-1] == 2 * n_mt and flags[-1] == 0
+        assert torch.equal(got[:len(ids)], ids) and torch.equal(flags[:len(ids)], halves[ids])
+    with pytest.raises((ValueError, RuntimeError)):
+        SP.kv_pair_lists(torch.ones(1, 1, 1, 8150, dtype=torch.uint8, device="cuda"))
+
+
 def test_sparse_backward_bitwise_repeatable(SP):
     from imfvideo_b200.ops import kernels
     """Block-sparse backward with the device-built lists and ranks: dQ bit-identical from run
