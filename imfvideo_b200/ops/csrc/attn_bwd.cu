@@ -404,14 +404,16 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const int ord = qrank ? (int)qrank[i] : kvb;
         if (turn && turn_live) turn_live = turn_wait(turn + qt, ord, abort_flag, p.status);
         if (!turn || turn_live) {
-          if (SPARSE) {                    // boxes of 64 rows; a dead block has nothing to add
+          if (SPARSE) {      // boxes of 64 rows; a dead block, or one past the end, has nothing to add
             const uint32_t f = flags_at(i);
 #pragma unroll
-            for (int half = 0; half < 2; ++half)
-              if (f & (5u << half))
+            for (int half = 0; half < 2; ++half) {
+              const int r0 = q_block(p, qlist[i], half) * 64;
+              if ((f & (5u << half)) && r0 < p.L)
                 for (int pnl = 0; pnl < 2; ++pnl)
                   tma_reduce_add_4d(&tm_dq, stage + pnl * (BW_T * 128) + half * 64 * 128, pnl * 32, h,
-                                    q_block(p, qlist[i], half) * 64, b);
+                                    r0, b);
+            }
           } else {
 #pragma unroll
             for (int pnl = 0; pnl < 2; ++pnl)

@@ -228,6 +228,33 @@ def test_sparse_backward_block_pairs(SP, qblk, L, T):
     kernels.check_status()
 
 
+@pytest.mark.parametrize("L", [40, 130, 680])
+@pytest.mark.parametrize("pairs", [False, True])
+def test_sparse_backward_last_tile_with_one_half(SP, L, pairs):
+    """128-row routing blocks whose last one ends in the first half of its query tile: the second half
+    is marked live like the first and lies past the end, where nothing is added.  Bounds as in
+    test_sparse_backward_kernel."""
+    from imfvideo_b200.models import sla2 as S
+    from imfvideo_b200.ops import kernels
+
+    g = torch.Generator(device="cuda").manual_seed(L)
+    q, k, v, go = (torch.randn(1, L, 2, 64, device="cuda", generator=g).bfloat16() for _ in range(4))
+    Mb, Nb = -(-L // 128), -(-L // 64)
+    sel = torch.rand(1, 2, Mb, Nb, device="cuda", generator=g).argsort(-1)[..., :max(1, Nb // 2)].int()
+    lut, flags, cnt, maps = SP.route_tables(sel, 128, L)
+    o, _, lse = SP.sparse_fwd(q, k, v, None, None, None, lut, flags, 128, False, quant_p=False, cnt=cnt)
+    ql, qf = SP.kv_pair_lists(maps) if pairs else SP.kv_lists(maps)
+    got = kernels.attn_bwd(q, k, v, o, lse, go, qlist=ql, qflags=qf, qpairs=pairs)
+    ph = lambda t: t.permute(0, 2, 1, 3).float()
+    ref = [ph(t).requires_grad_(True) for t in (q, k, v)]
+    _, o_s, _, _ = S.sparse_linear_attention(*ref, sel, 128, 64, torch.ones(2, L, device="cuda"),
+                                             return_parts=True)
+    o_s.backward(ph(go))
+    for a, b in zip(got, ref):
+        assert _rel(a.permute(0, 2, 1, 3), b.grad) < 2e-2
+    kernels.check_status()
+
+
 @pytest.mark.parametrize("n_mt", [1, 255, 2048, 8149])
 def test_block_pair_lists_of_long_rows(SP, n_mt):
     """Every length of a row of maps up to what the kernel's staging holds; one more is refused."""
