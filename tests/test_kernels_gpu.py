@@ -209,12 +209,13 @@ def test_attention_forward_shares(K, hd, B, L, H, grow):
 
 
 @pytest.mark.parametrize("hd", [64, 128])
-@pytest.mark.parametrize("B,L,H", [(1, 532, 4), (1, 7000, 10)])
+@pytest.mark.parametrize("B,L,H", [(1, 576, 4), (1, 7040, 10)])
 @pytest.mark.parametrize("scale", [0.0, -0.1])
 def test_attention_forward_scale_of_zero_and_below(K, hd, B, L, H, scale):
     """Split items (few, and more than SMs) with every weight equal, and with the sign of the scores
-    turned over.  The rounding of P and of the result to bf16, 2^-9 each, bounds the error; the
-    tangent is a difference of two such sums."""
+    turned over.  Whole K/V tiles only: the keys past a ragged end are masked by a score of -inf
+    before the scale is applied, which needs a scale above zero.  The rounding of P and of the
+    result to bf16, 2^-9 each, bounds the error; the tangent is a difference of two such sums."""
     from imfvideo_b200.ops import reference as ref
 
     g = torch.Generator(device="cuda").manual_seed(L + hd)
