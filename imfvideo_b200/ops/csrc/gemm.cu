@@ -571,21 +571,31 @@ extern "C" int imf_gemm_fp8(const void* A, const void* B, void* C, const float* 
 // Slices for a persistent grid of `ctas` CTAs (one per SM: the fp32 staging tile leaves room for no
 // second one): the count with the least waves x (k-blocks per slice + what a tile costs besides)
 // + the writing and adding up of the slices.  A k-block of 128 x 128 x 64 lands every 0.27 us; a
-// tile's fill and epilogue take about six of them (an unsplit product adds to its destination in
-// the epilogue, some twenty); the partials move at some 5 TB/s.  (Always filling two waves made 308
-// tiles of 22, three waves on 148 SMs, and wrote twice the partials: the nine weight gradients of a
-// block, d 256, 29,140 tokens, 153 us against 133.)
-extern "C" int imf_gemm_splitk_count(int M, int N, int K, int ctas) {
+// tile's fill and epilogue take about six of them; the partials move at some 5 TB/s.  (Always
+// filling two waves made 308 tiles of 22, three waves on 148 SMs, and wrote twice the partials: the
+// nine weight gradients of a block, d 256, 29,140 tokens, 153 us against 133.)
+// An unsplit product is stored as it is; with `accumulate` it is added to its destination in the
+// epilogue, a row per thread, which takes some hundred k-blocks a tile, behind the next tile's
+// products if there is one.  2,752 x 1,024 (two waves), 532 rows: 10 us unsplit without accumulate,
+// 58 with it; two slices 22 and 24.
+extern "C" int imf_gemm_splitk_count(int M, int N, int K, int ctas, int accumulate) {
   const long tiles = (long)((M + 127) / 128) * ((N + 127) / 128);
   const int nkb = (K + imf::GEMM_BK - 1) / imf::GEMM_BK;
+  constexpr double ADD = 100;
   if (ctas < 1) ctas = 1;
   int best = 1;
   double best_cost = 1e30;
   const long most = 2 * ctas / tiles + 2;
   for (int want = 1; want <= nkb / 4 && want <= most; ++want) {         // at least four k-blocks per slice
     const int per = (nkb + want - 1) / want, s = (nkb + per - 1) / per;
-    const double waves = (double)((tiles * s + ctas - 1) / ctas);
-    const double cost = waves * (per + 6) + (s > 1 ? 8.0 + 8.0 * s * M * N / 5e12 / 0.27e-6 : 20.0);
+    const double waves = (double)((tiles * s + ctas - 1) / ctas), tile = per + 6;
+    double cost;
+    if (s > 1)
+      cost = waves * tile + 8 + 8.0 * s * M * N / 5e12 / 0.27e-6;
+    else if (accumulate)
+      cost = tile + (waves - 1) * (tile > ADD ? tile : ADD) + ADD;
+    else
+      cost = waves * tile + 20;
     if (cost < best_cost) {
       best_cost = cost;
       best = s;

@@ -118,7 +118,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
 
 if _has("imf_gemm_bf16_splitk"):
     _lib.imf_gemm_splitk_count.restype = c_int
-    _lib.imf_gemm_splitk_count.argtypes = [c_int] * 4
+    _lib.imf_gemm_splitk_count.argtypes = [c_int] * 5
     _lib.imf_gemm_bf16_splitk.restype = c_int
     _lib.imf_gemm_bf16_splitk.argtypes = [c_void_p] * 3 + [c_int] * 3 + [c_int64] * 2 + \
         [c_int] * 3 + [c_void_p, c_void_p]
@@ -205,7 +205,7 @@ def gemm_wgrad(dy: torch.Tensor, x: torch.Tensor, out: Optional[torch.Tensor] = 
         out = torch.empty(M, N, dtype=torch.float32, device=dy.device)
         accumulate = False
     assert out.dtype == torch.float32 and out.shape == (M, N) and out.stride(1) == 1
-    splits = int(_lib.imf_gemm_splitk_count(M, N, rows, SPLITK_CTAS))
+    splits = int(_lib.imf_gemm_splitk_count(M, N, rows, SPLITK_CTAS, int(accumulate)))
     st = _ptr(status_word(dy.device))
     if splits < 2:
         _check(_lib.imf_gemm_bf16(_ptr(dy), _ptr(x), _ptr(out), None, M, N, rows, dy.stride(0),

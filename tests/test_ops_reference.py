@@ -75,3 +75,23 @@ def test_newton_schulz_reference_orthogonalises():
     X = ref.newton_schulz(G, (3.4445, -4.7750, 2.0315), steps=5)
     s = torch.linalg.svdvals(X)
     assert s.min() > 0.5 and s.max() < 1.3
+
+
+def test_splitk_counts():
+    """Slices of the weight-gradient products (host rule of the kernel library): the count is one its
+    launcher accepts, leaves four k-blocks to a slice, and splits what would be added to its
+    destination from the epilogue of a short product but not what is only stored."""
+    from imfvideo_b200.ops import cuda as cu
+
+    lib = cu.lib()
+    if lib is None:
+        pytest.skip("kernel library not built")
+    count = lib.imf_gemm_splitk_count
+    for M, N in ((128, 64), (256, 256), (384, 96), (1376, 256), (2752, 1024), (1536, 1536), (8960, 1536)):
+        for rows in (1, 64, 300, 532, 1000, 2068, 7820, 32780):
+            for acc in (0, 1):
+                s, nkb = count(M, N, rows, 148, acc), -(-rows // 64)
+                assert s >= 1 and (s == 1 or (nkb // s >= 3 and -(-nkb // -(-nkb // s)) == s))
+    for M, N in ((2752, 1024), (1024, 2752), (1536, 1536)):
+        for rows in (532, 1000, 2068):
+            assert count(M, N, rows, 148, 1) > 1 and count(M, N, rows, 148, 0) == 1
