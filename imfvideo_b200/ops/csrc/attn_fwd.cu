@@ -11,8 +11,9 @@
 // models/triton_block_jvp.py:228-346) and the FA/SDPA primal forward.
 //
 // Work item = NT 128-row query tiles that share every 64-row K/V tile, of one (batch,
-// head): four tiles in the primal kernel (three where rounding L up to 512 rows wastes more
-// than that gains), two in the tangent kernel; TMEM (512 columns) holds no more.  Warps
+// head): four tiles in the primal kernel (three or two where rounding L up to 512 rows wastes more
+// than that gains or SMs would stand idle, see primal_nt), two in the tangent kernel; TMEM (512
+// columns) holds no more.  Warps
 // 4t .. 4t+3: softmax + O-correction + epilogue of tile t (one query row per thread, rows live
 // in TMEM lanes); then one warp with the single-thread tcgen05.mma issuer, one TMA producer
 // warp and two warps that only donate registers (setmaxnreg).  The tiles take turns: while
@@ -42,7 +43,7 @@ constexpr int ATT_TILE_M = 128;
 
 // Work item = NT query tiles of 128 rows that share every 64-row K/V tile.
 //   tangent kernel : NT 2, TMEM per tile S|dS|O|dO
-//   primal kernel  : NT 3 or 4, TMEM per tile S|O
+//   primal kernel  : NT 2, 3 or 4, TMEM per tile S|O
 template <bool TANGENT, int NTP>
 struct AttCfg {
   static constexpr int NT = NTP;
@@ -74,6 +75,7 @@ struct AttCfg {
   static constexpr int TMEM_COLS = 512;
   static constexpr int ACC = TANGENT ? 2 * ATT_HD : ATT_HD;   // fp32 accumulators per row
   static_assert(COL_O + ACC <= TILE_COLS && NT * TILE_COLS <= 512, "");
+  static constexpr float PART_COST = TANGENT ? 0.65f : 0.4f;  // see fwd_share_cost
 };
 
 // scratch record of one part of a split item: [ACC][ITEM_M] accumulators (a column per row of the
@@ -576,8 +578,8 @@ static int launch_attn_fwd(const void* q, const void* k, const void* v, const vo
   prm.sh.n_items = prm.n_qblk * H * B;
   prm.sh.n_kv = (L + C::BN - 1) / C::BN;
   prm.sh.total = (long)prm.sh.n_items * prm.sh.n_kv;
-  const int G = fwd_grid(prm.sh.n_items, prm.sh.n_kv, prm.scratch, scratch_bytes / sizeof(float),
-                         att_part_floats<TANGENT, NTP>());
+  const int G = fwd_grid(prm.sh.n_items, prm.sh.n_kv, C::PART_COST, prm.scratch,
+                         scratch_bytes / sizeof(float), att_part_floats<TANGENT, NTP>());
   if (G == 0) return IMF_ERR_ARG;
   // strides: [q_sb,q_sl,q_sh, k_sb,k_sl,k_sh, v_sb,v_sl,v_sh, dq.., dk.., dv..]
   if ((rc = make_qkv_map(&mq, q, B, L, H, strides[0], strides[1], strides[2], ATT_TILE_M))) return rc;
@@ -613,20 +615,42 @@ template <bool TANGENT, int NTP>
 static size_t att_scratch_bytes(int B, int L, int H) {
   using C = AttCfg<TANGENT, NTP>;
   const long n_items = (long)((L + C::ITEM_M - 1) / C::ITEM_M) * H * B;
-  const int G = fwd_grid(n_items, (L + C::BN - 1) / C::BN);
+  const int G = fwd_grid(n_items, (L + C::BN - 1) / C::BN, C::PART_COST);
   return G == n_items ? 0 : (size_t)G * 2 * att_part_floats<TANGENT, NTP>() * sizeof(float);
 }
 
-// Query tiles per work item of the primal kernel: four (1.04 ms at B 1, H 4, L 29,140; three:
-// 1.16 ms), unless rounding L up to 512 rows wastes more than that gains over 384.
-static int primal_nt(int L) {
-  const int rows4 = (L + 511) / 512 * 512, rows3 = (L + 383) / 384 * 384;
-  return rows4 * 9L <= rows3 * 10L ? 4 : 3;
+static long primal_items(int B, int L, int H, int nt) {
+  const int item_m = nt * ATT_TILE_M;
+  return (long)((L + item_m - 1) / item_m) * H * B;
 }
 
-static long primal_items(int B, int L, int H) {
-  const int item_m = primal_nt(L) * ATT_TILE_M;
-  return (long)((L + item_m - 1) / item_m) * H * B;
+// Query tiles per work item of the primal kernel: of two, three and four the one with the least time
+// by the following account.  A K/V tile takes 1.13, 1.19 and 1.43 us, so that with many items four
+// are the best (B 1, H 4, L 29,140: 1.02 ms, three 1.16) unless rounding L up to 512 rows wastes more
+// than that gains over 384; with few items, SMs that would stand idle take smaller ones (H 4, L 532:
+// 15.7, 17.3 and 20.5 us).  A launch takes 5.1, 6.0 and 6.5 us besides, and the merge of split items
+// that are more than the SMs six tiles.  (177 shapes of 1 to 64 heads and 130 to 7,820 rows: 0.4 %
+// from the best of the six forms on average.)
+static int primal_nt(int B, int L, int H) {
+  constexpr float TILE_US[3] = {1.13f, 1.19f, 1.43f}, BASE_US[3] = {5.1f, 6.0f, 6.5f};
+  constexpr float PART_COST = AttCfg<false, 4>::PART_COST;
+  constexpr int BN = AttCfg<false, 4>::BN;
+  const int n_kv = (L + BN - 1) / BN, sms = fwd_sm_count();
+  int best = 4;
+  float best_us = 0.f;
+  for (int nt = 2; nt <= 4; ++nt) {
+    const long items = primal_items(B, L, H, nt);
+    const int g = fwd_grid(items, n_kv, PART_COST);
+    const float walk = (float)((items * n_kv + g - 1) / g);
+    const float tiles = items > sms ? walk + 6.f
+                        : g == items ? walk : walk + fwd_share_cost(items, n_kv, g, PART_COST);
+    const float us = BASE_US[nt - 2] + TILE_US[nt - 2] * tiles;
+    if (nt == 2 || us < best_us) {
+      best = nt;
+      best_us = us;
+    }
+  }
+  return best;
 }
 
 }  // namespace imf
@@ -634,9 +658,12 @@ static long primal_items(int B, int L, int H) {
 // Bytes of scratch the forward takes for (B, L, H): 0 when no item is split.
 extern "C" long imf_attn_fwd_scratch_bytes(int B, int L, int H, int tangent) {
   using namespace imf;
-  return (long)(tangent ? att_scratch_bytes<true, 2>(B, L, H)
-                        : (primal_nt(L) == 4 ? att_scratch_bytes<false, 4>(B, L, H)
-                                             : att_scratch_bytes<false, 3>(B, L, H)));
+  if (tangent) return (long)att_scratch_bytes<true, 2>(B, L, H);
+  switch (primal_nt(B, L, H)) {
+    case 2: return (long)att_scratch_bytes<false, 2>(B, L, H);
+    case 3: return (long)att_scratch_bytes<false, 3>(B, L, H);
+    default: return (long)att_scratch_bytes<false, 4>(B, L, H);
+  }
 }
 
 // Same for either head_dim (64 or 128).
@@ -685,11 +712,15 @@ extern "C" int imf_attn_fwd(const void* q, const void* k, const void* v, const v
     if (dout == nullptr || (reinterpret_cast<uintptr_t>(dout) & 15)) return IMF_ERR_ARG;
     return launch_attn_fwd<true, 2>(q, k, v, dq, dk, dv, strides, prm, (size_t)scratch_bytes, st);
   }
-  if (primal_nt(L) == 4)
-    return launch_attn_fwd<false, 4>(q, k, v, nullptr, nullptr, nullptr, strides, prm,
-                                     (size_t)scratch_bytes, st);
-  return launch_attn_fwd<false, 3>(q, k, v, nullptr, nullptr, nullptr, strides, prm,
-                                   (size_t)scratch_bytes, st);
+#define IMF_PRIMAL(NT)                                                                              \
+  return launch_attn_fwd<false, NT>(q, k, v, nullptr, nullptr, nullptr, strides, prm,               \
+                                    (size_t)scratch_bytes, st)
+  switch (primal_nt(B, L, H)) {
+    case 2: IMF_PRIMAL(2);
+    case 3: IMF_PRIMAL(3);
+    default: IMF_PRIMAL(4);
+  }
+#undef IMF_PRIMAL
 }
 
 // ---------------------------------------------------------------------------
@@ -729,7 +760,8 @@ extern "C" int imf_attn_fwd_noalloc(const void* q, const void* k, const void* v,
   if (head_dim != ATT_HD) return IMF_ERR_ARG;     // the built-in scratch is sized for head_dim 64
   // problems of no more items than SMs leave the array alone (one CTA per item), so that short calls
   // on several streams share nothing
-  const bool shares = B > 0 && L > 0 && H > 0 && primal_items(B, L, H) > fwd_sm_count();
+  const bool shares = B > 0 && L > 0 && H > 0 &&
+                      primal_items(B, L, H, primal_nt(B, L, H)) > fwd_sm_count();
   const long need = shares ? imf_attn_fwd_scratch_bytes(B, L, H, 0) : 0;
   if (need > (long)(NOALLOC_FLOATS * sizeof(float))) {
     fprintf(stderr,

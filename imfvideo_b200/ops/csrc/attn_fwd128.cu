@@ -65,6 +65,7 @@ struct Cfg {
   static constexpr int NC = SPLIT ? BN / 2 : BN;             // score columns per thread
   static constexpr int ROW_THREADS = SPLIT ? 2 * TM : TM;    // softmax threads of one tile
   static_assert(NT * TILE_COLS <= 512, "TMEM budget");
+  static constexpr float PART_COST = TANGENT ? 0.9f : 0.6f;  // see fwd_share_cost
 };
 
 template <bool TANGENT>
@@ -603,7 +604,7 @@ static int launch(const Fwd128Args& a) {
   prm.sh.n_items = prm.n_qblk * a.H * a.B;
   prm.sh.n_kv = (a.L + BN - 1) / BN;
   prm.sh.total = (long)prm.sh.n_items * prm.sh.n_kv;
-  const int G = fwd_grid(prm.sh.n_items, prm.sh.n_kv, prm.scratch,
+  const int G = fwd_grid(prm.sh.n_items, prm.sh.n_kv, C::PART_COST, prm.scratch,
                          (size_t)a.scratch_bytes / sizeof(float), part_floats<TANGENT>());
   if (G == 0) return IMF_ERR_ARG;
   CUtensorMap mq, mk, mv, mdq, mdk, mdv;
@@ -641,7 +642,8 @@ static int launch(const Fwd128Args& a) {
 long attn_fwd128_scratch_bytes(int B, int L, int H, int tangent) {
   const int item_m = tangent ? a128::Cfg<true>::ITEM_M : a128::Cfg<false>::ITEM_M;
   const long n_items = (long)((L + item_m - 1) / item_m) * H * B;
-  const int G = fwd_grid(n_items, (L + a128::BN - 1) / a128::BN);
+  const int G = fwd_grid(n_items, (L + a128::BN - 1) / a128::BN,
+                         tangent ? a128::Cfg<true>::PART_COST : a128::Cfg<false>::PART_COST);
   if (G == n_items) return 0;
   const size_t per = tangent ? a128::part_floats<true>() : a128::part_floats<false>();
   return (long)((size_t)G * 2 * per * sizeof(float));

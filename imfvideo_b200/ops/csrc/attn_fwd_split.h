@@ -130,22 +130,33 @@ inline int fwd_sm_count() {
 }
 
 // CTAs of the persistent grid.  Fewer items than SMs: shares of at least two K/V tiles, if that
-// shortens a CTA's walk by four tiles or more; the second kernel and the extra stores cost what
-// about three tiles do (4 us).
-inline int fwd_grid(long n_items, int n_kv) {
+// shortens a CTA's walk by more than it costs.  In K/V tiles (1 to 1.4 us) the second kernel and the
+// extra stores cost three, `part_cost` for each part of an item, and seven parts' worth more where
+// shares and items do not end together, so that a CTA begins and stores two.  Fitted to 375 shapes
+// of the four kernels timed both ways (1 to 96 heads, 300 to 6,500 rows; 1.4 to 1.9 us rms):
+// head_dim 128 with tangent, 8 heads, 532 rows 18 us without shares and 25 with; 1 head, 4,116 rows
+// 80 and 42.
+inline float fwd_share_cost(long n_items, int n_kv, long g, float part_cost) {
+  const long total = n_items * n_kv, walk = (total + g - 1) / g;
+  const bool uneven = total % g != 0 || n_kv % walk != 0;
+  return 3.f + part_cost * ((float)g / (float)n_items + (uneven ? 7.f : 0.f));
+}
+inline int fwd_grid(long n_items, int n_kv, float part_cost) {
   const int sms = fwd_sm_count();
   if (n_items >= sms) return sms;
   const long total = n_items * n_kv;
   const long g = total / 2 < sms ? total / 2 : sms;
-  if (g <= n_items || n_kv - (total + g - 1) / g < 4) return (int)n_items;
-  return (int)g;
+  if (g <= n_items) return (int)n_items;
+  const float saved = (float)(n_kv - (total + g - 1) / g);
+  return saved < 1.f + fwd_share_cost(n_items, n_kv, g, part_cost) ? (int)n_items : (int)g;
 }
 
 // The same for a launch whose caller gave `have` floats of scratch, at two records of `rec` floats
 // per CTA.  Fewer items than SMs need none: one CTA takes each of them then, longer but as correct.
 // 0: the scratch is too small for a problem that cannot do without.
-inline int fwd_grid(long n_items, int n_kv, const float* scratch, size_t have, size_t rec) {
-  const int g = fwd_grid(n_items, n_kv);
+inline int fwd_grid(long n_items, int n_kv, float part_cost, const float* scratch, size_t have,
+                    size_t rec) {
+  const int g = fwd_grid(n_items, n_kv, part_cost);
   if (g == n_items || (scratch != nullptr && have >= (size_t)g * 2 * rec)) return g;
   return n_items <= fwd_sm_count() ? (int)n_items : 0;
 }

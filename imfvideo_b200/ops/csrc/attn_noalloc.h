@@ -15,7 +15,7 @@
 // Limits and rules:
 //  * primal forward only (no tangent), head_dim 64, bf16, same layouts as
 //    imf_attn_fwd;
-//  * a work item is 384 or 512 query rows of one (batch, head).  A problem of no
+//  * a work item is 256, 384 or 512 query rows of one (batch, head).  A problem of no
 //    more items than the GPU has SMs runs with one thread block per item and
 //    does not use the built-in scratch (the regular entry point spreads such
 //    items over several thread blocks, which takes scratch and less time);

@@ -208,6 +208,20 @@ def test_attention_forward_shares(K, hd, B, L, H, grow):
     K.check_status()
 
 
+@pytest.mark.parametrize("L,H", [(200, 3), (1000, 2), (850, 40), (2600, 8), (850, 64), (5200, 8)])
+def test_attention_forward_items(K, L, H):
+    """The primal kernel's work items of two, three and four query tiles, each whole and in shares (in
+    this order two whole, two, three whole, three, four whole, four on 148 SMs); bounds as above."""
+    from imfvideo_b200.ops import reference as ref
+
+    g = torch.Generator(device="cuda").manual_seed(L + H)
+    q, k, v = (torch.randn(1, L, H, 64, device="cuda", generator=g).bfloat16() for _ in range(3))
+    o, _, lse = K.attn_fwd(q, k, v)
+    assert _rel(o, ref.attention(q.float(), k.float(), v.float())) < 6e-3
+    assert (lse - ref.attention_lse(q.float(), k.float())).abs().max() < 1e-3
+    K.check_status()
+
+
 @pytest.mark.parametrize("hd", [64, 128])
 @pytest.mark.parametrize("B,L,H", [(1, 576, 4), (1, 7040, 10)])
 @pytest.mark.parametrize("scale", [0.0, -0.1])
