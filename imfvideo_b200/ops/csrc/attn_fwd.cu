@@ -80,7 +80,7 @@ struct AttCfg {
 
 // scratch record of one part of a split item: [ACC][ITEM_M] accumulators (a column per row of the
 // record: the softmax threads own a query row each, so a warp stores 128 consecutive bytes), then
-// m, l, mu per query row
+// m, l, mu per query row (primal: in mu's place the row sum of the exact exponentials)
 template <bool TANGENT, int NTP>
 constexpr size_t att_part_floats() {
   return (size_t)AttCfg<TANGENT, NTP>::ITEM_M * (AttCfg<TANGENT, NTP>::ACC + 3);
@@ -115,7 +115,13 @@ struct AttParams {
   int* status;
 };
 
-template <bool TANGENT, int NTP>
+// The row sum that divides O is taken over P as the tensor core multiplies it, rounded to bf16: the
+// rounding errors of a row's weights then cancel in part (with a sum of the exponentials themselves
+// the error of O grows by 10 % where few keys carry the weight).  The log-sum-exp wants the exact
+// sum; LSE instances of the primal kernel take both (B 1, H 4, L 29,140: 1.07 ms, without 1.04, with
+// one exact sum for both 1.01; from the tensor core, three query tiles, 1.12).  The tangent kernel
+// takes the exact sum only, as its T = P dS does.
+template <bool TANGENT, int NTP, bool LSE>
 __global__ void __launch_bounds__(AttCfg<TANGENT, NTP>::THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_dq,
@@ -446,7 +452,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             }
           }
           const f32x2 neg_m2 = dup2(-m_used * scale_log2);
-          f32x2 l2 = pair2(__float_as_uint(l_sum), __float_as_uint(l_sum2));
+          f32x2 exact2 = pair2(__float_as_uint(mu_sum), __float_as_uint(mu_sum2));
 #pragma unroll
           for (int c = 0; c < BN; c += 32) {
             uint32_t x[32], pk[16];
@@ -458,12 +464,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               const f32x2 e = fma2(pair2(x[i], x[i + 1]), dup2(scale_log2), neg_m2);
               const float p0 = ex2(lo2(e)), p1 = ex2(hi2(e));
               pk[i / 2] = pack_bf16(p0, p1);
-              l2 = add2(l2, pair2(__float_as_uint(p0), __float_as_uint(p1)));
+              l_sum = add_bf16(pk[i / 2], l_sum);
+              l_sum2 = add_bf16(pk[i / 2] >> 16, l_sum2);
+              if (LSE) exact2 = add2(exact2, pair2(__float_as_uint(p0), __float_as_uint(p1)));
             }
             tmem_st16(tb + C::COL_S + c / 2, pk);
           }
-          l_sum = lo2(l2);
-          l_sum2 = hi2(l2);
+          if (LSE) {
+            mu_sum = lo2(exact2);
+            mu_sum2 = hi2(exact2);
+          }
         }
         tc_wait_st();
         tc_fence_before();
@@ -519,10 +529,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             }
           }
         }
-        if (live && p.lse)
-          p.lse[((int64_t)b * p.H + h) * p.L + q_row] = m_used * p.scale + __logf(l_tot);
+        if (LSE && live && p.lse)
+          p.lse[((int64_t)b * p.H + h) * p.L + q_row] =
+              m_used * p.scale + __logf(TANGENT ? l_tot : mu_tot);
       } else {
-        // partial result of a split item: raw accumulators + (m, l, mu)
+        // partial result of a split item: raw accumulators + (m, l, mu; primal: the exact row sum)
         float* part = p.scratch + (size_t)sg.rec * att_part_floats<TANGENT, NTP>();
 #pragma unroll
         for (int c = 0; c < C::ACC; c += 32) {
@@ -597,10 +608,11 @@ static int launch_attn_fwd(const void* q, const void* k, const void* v, const vo
     mdk = mk;
     mdv = mv;
   }
-  auto kern = attn_fwd_kernel<TANGENT, NTP>;
+  const bool lse = TANGENT || prm.lse != nullptr;
+  auto kern = lse ? attn_fwd_kernel<TANGENT, NTP, true> : attn_fwd_kernel<TANGENT, NTP, TANGENT>;
   const size_t smem = sizeof(AttSmem<TANGENT, NTP>) + 1024;
-  static bool smem_set[HOST_MAX_DEVICES] = {false};
-  if (!allow_smem((const void*)kern, smem, smem_set)) return IMF_ERR_LAUNCH;
+  static bool smem_set[2][HOST_MAX_DEVICES] = {{false}};
+  if (!allow_smem((const void*)kern, smem, smem_set[lse])) return IMF_ERR_LAUNCH;
   kern<<<G, C::THREADS, smem, stream>>>(mq, mk, mv, mdq, mdk, mdv, prm);
   if (cudaGetLastError() != cudaSuccess) return IMF_ERR_LAUNCH;
   if (G != prm.sh.n_items) {

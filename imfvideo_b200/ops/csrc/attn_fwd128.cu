@@ -556,7 +556,7 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           float* stats = part + (size_t)C::ITEM_M * C::ACC;
           stats[row_in_item] = m_used;
           stats[C::ITEM_M + row_in_item] = l_tot;
-          stats[2 * C::ITEM_M + row_in_item] = mu_tot;
+          stats[2 * C::ITEM_M + row_in_item] = TANGENT ? mu_tot : l_tot;
         }
       }
       tc_fence_before();

@@ -60,7 +60,8 @@ __device__ __forceinline__ bool split_item(const FwdShares& p, int c, int G, int
 }
 
 // Merge the parts of every split item.  A record is [ACC][ITEM_M] accumulators (o, then dout with
-// a tangent), then m, l, mu per query row.  A CTA takes 32 query rows (a lane each), a warp 8 of
+// a tangent), then m, l, mu per query row; without a tangent mu's place holds the row sum of the
+// exact exponentials, for the log-sum-exp.  A CTA takes 32 query rows (a lane each), a warp 8 of
 // the HD columns.  All of it is load latency, so the parts are merged in one pass (running maximum)
 // whose loads are independent of one another.  147 split items of 384 to 512 rows took 16 us
 // (head_dim 64, a warp per row) and 58 us (head_dim 128, a thread per row) before.
@@ -92,7 +93,7 @@ __device__ __forceinline__ void combine_split_items(const P& p, int G) {
     const float w0 = ex2((m - mn) * scale_log2), w1 = ex2((mk - mn) * scale_log2);
     m = mn;
     l = l * w0 + x[STATS + ITEM_M] * w1;
-    if (TANGENT) mu = mu * w0 + x[STATS + 2 * ITEM_M] * w1;
+    mu = mu * w0 + x[STATS + 2 * ITEM_M] * w1;
 #pragma unroll
     for (int i = 0; i < COMBINE_COLS; ++i) {
       o[i] = o[i] * w0 + x[(col + i) * ITEM_M] * w1;
@@ -110,7 +111,8 @@ __device__ __forceinline__ void combine_split_items(const P& p, int G) {
   }
   *reinterpret_cast<uint4*>(p.o + off) = make_uint4(ob[0], ob[1], ob[2], ob[3]);
   if (TANGENT) *reinterpret_cast<uint4*>(p.dout + off) = make_uint4(db[0], db[1], db[2], db[3]);
-  if (p.lse && col == 0) p.lse[((int64_t)b * p.H + h) * p.L + q_row] = m * p.scale + __logf(l);
+  if (p.lse && col == 0)
+    p.lse[((int64_t)b * p.H + h) * p.L + q_row] = m * p.scale + __logf(TANGENT ? l : mu);
 }
 
 // SM count of the CURRENT device (cached per device index: a host may hold GPUs of

@@ -411,6 +411,12 @@ IMF_DEVICE f32x2 add2(f32x2 a, f32x2 b) {
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
+// c + a with `a` a bf16 value in the low half of the register, rounded once, to fp32
+IMF_DEVICE float add_bf16(uint32_t a, float c) {
+  float r;
+  asm("add.f32.bf16 %0, %1, %2;" : "=f"(r) : "h"((unsigned short)a), "f"(c));
+  return r;
+}
 IMF_DEVICE uint32_t pack_bf16(float lo, float hi) {
   uint32_t r;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));

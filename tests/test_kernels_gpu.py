@@ -208,6 +208,28 @@ def test_attention_forward_shares(K, hd, B, L, H, grow):
     K.check_status()
 
 
+@pytest.mark.parametrize("L,H", [(130, 24), (2049, 8)])
+@pytest.mark.parametrize("need_lse", [False, True])
+def test_attention_forward_divides_by_the_sum_of_rounded_weights(K, L, H, need_lse):
+    """Scores of standard deviation 16, few keys carry the weight: the error of o is that of weights
+    rounded to bf16 and divided by their own sum (5 % for where a row's reference maximum lies and
+    fp32 sums; the division by the sum of the exact weights costs 10 % and more); the log-sum-exp
+    is that of the exact ones (1e-4: fp32 scores of up to 100)."""
+    g = torch.Generator(device="cuda").manual_seed(L)
+    q, k, v = ((torch.randn(1, L, H, 64, device="cuda", generator=g) * s).bfloat16() for s in (4, 4, 1))
+    s = torch.einsum("blhd,bshd->bhls", q.double(), k.double()) / 8
+    p = torch.exp(s - s[..., :64].amax(-1, keepdim=True))
+    pr = p.float().bfloat16().double()
+    mul = lambda w, d: (torch.einsum("bhls,bshd->bhld", w, v.double()) / d.sum(-1, keepdim=True)).transpose(1, 2)
+    exact = mul(p, p)
+    own = _rel(mul(pr, pr).bfloat16(), exact)
+    o, _, lse = K.attn_fwd(q, k, v, need_lse=need_lse)
+    assert _rel(o, exact) < 1.05 * own
+    assert (lse is not None) == need_lse
+    assert not need_lse or (lse - torch.logsumexp(s, -1)).abs().max() < 1e-4
+    K.check_status()
+
+
 @pytest.mark.parametrize("L,H", [(200, 3), (1000, 2), (850, 40), (2600, 8), (850, 64), (5200, 8)])
 def test_attention_forward_items(K, L, H):
     """The primal kernel's work items of two, three and four query tiles, each whole and in shares (in
