@@ -47,11 +47,15 @@ inline BwdSplit bwd_split(long items, int n_steps, int sms, float cta_steps) {
   r.parts = 1;
   r.n_split = 0;
   if (rest == 0) return r;
+  // the kernel that adds the partials up is one launch more, some 2 (head_dim 64) to 4 us (128), which
+  // short walks do not make up for (head_dim 64, 12 heads, 385 rows: 18.4 us whole, 20.1 split;
+  // head_dim 128, 8 heads, 256 rows: 19.3 and 20.3)
+  const float launch = 0.6f * cta_steps;
   float best = (float)n_steps + cta_steps;
   for (int p = 2; p <= n_steps && (long)rest * p <= 6L * sms; ++p) {
     const int waves = (rest * p + sms - 1) / sms;
     // the partials are written and summed on top: about half a CTA start per wave
-    const float t = waves * ((float)((n_steps + p - 1) / p) + 1.5f * cta_steps);
+    const float t = waves * ((float)((n_steps + p - 1) / p) + 1.5f * cta_steps) + launch;
     if (t < best - 0.01f) {
       best = t;
       r.parts = p;
