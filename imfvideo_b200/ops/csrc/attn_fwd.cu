@@ -18,10 +18,11 @@
 // in TMEM lanes); then one warp with the single-thread tcgen05.mma issuer, one TMA producer
 // warp and two warps that only donate registers (setmaxnreg).  The tiles take turns: while
 // one tile's softmax runs on the CUDA cores the tensor core works on another.
-// The softmax warps are bound by dependency latency first (0.4 instructions per cycle and
-// scheduler, exponential unit three quarters busy), so what counts is how many tiles are in
-// flight: B 1, H 4, L 29,140 takes 1.02 ms with four tiles, 1.08 to 1.16 with three.  Pairs of
-// scores go through packed fp32 instructions.  P (and T) are written back to TMEM as bf16 over
+// The softmax warps are bound by dependency latency (0.4 instructions per cycle and scheduler,
+// exponential unit some 70 % busy), so what counts is how many tiles are in flight: B 1, H 4,
+// L 29,140 took 1.01 ms with four tiles and 1.08 to 1.16 with three when the row sum was of the
+// exact exponentials; as it is now (below) four take 1.04 ms.  Pairs of scores go through packed
+// fp32 instructions.  P (and T) are written back to TMEM as bf16 over
 // the S (dS) columns and are the A operand of the second GEMM.  O is rescaled lazily (only
 // when the running max grows by > 2^8).
 //
@@ -638,8 +639,8 @@ static long primal_items(int B, int L, int H, int nt) {
 
 // Query tiles per work item of the primal kernel: of two, three and four the one with the least time
 // by the following account.  A K/V tile takes 1.13, 1.19 and 1.43 us, so that with many items four
-// are the best (B 1, H 4, L 29,140: 1.02 ms, three 1.16) unless rounding L up to 512 rows wastes more
-// than that gains over 384; with few items, SMs that would stand idle take smaller ones (H 4, L 532:
+// are the best (B 1, H 4, L 29,140: 1.01 ms, three 1.16, with exact row sums) unless rounding L up to
+// 512 rows wastes more than that gains over 384; with few items, SMs that would stand idle take smaller ones (H 4, L 532:
 // 15.7, 17.3 and 20.5 us).  A launch takes 5.1, 6.0 and 6.5 us besides, and the merge of split items
 // that are more than the SMs six tiles.  (177 shapes of 1 to 64 heads and 130 to 7,820 rows: 0.4 %
 // from the best of the six forms on average.)
