@@ -650,6 +650,7 @@ static int primal_nt(int B, int L, int H) {
   constexpr int BN = AttCfg<false, 4>::BN;
   const int n_kv = (L + BN - 1) / BN, sms = fwd_sm_count();
   int best = 4;
+  if (B <= 0 || L <= 0 || H <= 0) return best;      // refused at the launch
   float best_us = 0.f;
   for (int nt = 2; nt <= 4; ++nt) {
     const long items = primal_items(B, L, H, nt);

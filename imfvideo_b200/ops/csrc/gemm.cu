@@ -582,6 +582,7 @@ extern "C" int imf_gemm_splitk_count(int M, int N, int K, int ctas, int accumula
   const long tiles = (long)((M + 127) / 128) * ((N + 127) / 128);
   const int nkb = (K + imf::GEMM_BK - 1) / imf::GEMM_BK;
   constexpr double ADD = 100;
+  if (tiles < 1) return 1;         // refused at the launch
   if (ctas < 1) ctas = 1;
   int best = 1;
   double best_cost = 1e30;

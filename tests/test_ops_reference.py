@@ -95,3 +95,21 @@ def test_splitk_counts():
     for M, N in ((2752, 1024), (1024, 2752), (1536, 1536)):
         for rows in (532, 1000, 2068):
             assert count(M, N, rows, 148, 1) > 1 and count(M, N, rows, 148, 0) == 1
+    assert count(0, 128, 532, 148, 1) == 1 and count(128, 0, 532, 148, 0) == 1
+
+
+def test_attention_scratch_of_nothing():
+    """Empty problems, which the launchers refuse, need no scratch."""
+    import ctypes
+
+    from imfvideo_b200.ops import cuda as cu
+
+    lib = cu.lib()
+    if lib is None:
+        pytest.skip("kernel library not built")
+    f = lib.imf_attn_fwd_scratch_bytes_hd
+    f.restype, f.argtypes = ctypes.c_long, [ctypes.c_int] * 5
+    for size in ((0, 532, 4), (1, 0, 4), (1, 532, 0)):
+        for tangent in (0, 1):
+            for hd in (64, 128):
+                assert f(*size, tangent, hd) == 0
