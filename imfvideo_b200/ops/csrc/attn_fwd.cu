@@ -12,7 +12,7 @@
 //
 // Work item = NT 128-row query tiles that share every 64-row K/V tile, of one (batch,
 // head): four tiles in the primal kernel (three or two where rounding L up to 512 rows wastes more
-// than that gains or SMs would stand idle, see primal_nt), two in the tangent kernel; TMEM (512
+// than that gains or SMs would stand idle, see primal_form), two in the tangent kernel; TMEM (512
 // columns) holds no more.  Warps
 // 4t .. 4t+3: softmax + O-correction + epilogue of tile t (one query row per thread, rows live
 // in TMEM lanes); then one warp with the single-thread tcgen05.mma issuer, one TMA producer
@@ -42,14 +42,17 @@ namespace imf {
 constexpr int ATT_HD = 64;
 constexpr int ATT_TILE_M = 128;
 
-// Work item = NT query tiles of 128 rows that share every 64-row K/V tile.
+// Work item = NT query tiles of 128 rows that share every K/V tile (64 rows).
 //   tangent kernel : NT 2, TMEM per tile S|dS|O|dO
-//   primal kernel  : NT 2, 3 or 4, TMEM per tile S|O
+//   primal kernel  : NT 2, 3 or 4, TMEM per tile S|O; or NT 2 with K/V tiles of 128 rows, for items
+//                    that are not split (ATT_WIDE)
+constexpr int ATT_WIDE = 1;
 template <bool TANGENT, int NTP>
 struct AttCfg {
-  static constexpr int NT = NTP;
+  static constexpr bool WIDE = NTP == ATT_WIDE;
+  static constexpr int NT = WIDE ? 2 : NTP;
   static constexpr int ITEM_M = NT * ATT_TILE_M;
-  static constexpr int BN = 64;
+  static constexpr int BN = WIDE ? 128 : 64;
   static constexpr int NQ = TANGENT ? 2 : 1;       // q + dq
   static constexpr int NKV = TANGENT ? 4 : 2;      // k, v (+ dk, dv)
   static constexpr int V = TANGENT ? 2 : 1;        // v's place: k, v  or  k, dk, v, dv
@@ -72,11 +75,11 @@ struct AttCfg {
   static constexpr int COL_DS = BN;
   static constexpr int COL_O = TANGENT ? 2 * BN : BN;
   static constexpr int COL_DO = COL_O + ATT_HD;    // tangent only
-  static constexpr int TILE_COLS = TANGENT ? 256 : 128;
+  static constexpr int TILE_COLS = TANGENT || WIDE ? 256 : 128;
   static constexpr int TMEM_COLS = 512;
   static constexpr int ACC = TANGENT ? 2 * ATT_HD : ATT_HD;   // fp32 accumulators per row
   static_assert(COL_O + ACC <= TILE_COLS && NT * TILE_COLS <= 512, "");
-  static constexpr float PART_COST = TANGENT ? 0.65f : 0.4f;  // see fwd_share_cost
+  static constexpr float PART_COST = WIDE ? 1e9f : (TANGENT ? 0.65f : 0.3f);  // see fwd_share_cost
 };
 
 // scratch record of one part of a split item: [ACC][ITEM_M] accumulators (a column per row of the
@@ -632,35 +635,40 @@ static size_t att_scratch_bytes(int B, int L, int H) {
   return G == n_items ? 0 : (size_t)G * 2 * att_part_floats<TANGENT, NTP>() * sizeof(float);
 }
 
-static long primal_items(int B, int L, int H, int nt) {
-  const int item_m = nt * ATT_TILE_M;
+static long primal_items(int B, int L, int H, int form) {
+  const int item_m = (form == ATT_WIDE ? 2 : form) * ATT_TILE_M;
   return (long)((L + item_m - 1) / item_m) * H * B;
 }
 
-// Query tiles per work item of the primal kernel: of two, three and four the one with the least time
-// by the following account.  A K/V tile takes 1.13, 1.19 and 1.43 us, so that with many items four
-// are the best (B 1, H 4, L 29,140: 1.01 ms, three 1.16, with exact row sums) unless rounding L up to
-// 512 rows wastes more than that gains over 384; with few items, SMs that would stand idle take smaller ones (H 4, L 532:
-// 15.7, 17.3 and 20.5 us).  A launch takes 5.1, 6.0 and 6.5 us besides, and the merge of split items
-// that are more than the SMs six tiles.  (177 shapes of 1 to 64 heads and 130 to 7,820 rows: 0.4 %
-// from the best of the six forms on average.)
-static int primal_nt(int B, int L, int H) {
-  constexpr float TILE_US[3] = {1.13f, 1.19f, 1.43f}, BASE_US[3] = {5.1f, 6.0f, 6.5f};
+// Form of the primal kernel's work items: of two, three and four query tiles, and two with K/V tiles of
+// 128 rows (never split), the one with the least time by the following account.  A K/V tile takes
+// 1.13, 1.26 and 1.46 us (1.95 for the double one), so that with many items four are the best
+// (B 1, H 4, L 29,140: 1.01 ms, three 1.16, both with exact row sums) unless rounding L up to 512 rows
+// wastes more than that gains; with few items, SMs that would stand idle take smaller ones
+// (H 4, L 532: two 15.7 us, three 17.3, four 20.5), and long walks the double tiles (H 24, L 1,000:
+// 23.0 us against 25.5 and, three, 29.9).  A launch takes 5 to 7 us besides, and the merge of split
+// items that are more than the SMs six tiles.  (165 shapes of 1 to 64 heads and 130 to 7,820 rows:
+// 0.4 % from the best form on average.)
+static int primal_form(int B, int L, int H) {
+  constexpr int FORMS[4] = {2, 3, 4, ATT_WIDE};
+  constexpr float TILE_US[4] = {1.13f, 1.26f, 1.46f, 1.95f}, BASE_US[4] = {5.1f, 6.5f, 7.0f, 5.7f};
   constexpr float PART_COST = AttCfg<false, 4>::PART_COST;
-  constexpr int BN = AttCfg<false, 4>::BN;
-  const int n_kv = (L + BN - 1) / BN, sms = fwd_sm_count();
+  const int sms = fwd_sm_count();
   int best = 4;
   if (B <= 0 || L <= 0 || H <= 0) return best;      // refused at the launch
-  float best_us = 0.f;
-  for (int nt = 2; nt <= 4; ++nt) {
-    const long items = primal_items(B, L, H, nt);
-    const int g = fwd_grid(items, n_kv, PART_COST);
+  float best_us = 1e30f;
+  for (int f = 0; f < 4; ++f) {
+    const bool wide = FORMS[f] == ATT_WIDE;
+    const long items = primal_items(B, L, H, FORMS[f]);
+    const int bn = wide ? AttCfg<false, ATT_WIDE>::BN : AttCfg<false, 4>::BN, n_kv = (L + bn - 1) / bn;
+    if (wide && items > sms) continue;
+    const int g = wide ? (int)items : fwd_grid(items, n_kv, PART_COST);
     const float walk = (float)((items * n_kv + g - 1) / g);
     const float tiles = items > sms ? walk + 6.f
                         : g == items ? walk : walk + fwd_share_cost(items, n_kv, g, PART_COST);
-    const float us = BASE_US[nt - 2] + TILE_US[nt - 2] * tiles;
-    if (nt == 2 || us < best_us) {
-      best = nt;
+    const float us = BASE_US[f] + TILE_US[f] * tiles;
+    if (us < best_us) {
+      best = FORMS[f];
       best_us = us;
     }
   }
@@ -673,7 +681,8 @@ static int primal_nt(int B, int L, int H) {
 extern "C" long imf_attn_fwd_scratch_bytes(int B, int L, int H, int tangent) {
   using namespace imf;
   if (tangent) return (long)att_scratch_bytes<true, 2>(B, L, H);
-  switch (primal_nt(B, L, H)) {
+  switch (primal_form(B, L, H)) {
+    case ATT_WIDE: return 0;
     case 2: return (long)att_scratch_bytes<false, 2>(B, L, H);
     case 3: return (long)att_scratch_bytes<false, 3>(B, L, H);
     default: return (long)att_scratch_bytes<false, 4>(B, L, H);
@@ -729,7 +738,8 @@ extern "C" int imf_attn_fwd(const void* q, const void* k, const void* v, const v
 #define IMF_PRIMAL(NT)                                                                              \
   return launch_attn_fwd<false, NT>(q, k, v, nullptr, nullptr, nullptr, strides, prm,               \
                                     (size_t)scratch_bytes, st)
-  switch (primal_nt(B, L, H)) {
+  switch (primal_form(B, L, H)) {
+    case ATT_WIDE: IMF_PRIMAL(ATT_WIDE);
     case 2: IMF_PRIMAL(2);
     case 3: IMF_PRIMAL(3);
     default: IMF_PRIMAL(4);
@@ -775,7 +785,7 @@ extern "C" int imf_attn_fwd_noalloc(const void* q, const void* k, const void* v,
   // problems of no more items than SMs leave the array alone (one CTA per item), so that short calls
   // on several streams share nothing
   const bool shares = B > 0 && L > 0 && H > 0 &&
-                      primal_items(B, L, H, primal_nt(B, L, H)) > fwd_sm_count();
+                      primal_items(B, L, H, primal_form(B, L, H)) > fwd_sm_count();
   const long need = shares ? imf_attn_fwd_scratch_bytes(B, L, H, 0) : 0;
   if (need > (long)(NOALLOC_FLOATS * sizeof(float))) {
     fprintf(stderr,

@@ -230,10 +230,12 @@ def test_attention_forward_divides_by_the_sum_of_rounded_weights(K, L, H, need_l
     K.check_status()
 
 
-@pytest.mark.parametrize("L,H", [(200, 3), (1000, 2), (850, 40), (2600, 8), (850, 64), (5200, 8)])
+@pytest.mark.parametrize("L,H", [(130, 3), (1000, 2), (850, 40), (2600, 8), (850, 64), (5200, 8), (200, 3),
+                                 (1000, 24), (2068, 16)])
 def test_attention_forward_items(K, L, H):
-    """The primal kernel's work items of two, three and four query tiles, each whole and in shares (in
-    this order two whole, two, three whole, three, four whole, four on 148 SMs); bounds as above."""
+    """The primal kernel's work items of two, three and four query tiles, each whole and in shares, and
+    of two with 128-row K/V tiles whose last one has 72, 104 and 20 rows (in this order two whole,
+    two, three whole, three, four whole, four on 148 SMs); bounds as above."""
     from imfvideo_b200.ops import reference as ref
 
     g = torch.Generator(device="cuda").manual_seed(L + H)
