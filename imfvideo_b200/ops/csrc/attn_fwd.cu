@@ -10,7 +10,8 @@
 // flash-JVP kernel (reference models/flash_jvp_kernel.py:51-570,
 // models/triton_block_jvp.py:228-346) and the FA/SDPA primal forward.
 //
-// Work item = NT 128-row query tiles that share every 64-row K/V tile, of one (batch,
+// The tangent is attn_jvp.cu's business except for short problems of more query tiles than SMs, see
+// tangent_pairs.  Work item = NT 128-row query tiles that share every 64-row K/V tile, of one (batch,
 // head): four tiles in the primal kernel (three or two where rounding L up to 512 rows wastes more
 // than that gains or SMs would stand idle, see primal_form), two in the tangent kernel; TMEM (512
 // columns) holds no more.  Warps
@@ -33,6 +34,7 @@
 // Tensors are (B, L, H, 64) bf16 with arbitrary 16-byte-aligned strides;
 // ragged L is handled by TMA zero fill + masking of the last K/V tile.
 #include "attn_fwd128.h"
+#include "attn_jvp.h"
 #include "attn_fwd_split.h"
 #include "common.cuh"
 #include "host_util.h"
@@ -635,6 +637,17 @@ static size_t att_scratch_bytes(int B, int L, int H) {
   return G == n_items ? 0 : (size_t)G * 2 * att_part_floats<TANGENT, NTP>() * sizeof(float);
 }
 
+// With tangent: one query tile per item (attn_jvp.cu) is 1.1 to 2 times faster than two, but a CTA's
+// next item costs 7 us more than its K/V tiles.  So where the tiles are more than the SMs, pairs are
+// not, and walks are of nine K/V tiles at most, two: H 80, L 130 12.4 us against 17.4; B 2, H 24, L 532
+// 23.9 and 24.9; B 2, H 24, L 700 27.3 and 26.7.
+static bool tangent_pairs(int B, int L, int H) {
+  const long pairs = (long)((L + 2 * ATT_TILE_M - 1) / (2 * ATT_TILE_M)) * H * B;
+  const long tiles = (long)((L + ATT_TILE_M - 1) / ATT_TILE_M) * H * B;
+  const int sms = fwd_sm_count();
+  return pairs <= sms && tiles > sms && L <= 9 * AttCfg<true, 2>::BN;
+}
+
 static long primal_items(int B, int L, int H, int form) {
   const int item_m = (form == ATT_WIDE ? 2 : form) * ATT_TILE_M;
   return (long)((L + item_m - 1) / item_m) * H * B;
@@ -680,7 +693,9 @@ static int primal_form(int B, int L, int H) {
 // Bytes of scratch the forward takes for (B, L, H): 0 when no item is split.
 extern "C" long imf_attn_fwd_scratch_bytes(int B, int L, int H, int tangent) {
   using namespace imf;
-  if (tangent) return (long)att_scratch_bytes<true, 2>(B, L, H);
+  if (B <= 0 || L <= 0 || H <= 0) return 0;       // refused at the launch
+  if (tangent)
+    return tangent_pairs(B, L, H) ? (long)att_scratch_bytes<true, 2>(B, L, H) : attn_jvp_scratch_bytes(B, L, H);
   switch (primal_form(B, L, H)) {
     case ATT_WIDE: return 0;
     case 2: return (long)att_scratch_bytes<false, 2>(B, L, H);
@@ -710,12 +725,11 @@ extern "C" int imf_attn_fwd(const void* q, const void* k, const void* v, const v
   if ((head_dim != ATT_HD && head_dim != 128) || B <= 0 || L <= 0 || H <= 0) return IMF_ERR_ARG;
   if ((o_sl & 7) || (o_sh & 7) || (o_sb & 7) || (reinterpret_cast<uintptr_t>(o) & 15))
     return IMF_ERR_ARG;
-  if (head_dim == 128) {
-    if (dq != nullptr && (dout == nullptr || (reinterpret_cast<uintptr_t>(dout) & 15)))
-      return IMF_ERR_ARG;
+  if (dq != nullptr && (dout == nullptr || (reinterpret_cast<uintptr_t>(dout) & 15))) return IMF_ERR_ARG;
+  if (head_dim == 128 || (dq != nullptr && !tangent_pairs(B, L, H))) {
     Fwd128Args a{q, k, v, dq, dk, dv, o, dout, lse, B, L, H, strides, o_sb, o_sl, o_sh, scale,
                  scratch, scratch_bytes, status, stream};
-    return attn_fwd128_launch(a);
+    return head_dim == 128 ? attn_fwd128_launch(a) : attn_jvp_launch(a);
   }
   AttParams prm;
   prm.o = static_cast<__nv_bfloat16*>(o);
@@ -732,7 +746,6 @@ extern "C" int imf_attn_fwd(const void* q, const void* k, const void* v, const v
   prm.status = status;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dq != nullptr) {
-    if (dout == nullptr || (reinterpret_cast<uintptr_t>(dout) & 15)) return IMF_ERR_ARG;
     return launch_attn_fwd<true, 2>(q, k, v, dq, dk, dv, strides, prm, (size_t)scratch_bytes, st);
   }
 #define IMF_PRIMAL(NT)                                                                              \

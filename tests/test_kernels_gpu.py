@@ -246,6 +246,25 @@ def test_attention_forward_items(K, L, H):
     K.check_status()
 
 
+@pytest.mark.parametrize("B,L,H,scale", [(1, 64, 1, 0.125), (1, 65, 1, 0.125), (1, 129, 2, 1.0), (1, 193, 1, 0.1),
+                                         (1, 300, 2, 2.0 ** -8), (1, 300, 2, 2.0 ** -9), (3, 140, 60, 0.125),
+                                         (1, 130, 80, 0.125), (1, 600, 40, 0.125), (1, 2600, 2, 0.125)])
+def test_attention_forward_tangent_items(K, B, L, H, scale):
+    """The tangent kernel's steps alternate between two groups of warps: one step, two, three and four
+    of them; scales that are powers of two (multiplied into q and dq) and others; three rounds of whole
+    items, items of two query tiles, two rounds, shares (in this order, on 148 SMs).  Bounds as above."""
+    from imfvideo_b200.ops import reference as ref
+
+    g = torch.Generator(device="cuda").manual_seed(L + H)
+    q, k, v, dq, dk, dv = (torch.randn(B, L, H, 64, device="cuda", generator=g).bfloat16() for _ in range(6))
+    f = lambda t: t.float()
+    ro, rdo = ref.attention_jvp(*map(f, (q, k, v, dq, dk, dv)), scale=scale)
+    o, do, lse = K.attn_fwd(q, k, v, dq, dk, dv, scale=scale)
+    assert _rel(o, ro) < 6e-3 and _rel(do, rdo) < 1.2e-2
+    assert (lse - ref.attention_lse(f(q), f(k), scale=scale)).abs().max() < 1e-3
+    K.check_status()
+
+
 @pytest.mark.parametrize("hd", [64, 128])
 @pytest.mark.parametrize("B,L,H", [(1, 576, 4), (1, 7040, 10)])
 @pytest.mark.parametrize("scale", [0.0, -0.1])
