@@ -17,11 +17,12 @@
 //   primal  : two 128-row query tiles per item, per tile S (64) + O (128) + P (bf16, 32);
 //             four softmax warps per tile.  P has columns of its own, so S is free again once the
 //             softmax warps have it in registers, and the next Q K^T runs while they are at the
-//             exponentials; Q K^T and P V are issued by two warps, so that neither waits for the
-//             other's barriers.  B 1, L 7,820, H 12: 402 -> 358 us (loop 425 -> 390); L 32,780, H 4
-//             2.28 -> 2.09 ms in a loop; before, P lay over S and one warp issued P V, then
-//             the next Q K^T.  The tensor core needs 640 clocks of a tile's step (Q K^T 8 x 48 at 128 B
-//             of operands per clock, P V 4 x 64), the exponential unit 512; a step takes 1,090.
+//             exponentials, and P is stored as it is made (maximum first).  Q K^T and P V are
+//             issued by two warps, so that neither waits for the other's barriers.  B 1, L 7,820,
+//             H 12: 402 -> 311 us (loop 425 -> 360); L 32,780, H 4 2.28 -> 1.90 ms in a loop; before,
+//             P lay over S and one warp issued P V, then the next Q K^T (P beside S and two warps
+//             alone: 350 and 390 us).  The tensor core needs 640 clocks of a tile's step (Q K^T 8 x 48
+//             at 128 B of operands per clock, P V 4 x 64), the exponential unit 512; a step takes 950.
 //   tangent : ONE query tile per item, O (128) + dO (128) and TWO S|dS buffers
 //             (64 + 64 each), so Q K^T of K/V tile j+1 runs on the tensor core
 //             while the CUDA cores do the softmax of tile j.  Eight softmax
@@ -416,61 +417,15 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           for (int i = 0; i < NC; ++i)
             if (i >= kv_rem) sv[i] = 0xff800000u;  // -inf
         }
-        // The exponentials are taken against the reference maximum that the rows already have
-        // while the new maximum is formed alongside; only when a row has outgrown its reference
-        // by more than 2^8 (or has none yet) is the reference moved, O rescaled and the tile done
-        // again from the scores, which are still in registers.
         const bool first = j == sg.j0;
-        uint32_t pk[NC / 2];
-        uint32_t tk[TANGENT ? NC / 2 : 1];
         float alpha = 1.f;
-        f32x2 l_new, mu_new;
-        for (bool redo = false;; redo = true) {
-          const f32x2 neg_m2 = dup2(-m_used * scale_log2);
-          l_new = mu_new = dup2(0.f);
-          float mx0 = -INFINITY, mx1 = -INFINITY;
-#pragma unroll
-          for (int i = 0; i < NC; i += 2) {
-            float& mxi = (i & 2) ? mx1 : mx0;
-            asm("max.f32 %0, %0, %1, %2;" : "+f"(mxi) : "f"(__uint_as_float(sv[i])), "f"(__uint_as_float(sv[i + 1])));
-            const f32x2 e = fma2(pair2(sv[i], sv[i + 1]), dup2(scale_log2), neg_m2);
-            const float p0 = ex2(lo2(e)), p1 = ex2(hi2(e));
-            const f32x2 pp = pair2(__float_as_uint(p0), __float_as_uint(p1));
-            pk[i / 2] = pack_bf16(p0, p1);
-            l_new = add2(l_new, pp);
-            if (TANGENT) {
-              const f32x2 tt = mul2(mul2(pp, pair2(dsv[i], dsv[i + 1])), dup2(p.scale));
-              mu_new = add2(mu_new, tt);
-              tk[i / 2] = pack_bf16(lo2(tt), hi2(tt));
-            }
-          }
-          if (redo) break;
-          float mx = fmaxf(mx0, mx1);
-          if (C::SPLIT) {
-            // both column halves of a row must use the same maximum.  The exchange is also the
-            // point after which every S / dS column of this buffer has been read, so the bf16
-            // P / T written below may overlap the partner's score columns.
-            s.xmx[it & 1][half][row] = mx;
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&s.xbar);
-            ok = __all_sync(0xffffffffu, mbar_wait(&s.xbar, xn & 1, abort_flag, p.status,
-                                                   STATUS_TIMEOUT_SOFTMAX));
-            ++xn;
-            if (!ok) break;
-            mx = fmaxf(mx, s.xmx[it & 1][half ^ 1][row]);
-          }
-          const bool need = first || (mx - m_used) * scale_log2 > 8.0f;
-          if (!__any_sync(0xffffffffu, need)) break;
-          if (need) {
-            if (!first) alpha = ex2((m_used - mx) * scale_log2);
-            m_used = mx;
-          }
-          if (first) continue;               // nothing in O yet
-          ok = __all_sync(0xffffffffu, mbar_wait(&s.o_done[t], (uint32_t)((it - 1) & 1),
-                                                 abort_flag, p.status, STATUS_TIMEOUT_MMA));
-          if (!ok) break;
+        // O, once P V of the step before has run, to the reference maximum that the rows have now; split
+        // rows: half 0 rescales O, half 1 dO
+        auto rescale = [&]() {
+          if (!__all_sync(0xffffffffu, mbar_wait(&s.o_done[t], (uint32_t)((it - 1) & 1), abort_flag,
+                                                 p.status, STATUS_TIMEOUT_MMA)))
+            return false;
           tc_fence_after();
-          // split rows: half 0 rescales O, half 1 rescales dO
           const uint32_t rb = tb + (C::SPLIT && half ? C::COL_DO : C::COL_O);
 #pragma unroll 1
           for (int c = 0; c < HD; c += 32) {
@@ -482,24 +437,102 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             tmem_st32(rb + c, ov);
           }
           tc_wait_st();
-        }
-        if (!ok) break;
-        l_sum = fmaf(l_sum, alpha, lo2(l_new));
-        l_sum2 = fmaf(l_sum2, alpha, hi2(l_new));
-        if (TANGENT) {
+          return true;
+        };
+        if constexpr (TANGENT) {
+          // The exponentials are taken against the reference maximum that the rows already have
+          // while the new maximum is formed alongside; only when a row has outgrown its reference
+          // by more than 2^8 (or has none yet) is the reference moved, O rescaled and the tile done
+          // again from the scores, which are still in registers.
+          uint32_t pk[NC / 2];
+          uint32_t tk[NC / 2];
+          f32x2 l_new, mu_new;
+          for (bool redo = false;; redo = true) {
+            const f32x2 neg_m2 = dup2(-m_used * scale_log2);
+            l_new = mu_new = dup2(0.f);
+            float mx0 = -INFINITY, mx1 = -INFINITY;
+#pragma unroll
+            for (int i = 0; i < NC; i += 2) {
+              float& mxi = (i & 2) ? mx1 : mx0;
+              asm("max.f32 %0, %0, %1, %2;" : "+f"(mxi) : "f"(__uint_as_float(sv[i])), "f"(__uint_as_float(sv[i + 1])));
+              const f32x2 e = fma2(pair2(sv[i], sv[i + 1]), dup2(scale_log2), neg_m2);
+              const float p0 = ex2(lo2(e)), p1 = ex2(hi2(e));
+              const f32x2 pp = pair2(__float_as_uint(p0), __float_as_uint(p1));
+              pk[i / 2] = pack_bf16(p0, p1);
+              l_new = add2(l_new, pp);
+              const f32x2 tt = mul2(mul2(pp, pair2(dsv[i], dsv[i + 1])), dup2(p.scale));
+              mu_new = add2(mu_new, tt);
+              tk[i / 2] = pack_bf16(lo2(tt), hi2(tt));
+            }
+            if (redo) break;
+            float mx = fmaxf(mx0, mx1);
+            // both column halves of a row must use the same maximum.  The exchange is also the
+            // point after which every S / dS column of this buffer has been read, so the bf16
+            // P / T written below may overlap the partner's score columns.
+            s.xmx[it & 1][half][row] = mx;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s.xbar);
+            ok = __all_sync(0xffffffffu, mbar_wait(&s.xbar, xn & 1, abort_flag, p.status,
+                                                   STATUS_TIMEOUT_SOFTMAX));
+            ++xn;
+            if (!ok) break;
+            mx = fmaxf(mx, s.xmx[it & 1][half ^ 1][row]);
+            const bool need = first || (mx - m_used) * scale_log2 > 8.0f;
+            if (!__any_sync(0xffffffffu, need)) break;
+            if (need) {
+              if (!first) alpha = ex2((m_used - mx) * scale_log2);
+              m_used = mx;
+            }
+            if (first) continue;               // nothing in O yet
+            ok = rescale();
+            if (!ok) break;
+          }
+          if (!ok) break;
+          l_sum = fmaf(l_sum, alpha, lo2(l_new));
+          l_sum2 = fmaf(l_sum2, alpha, hi2(l_new));
           mu_sum = fmaf(mu_sum, alpha, lo2(mu_new));
           mu_sum2 = fmaf(mu_sum2, alpha, hi2(mu_new));
-        }
-        if (!TANGENT && !__all_sync(0xffffffffu, p_ok)) {
-          ok = __all_sync(0xffffffffu, mbar_wait(&s.o_done[t], (uint32_t)((it - 1) & 1), abort_flag,
-                                                 p.status, STATUS_TIMEOUT_MMA));
-          if (!ok) break;
-          tc_fence_after();
-        }
+          tmem_st16(tb + C::col_p(buf) + c0 / 2, pk);
+          tmem_st16(tb + C::col_ds(buf) + c0 / 2, tk);
+        } else {
+          // Maximum first, so that P can be stored as it is made.  The reference moves only when a row
+          // has outgrown it by more than 2^8.
+          float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int c = 0; c < NC; c += 32) {
-          tmem_st16(tb + C::col_p(buf) + (c0 + c) / 2, pk + c / 2);
-          if (TANGENT) tmem_st16(tb + C::col_ds(buf) + (c0 + c) / 2, tk + c / 2);
+          for (int i = 0; i < NC; i += 2)
+            asm("max.f32 %0, %0, %1, %2;" : "+f"(mx[(i / 2) & 3]) : "f"(__uint_as_float(sv[i])), "f"(__uint_as_float(sv[i + 1])));
+          mx[0] = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+          const bool need = first || (mx[0] - m_used) * scale_log2 > 8.0f;
+          if (__any_sync(0xffffffffu, need)) {
+            if (need) {
+              if (!first) alpha = ex2((m_used - mx[0]) * scale_log2);
+              m_used = mx[0];
+            }
+            if (!first) ok = rescale();
+            if (!ok) break;
+          }
+          if (!__all_sync(0xffffffffu, p_ok)) {      // P of the step before is still being read
+            ok = __all_sync(0xffffffffu, mbar_wait(&s.o_done[t], (uint32_t)((it - 1) & 1), abort_flag,
+                                                   p.status, STATUS_TIMEOUT_MMA));
+            if (!ok) break;
+          }
+          tc_fence_after();
+          const f32x2 neg_m2 = dup2(-m_used * scale_log2);
+          f32x2 l_new = dup2(0.f);
+#pragma unroll
+          for (int c = 0; c < NC; c += 32) {
+            uint32_t pk[32 / 2];
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) {
+              const f32x2 e = fma2(pair2(sv[c + i], sv[c + i + 1]), dup2(scale_log2), neg_m2);
+              const float p0 = ex2(lo2(e)), p1 = ex2(hi2(e));
+              pk[i / 2] = pack_bf16(p0, p1);
+              l_new = add2(l_new, pair2(__float_as_uint(p0), __float_as_uint(p1)));
+            }
+            tmem_st16(tb + C::col_p(0) + c / 2, pk);
+          }
+          l_sum = fmaf(l_sum, alpha, lo2(l_new));
+          l_sum2 = fmaf(l_sum2, alpha, hi2(l_new));
         }
         tc_wait_st();
         tc_fence_before();
