@@ -187,7 +187,12 @@ __global__ void __launch_bounds__(256, TANGENT ? 2 : 4) lin_states_kernel(const 
   const int g = lane >> 2, t = lane & 3, mr = (warp & 3) * 16, nc = (warp >> 2) * 32;
   float acc[4][4] = {}, dacc[4][4] = {};
   float fr[4][4] = {}, dfr[4][4] = {};       // accumulator fragments of X^T Y and its tangent
-  float zacc = 0.f, dzacc = 0.f;
+  // the extra column, sum of phi weighted by w: every lane its two columns of its warp's rows, the
+  // eight warps' sums added in order at the end (64 threads walking the 64 rows in shared memory while
+  // six warps waited: 57 us a launch at 29,140 rows x 4 heads, 53 this way; what bounds it is
+  // 2,000 instructions a warp, 0.48 per clock and scheduler)
+  __shared__ float zs[TANGENT ? 2 : 1][8][64];
+  float2 zacc = make_float2(0.f, 0.f), dzacc = zacc;
   for (int c0 = 0; c0 < a.bs; c0 += 64) {
     // Every warp has eight rows.  All their loads are issued before the first softmax (a
     // row at a time would put eight global-memory latencies end to end), and the unrolled
@@ -220,7 +225,8 @@ __global__ void __launch_bounds__(256, TANGENT ? 2 : 4) lin_states_kernel(const 
       }
       *reinterpret_cast<float2*>(X + rr * LP + 2 * lane) = phi;
       *reinterpret_cast<float2*>(Y + rr * LP + 2 * lane) = yr[i];
-      if (lane == 0) Y[rr * LP + 64] = wr[i];
+      zacc = make_float2(fmaf(phi.x, wr[i], zacc.x), fmaf(phi.y, wr[i], zacc.y));
+      if (TANGENT) dzacc = make_float2(fmaf(dphi.x, wr[i], dzacc.x), fmaf(dphi.y, wr[i], dzacc.y));
       if (TANGENT) {
         *reinterpret_cast<float2*>(dX + rr * LP + 2 * lane) = dphi;
         *reinterpret_cast<float2*>(dY + rr * LP + 2 * lane) = dyr[i];
@@ -233,16 +239,11 @@ __global__ void __launch_bounds__(256, TANGENT ? 2 : 4) lin_states_kernel(const 
       warp_mm_tf32<true>(dX, Y, mr, nc, g, t, dfr);
       warp_mm_tf32<true>(X, dY, mr, nc, g, t, dfr);
     }
-    if (tid < 64) {                  // the extra column: sum of phi weighted by w
-#pragma unroll 8
-      for (int rr = 0; rr < 64; ++rr) {
-        const float wv = Y[rr * LP + 64];
-        zacc = fmaf(X[rr * LP + tid], wv, zacc);
-        if (TANGENT) dzacc = fmaf(dX[rr * LP + tid], wv, dzacc);
-      }
-    }
     __syncthreads();
   }
+  *reinterpret_cast<float2*>(&zs[0][warp][2 * lane]) = zacc;
+  if (TANGENT) *reinterpret_cast<float2*>(&zs[TANGENT ? 1 : 0][warp][2 * lane]) = dzacc;
+  __syncthreads();
   frags_to_blocks(fr, S, mr, nc, g, t, d0, e0, acc);
   if (TANGENT) frags_to_blocks(dfr, S, mr, nc, g, t, d0, e0, dacc);
   const int64_t base = ((int64_t)b * a.H + h) * 2 * a.nblk_pad * LSTATE + (int64_t)n * LSTATE;
@@ -269,8 +270,14 @@ __global__ void __launch_bounds__(256, TANGENT ? 2 : 4) lin_states_kernel(const 
     if (TANGENT) put4(a.dout, d0 + i, e0, dacc[i]);
   }
   if (tid < 64) {
-    put(a.out, tid, 64, zacc);
-    if (TANGENT) put(a.dout, tid, 64, dzacc);
+    float z = 0.f, dz = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      z += zs[0][i][tid];
+      if (TANGENT) dz += zs[TANGENT ? 1 : 0][i][tid];
+    }
+    put(a.out, tid, 64, z);
+    if (TANGENT) put(a.dout, tid, 64, dz);
 #pragma unroll
     for (int e = 65; e < LW; ++e) {
       put(a.out, tid, e, 0.f);
