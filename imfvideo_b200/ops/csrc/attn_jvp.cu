@@ -373,6 +373,16 @@ attn_jvp_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         for (int i = 0; i < BN; i += 2)
           asm("max.f32 %0, %0, %1, %2;" : "+f"(mx[(i / 2) & 3]) : "f"(__uint_as_float(sv[i])), "f"(__uint_as_float(sv[i + 1])));
         mx[0] = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+        // P V of this group's step before, n - 2, is seen to be over before the reference of step n is
+        // published: whoever has that reference and asks o_done for P V of step n then finds the barrier
+        // in that phase or one further.  (A wait by parity on a barrier still two phases back returns at
+        // once: V late by two steps, and O would be rescaled under products that are still to run.)
+        // P of step n may be written from here on, too.
+        if (!__all_sync(0xffffffffu, p_ok)) {
+          ok = __all_sync(0xffffffffu, mbar_wait(&s.o_done[g], par ^ 1, abort_flag, p.status, STATUS_TIMEOUT_MMA));
+          if (!ok) break;
+        }
+        tc_fence_after();
         // The reference is moved only when a row has outgrown it by more than 2^8 (or has none yet)
         float m_prev;
         ok = ref_of_step(&s.m_ref[row], n - 1, m_prev, abort_flag, p.status);
@@ -408,11 +418,6 @@ attn_jvp_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           }
           m_used = m_new;
         }
-        if (!__all_sync(0xffffffffu, p_ok)) {
-          ok = __all_sync(0xffffffffu, mbar_wait(&s.o_done[g], par ^ 1, abort_flag, p.status, STATUS_TIMEOUT_MMA));
-          if (!ok) break;
-        }
-        tc_fence_after();
         const f32x2 neg_m2 = dup2(-m_used * scale_log2);
         f32x2 l_new = dup2(0.f), mu_new = dup2(0.f);
         uint32_t dsv[2][32];

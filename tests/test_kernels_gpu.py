@@ -265,6 +265,29 @@ def test_attention_forward_tangent_items(K, B, L, H, scale):
     K.check_status()
 
 
+@pytest.mark.parametrize("B,L,H", [(1, 2049, 2), (2, 2600, 4), (1, 600, 58), (3, 140, 60)])
+@pytest.mark.parametrize("scale", [0.125, 0.1])
+def test_attention_forward_tangent_growing_keys(K, B, L, H, scale):
+    """Keys that grow along the sequence: rows outgrow their reference maximum in step after step, which one
+    group of warps finds and the other has to take over.  Shares of few items and of more than SMs, whole
+    items in two and three rounds (on 148 SMs); either form of the scale.  Bounds as above; run twice: same
+    bits."""
+    from imfvideo_b200.ops import reference as ref
+
+    g = torch.Generator(device="cuda").manual_seed(L + H)
+    mk = lambda s=1.0: (torch.randn(B, L, H, 64, device="cuda", generator=g) * s).bfloat16()
+    q, k, v, dq, dk, dv = mk(), mk(), mk(), mk(.5), mk(.5), mk(.5)
+    k = (k * torch.linspace(0.05, 12.0, L, device="cuda").view(1, L, 1, 1)).bfloat16()
+    f = lambda t: t.float()
+    ro, rdo = ref.attention_jvp(*map(f, (q, k, v, dq, dk, dv)), scale=scale)
+    o, do, lse = K.attn_fwd(q, k, v, dq, dk, dv, scale=scale)
+    assert _rel(o, ro) < 6e-3 and _rel(do, rdo) < 1.2e-2
+    assert (lse - ref.attention_lse(f(q), f(k), scale=scale)).abs().max() < 1e-3
+    again = K.attn_fwd(q, k, v, dq, dk, dv, scale=scale)
+    assert all(torch.equal(a, b) for a, b in zip((o, do, lse), again))
+    K.check_status()
+
+
 @pytest.mark.parametrize("hd", [64, 128])
 @pytest.mark.parametrize("B,L,H", [(1, 576, 4), (1, 7040, 10)])
 @pytest.mark.parametrize("scale", [0.0, -0.1])
