@@ -82,7 +82,7 @@ struct Smem {
   alignas(1024) uint8_t q[2][QTILE];               // q, dq
   alignas(1024) uint8_t k[STAGES][2 * KTILE];      // k, dk
   alignas(1024) uint8_t v[STAGES][2 * KTILE];      // v, dv
-  int2 m_ref[TM];           // reference maximum of the row as of the last step decided, that step's number
+  uint64_t m_ref[TM];       // reference maximum of the row as of the last step decided | that step's number
   float xst[2][3][TM];      // l, mu and reference maximum of either group, at a segment's end
   uint64_t q_full, q_empty, q_ready;
   uint64_t k_full[STAGES], k_empty[STAGES];
@@ -136,15 +136,24 @@ IMF_DEVICE void scale_queries(uint8_t (&q)[2][QTILE], float f) {
   __syncwarp();
 }
 
-// The row's reference maximum as step `n` left it, from the warp of the other group (which decided long
-// before as a rule).  Bounded; false: gave up.
-IMF_DEVICE bool ref_of_step(const int2* addr, int n, float& m, volatile int* abort_flag, int* status) {
+// The row's reference maximum as step `n` left it goes to the warp of the other group in one 64-bit word,
+// the step's number in its upper half.  One scalar access each way: a vector of two words is two accesses
+// in no order, and the number could be seen before the maximum that it stands for.
+IMF_DEVICE uint64_t ref_word(float m, int n) {
+  return (uint64_t)(uint32_t)n << 32 | __float_as_uint(m);
+}
+IMF_DEVICE void publish_ref(uint64_t* addr, float m, int n) {
+  asm volatile("st.volatile.shared.b64 [%0], %1;" ::"r"(smem_u32(addr)), "l"(ref_word(m, n)) : "memory");
+}
+
+// From the other group's warp, which decided long before as a rule.  Bounded; false: gave up.
+IMF_DEVICE bool ref_of_step(const uint64_t* addr, int n, float& m, volatile int* abort_flag, int* status) {
   uint64_t t0 = 0;
   for (uint32_t spins = 1;; ++spins) {
-    int x, step;
-    asm volatile("ld.volatile.shared.v2.s32 {%0, %1}, [%2];" : "=r"(x), "=r"(step) : "r"(smem_u32(addr)) : "memory");
-    m = __int_as_float(x);
-    if (__all_sync(0xffffffffu, step >= n)) return true;
+    uint64_t word;
+    asm volatile("ld.volatile.shared.b64 %0, [%1];" : "=l"(word) : "r"(smem_u32(addr)) : "memory");
+    m = __uint_as_float((uint32_t)word);
+    if (__all_sync(0xffffffffu, (int)(word >> 32) >= n)) return true;
     if ((spins & 63u) == 0) {
       if (__any_sync(0xffffffffu, *abort_flag)) return false;
       const uint64_t now = globaltimer_ns();
@@ -191,7 +200,7 @@ attn_jvp_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     s.abort_flag = 0;
     fence_barrier_init();
   }
-  if (threadIdx.x < TM) s.m_ref[threadIdx.x] = make_int2(0, -1);
+  if (threadIdx.x < TM) s.m_ref[threadIdx.x] = ref_word(0.f, -1);
   if (warp == WARP_QK) {
     tmem_alloc(&s.tmem_base, 512);
     tmem_relinquish();
@@ -390,8 +399,7 @@ attn_jvp_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (j == sg.j0) m_prev = mx[0];
         const bool need = (mx[0] - m_prev) * scale_log2 > 8.0f;
         const float m_new = need ? mx[0] : m_prev;
-        asm volatile("st.volatile.shared.v2.s32 [%0], {%1, %2};" ::"r"(smem_u32(&s.m_ref[row])),
-                     "r"(__float_as_int(m_new)), "r"(n) : "memory");
+        publish_ref(&s.m_ref[row], m_new, n);
         if (__any_sync(0xffffffffu, m_new != m_used)) {
           if (__any_sync(0xffffffffu, need)) {      // O, as of the step before, to the new reference
             ok = __all_sync(0xffffffffu, mbar_wait(&s.o_done[g ^ 1], g == 0 ? par ^ 1 : par, abort_flag,
