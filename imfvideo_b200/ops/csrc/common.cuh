@@ -365,6 +365,10 @@ IMF_DEVICE void tmem_st8(uint32_t taddr, const uint32_t* r) {
                ::"r"(taddr), IMF_ST_ARGS8(r, 0)
                : "memory");
 }
+// eight columns, one value
+IMF_DEVICE void tmem_fill8(uint32_t taddr, uint32_t r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr), "r"(r) : "memory");
+}
 IMF_DEVICE void tmem_st16(uint32_t taddr, const uint32_t* r) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "

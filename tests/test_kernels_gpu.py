@@ -265,6 +265,26 @@ def test_attention_forward_tangent_items(K, B, L, H, scale):
     K.check_status()
 
 
+@pytest.mark.parametrize("rem", [1, 7, 8, 9, 31, 56, 57, 63])
+@pytest.mark.parametrize("tiles,scale", [(0, 0.125), (2, 0.1)])
+def test_attention_forward_tangent_ragged_tail(K, rem, tiles, scale):
+    """Keys of a partial last K/V tile, their number around the groups of eight columns in which the rest
+    is masked.  Bounds as above."""
+    from imfvideo_b200.ops import reference as ref
+
+    L = 64 * tiles + rem
+    g = torch.Generator(device="cuda").manual_seed(L)
+    q, k, v, dq, dk, dv = (torch.randn(1, L, 2, 64, device="cuda", generator=g).bfloat16() for _ in range(6))
+    f = lambda t: t.float()
+    ro, rdo = ref.attention_jvp(*map(f, (q, k, v, dq, dk, dv)), scale=scale)
+    o, do, lse = K.attn_fwd(q, k, v, dq, dk, dv, scale=scale)
+    assert _rel(o, ro) < 6e-3
+    # one key: the tangent of o is dv, with whatever P dS V leaves of cancelled bf16 products beside it
+    assert (do.float() - rdo).norm() < 1.2e-2 * max(rdo.norm(), v.float().norm())
+    assert (lse - ref.attention_lse(f(q), f(k), scale=scale)).abs().max() < 1e-3
+    K.check_status()
+
+
 @pytest.mark.parametrize("B,L,H", [(1, 2049, 2), (2, 2600, 4), (1, 600, 58), (3, 140, 60)])
 @pytest.mark.parametrize("scale", [0.125, 0.1])
 def test_attention_forward_tangent_growing_keys(K, B, L, H, scale):
