@@ -638,14 +638,21 @@ static size_t att_scratch_bytes(int B, int L, int H) {
 }
 
 // With tangent: one query tile per item (attn_jvp.cu) is 1.1 to 2 times faster than two, but a CTA's
-// next item costs 7 us more than its K/V tiles.  So where the tiles are more than the SMs, pairs are
-// not, and walks are of nine K/V tiles at most, two: H 80, L 130 12.4 us against 17.4; B 2, H 24, L 532
-// 23.9 and 24.9; B 2, H 24, L 700 27.3 and 26.7.
+// next item costs 5 us more than its K/V tiles.  So two where that counts:
+//  - the tiles are more than the SMs, pairs are not, and walks are of nine K/V tiles at most: H 80, L 133
+//    12.5 us against 16.0; B 3, H 40, L 205 14.8 and 16.9; H 48, L 576 24.0 and 24.6; B 3, H 16, L 955 32.9 and 32.8;
+//  - walks of three K/V tiles in many rounds.  A round of tiles costs 6.3 us there, pairs 16.5 us and 8.1 us for
+//    each of the SMs' number: B 8, H 128, L 145 (13.8 tiles an SM) 74.6 us against 82.5; B 6, H 80, L 143 (6.5)
+//    44.5 and 48.3; B 16, H 32, L 137 (6.9) 45.2 and 43.2.  Of four K/V tiles pairs take 75 us and tiles 72
+//    at 10.4 an SM, B 12, H 64, L 200.
 static bool tangent_pairs(int B, int L, int H) {
   const long pairs = (long)((L + 2 * ATT_TILE_M - 1) / (2 * ATT_TILE_M)) * H * B;
   const long tiles = (long)((L + ATT_TILE_M - 1) / ATT_TILE_M) * H * B;
-  const int sms = fwd_sm_count();
-  return pairs <= sms && tiles > sms && L <= 9 * AttCfg<true, 2>::BN;
+  const int sms = fwd_sm_count(), n_kv = (L + AttCfg<true, 2>::BN - 1) / AttCfg<true, 2>::BN;
+  if (tiles <= sms) return false;
+  if (pairs <= sms) return n_kv <= 9;
+  const long rounds = (tiles + sms - 1) / sms;
+  return n_kv == 3 && (float)rounds > 2.7f + 1.3f * (float)pairs / (float)sms;
 }
 
 static long primal_items(int B, int L, int H, int form) {

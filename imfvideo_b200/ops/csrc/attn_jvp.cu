@@ -559,12 +559,17 @@ attn_jvp_combine_kernel(const Params p, int G) {
 }
 
 // Whole items, CTA c taking items c, c + G, ..., or equal shares of the (item, K/V tile) space with a
-// merge.  In K/V tiles (0.57 us each): a further round of whole items costs some 12 for the epilogue,
-// the next queries' load and an empty pipeline; shares of more items than SMs cost 32 for the two parts
-// that each CTA stores and the merge, of fewer what fwd_share_cost says with PART_COST.  Fitted to 122
-// shapes of 1 to 80 heads and 130 to 6,500 rows timed both ways (1 head, 6,500 rows 63.5 us whole, 41.8
-// shared; 8 heads, 2,068 rows 28.4 and 37.1; B 4, H 16, L 532 33.0 and 38.2; H 16, L 2,500 90.6 and 77.9).
-constexpr float PART_COST = 2.2f, ROUND_COST = 12.f, ALL_SPLIT_COST = 32.f;
+// merge.  Either way an item costs some 5 us besides its K/V tiles (queries' load, empty pipeline,
+// epilogue), so only what differs is counted, in K/V tiles of 0.57 to 0.7 us.  Shares of more items than
+// SMs cost 18 for the two parts that each CTA stores and the merge; where all heads' K | dK | V | dV,
+// which shares walk at once and rounds a few heads at a time, are more than L2 holds, 5 % of the walk
+// besides (half of such shapes lose more, up to 40 %).  Shares of fewer items cost what fwd_share_cost
+// says with PART_COST.  986 shapes of 1 to 128 heads and 64 to 32,760 rows in 2 to 70 rounds, either way
+// timed in turn: 0.2 % behind the better one on average (8 % when a round was charged 12 tiles and shares
+// 32).  Whole and shared: B 3, H 96, L 192, four rounds 30.6 us and 58.4; H 16, L 7,820 642 and 617;
+// H 4, L 29,140 2,173 and 1,988; B 4, H 4, L 29,140 8,304 and 11,438.
+constexpr float PART_COST = 2.2f, ALL_SPLIT_COST = 18.f, L2_COST = 0.05f;
+constexpr long L2_BYTES = 126000000;
 struct Plan {
   int G;
   bool whole;
@@ -576,9 +581,11 @@ static Plan plan(int B, int L, int H) {
   const int one = (int)(n < sms ? n : sms);                       // CTAs that take whole items
   const int g = (int)(total / 2 < sms ? total / 2 : sms);         // .. shares of two tiles at least
   if (g <= one && n <= sms) return {one, true};
-  const float t_whole = (float)(rounds * n_kv) + ROUND_COST * (float)(rounds - 1);
-  const float cost = n > sms ? ALL_SPLIT_COST : 1.f + fwd_share_cost(n, n_kv, g, PART_COST);
-  return (float)((total + g - 1) / g) + cost < t_whole ? Plan{g, false} : Plan{one, true};
+  const float walk = (float)((total + g - 1) / g);
+  const bool spills = (long)B * L * H * (4 * HD * 2) > L2_BYTES;
+  const float cost = n > sms ? ALL_SPLIT_COST + (spills ? L2_COST * walk : 0.f)
+                             : 1.f + fwd_share_cost(n, n_kv, g, PART_COST);
+  return walk + cost < (float)(rounds * n_kv) ? Plan{g, false} : Plan{one, true};
 }
 
 static int make_map(CUtensorMap* m, const void* ptr, const JvpArgs& a, const int64_t* st, int rows) {

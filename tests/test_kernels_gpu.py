@@ -265,6 +265,27 @@ def test_attention_forward_tangent_items(K, B, L, H, scale):
     K.check_status()
 
 
+@pytest.mark.parametrize("B,L,H,whole", [(3, 192, 96, True), (8, 128, 64, True), (8, 150, 60, False),
+                                          (1, 2368, 16, False), (4, 8192, 8, True)])
+def test_attention_forward_tangent_rounds(K, B, L, H, whole):
+    """More query tiles than SMs: whole items in four rounds, of two K/V tiles, pairs of query tiles in shares,
+    tiles in shares, whole items of more K and V than L2 keeps (on 148 SMs).  Bounds as above, on the
+    first and the last head of a batch."""
+    from imfvideo_b200.ops import reference as ref
+
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert (K._lib.imf_attn_fwd_scratch_bytes_hd(B, L, H, 1, 64) == 0) == whole
+    g = torch.Generator(device="cuda").manual_seed(L + H)
+    xs = [torch.randn(B, L, H, 64, device="cuda", generator=g).bfloat16() for _ in range(6)]
+    o, do, lse = K.attn_fwd(*xs)
+    for h in (slice(0, 1), slice(H - 1, H)):
+        q, k, v, dq, dk, dv = (x[:, :, h].float() for x in xs)
+        ro, rdo = ref.attention_jvp(q, k, v, dq, dk, dv, scale=0.125)
+        assert _rel(o[:, :, h], ro) < 6e-3 and _rel(do[:, :, h], rdo) < 1.2e-2
+        assert (lse[:, h] - ref.attention_lse(q, k, scale=0.125)).abs().max() < 1e-3
+    K.check_status()
+
+
 @pytest.mark.parametrize("rem", [1, 7, 8, 9, 31, 56, 57, 63])
 @pytest.mark.parametrize("tiles,scale", [(0, 0.125), (2, 0.1)])
 def test_attention_forward_tangent_ragged_tail(K, rem, tiles, scale):
