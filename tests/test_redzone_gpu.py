@@ -87,3 +87,26 @@ def test_attention_outputs_stay_inside(K, hd, L, H):
     assert wide.intact() and (wide.t[..., :48] == SENTINEL[torch.bfloat16]).all()
     assert torch.isfinite(dq.float()).all() and torch.isfinite(dk.float()).all()
     K.check_status()
+
+
+@pytest.mark.parametrize("B,L,H,hd", [(1, 65, 1, 64), (1, 333, 3, 64), (1, 2100, 2, 64), (1, 2367, 16, 64),
+                                      (4, 167, 60, 64), (1, 133, 80, 64), (8, 140, 60, 64), (1, 333, 3, 128),
+                                      (1, 2100, 2, 128)])
+def test_attention_tangent_outputs_stay_inside(K, B, L, H, hd):
+    """The forward with tangent: one item, a few, shares of few items and of more than SMs, whole items in
+    rounds, and the form with two query tiles per item, whole and in shares (on 148 SMs); ragged ends."""
+    g = torch.Generator(device="cuda").manual_seed(L)
+    xs = [torch.randn(B, L, H, hd, device="cuda", generator=g).bfloat16() for _ in range(6)]
+    o, do = (Guarded((B, L, H, hd), torch.bfloat16) for _ in range(2))
+    lse = Guarded((B, H, L), torch.float32)
+    nscr = int(K._lib.imf_attn_fwd_scratch_bytes_hd(B, L, H, 1, hd))
+    scr = Guarded((nscr // 4,), torch.float32) if nscr else None
+    rc = K._lib.imf_attn_fwd(*[t.data_ptr() for t in xs], K._ptr(o.t), K._ptr(do.t), K._ptr(lse.t), B, L, H, hd,
+                             K._bls_array(xs, 18), *o.t.stride()[:3], 1.0 / math.sqrt(hd),
+                             K._ptr(scr.t) if scr else None, nscr, K._ptr(K.status_word(xs[0].device)), K._stream())
+    assert rc == 0
+    torch.cuda.synchronize()
+    assert o.intact() and do.intact() and lse.intact() and (scr is None or scr.intact())
+    for t, want in zip((o.t, do.t, lse.t), K.attn_fwd(*xs)):
+        assert torch.equal(t, want)
+    K.check_status()

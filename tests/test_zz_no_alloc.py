@@ -170,3 +170,32 @@ def test_regular_entry_without_scratch(hd, tangent):
         assert (lse - want[2]).abs().max() < 1e-4
         assert call(4000, 40, nbytes)[0] == -1
     K.check_status()
+
+
+@pytest.mark.parametrize("L,H", [(2600, 8), (3000, 8)])
+@pytest.mark.parametrize("nbytes", [0, 4096])
+def test_tangent_in_rounds_without_scratch(L, H, nbytes):
+    """head_dim 64 with tangent, a null (or too small) scratch, more query tiles than SMs but not more pairs of
+    them: taken, whole items in two rounds in the place of shares, with the same results (bounds as above)."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from imfvideo_b200.ops import cuda as cu
+
+    assert cu.available()
+    from imfvideo_b200.ops import kernels as K
+
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("sizes are for 148 SMs")
+    assert K._lib.imf_attn_fwd_scratch_bytes_hd(1, L, H, 1, 64) > nbytes
+    g = torch.Generator(device="cuda").manual_seed(L)
+    xs = [torch.randn(1, L, H, 64, device="cuda", generator=g).bfloat16() for _ in range(6)]
+    o, do, lse = torch.empty_like(xs[0]), torch.empty_like(xs[0]), torch.empty(1, H, L, device="cuda")
+    scr = torch.empty(nbytes, dtype=torch.uint8, device="cuda") if nbytes else None
+    rc = K._lib.imf_attn_fwd(*[t.data_ptr() for t in xs], o.data_ptr(), do.data_ptr(), lse.data_ptr(), 1, L, H, 64,
+                             K._bls_array(xs, 18), L * H * 64, H * 64, 64, 0.125, K._ptr(scr), nbytes,
+                             K.status_word(torch.device("cuda", 0)).data_ptr(), K._stream())
+    assert rc == 0
+    for a, b in zip((o, do), K.attn_fwd(*xs)):
+        assert ((a.float() - b.float()).norm() / b.float().norm()) < 6e-3
+    assert (lse - K.attn_fwd(*xs)[2]).abs().max() < 1e-4
+    K.check_status()
