@@ -721,8 +721,10 @@ extern "C" long imf_attn_fwd_scratch_bytes_hd(int B, int L, int H, int tangent, 
 // bf16, head_dim 64 or 128; `strides` holds (batch, row, head) element strides for q, k, v and,
 // when tangents are given, dq, dk, dv.  o/dout contiguous-in-last-dim with
 // strides (o_sb, o_sl, o_sh).  lse: (B, H, L) fp32 or null.  scratch: device
-// buffer of imf_attn_fwd_scratch_bytes_hd() bytes.  With less (or null), problems of
-// fewer work items than SMs run with one CTA per item, others are refused.
+// buffer of imf_attn_fwd_scratch_bytes_hd() bytes.  With less (or null), problems that need some run
+// without where their work items are no more than the SMs, one CTA per item, and are refused
+// otherwise.  head_dim 64 with tangent: where pairs of 128-row query tiles, ceil(L / 256) H B, are no
+// more than the SMs; the CTAs take whole items, tiles in rounds if need be.
 extern "C" int imf_attn_fwd(const void* q, const void* k, const void* v, const void* dq,
                             const void* dk, const void* dv, void* o, void* dout, float* lse,
                             int B, int L, int H, int head_dim, const int64_t* strides,
