@@ -177,7 +177,7 @@ template <bool TANGENT>
 __global__ void __launch_bounds__(256, TANGENT ? 2 : 4) lin_states_kernel(const StatesArgs a) {
   extern __shared__ __align__(16) float sm[];
   float* X = sm;                     // [64][LP]  phi rows
-  float* Y = X + 64 * LP;            // [64][LP]  y rows | w
+  float* Y = X + 64 * LP;            // [64][LP]  y rows (their weights stay in registers)
   float* S = X;                      // result tile of the products: X is dead by then
   float* dX = Y + 64 * LP;           // tangent only
   float* dY = dX + 64 * LP;
@@ -243,8 +243,7 @@ __global__ void __launch_bounds__(256, TANGENT ? 2 : 4) lin_states_kernel(const 
   }
   *reinterpret_cast<float2*>(&zs[0][warp][2 * lane]) = zacc;
   if (TANGENT) *reinterpret_cast<float2*>(&zs[TANGENT ? 1 : 0][warp][2 * lane]) = dzacc;
-  __syncthreads();
-  frags_to_blocks(fr, S, mr, nc, g, t, d0, e0, acc);
+  frags_to_blocks(fr, S, mr, nc, g, t, d0, e0, acc);      // its barriers are zs', too
   if (TANGENT) frags_to_blocks(dfr, S, mr, nc, g, t, d0, e0, dacc);
   const int64_t base = ((int64_t)b * a.H + h) * 2 * a.nblk_pad * LSTATE + (int64_t)n * LSTATE;
   const int64_t lo_off = (int64_t)a.nblk_pad * LSTATE;
