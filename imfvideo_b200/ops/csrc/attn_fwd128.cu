@@ -218,51 +218,45 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     } else if (warp == C::WARP_MMA) {
       // -------------------------------------------------------- MMA issuer --
       if (elect_one()) {
+        constexpr uint32_t idesc_qk = idesc_bf16(TM, C::NK * BN, 0, 0);
         // Tangent: Q [K | dK]^T -> S | dS and P [V | dV] -> O | dO are one product each (operands
         // adjacent in shared memory, accumulators adjacent in TMEM).  An SM reads 128 B of
         // operands per clock, exactly what M = N = 128 from shared memory asks for; the N = 64
         // products, 6 KB per 32 clocks, wait for it.
-        constexpr uint32_t idesc_qk = idesc_bf16(TM, C::NK * BN, 0, 0);
         constexpr uint32_t idesc_dqk = idesc_bf16(TM, BN, 0, 0);
         constexpr uint32_t idesc_pv = idesc_bf16(TM, C::NK * HD, 0, 1);
         constexpr uint32_t idesc_tv = idesc_bf16(TM, HD, 0, 1);
-        // S[buf] (and dS[buf]) of tile t from K stage st
-        auto issue_qk = [&](int t, int buf, int st) {
-          const uint32_t tb = tmem + t * C::TILE_COLS;
-          const uint32_t qa = smem_u32(s.q[0][t]), ka = smem_u32(s.k[st][0]);
+        // tangent: S[buf] and dS[buf] from K stage st
+        auto issue_qk = [&](int buf, int st) {
+          const uint32_t qa = smem_u32(s.q[0][0]), dqa = smem_u32(s.q[C::NQ - 1][0]);
+          const uint32_t ka = smem_u32(s.k[st][0]);
 #pragma unroll
           for (int ks = 0; ks < HD / 16; ++ks)
-            mma_ss(tb + C::col_s(buf), sdesc_kmajor(qa + (ks / 4) * QPANEL + (ks % 4) * 32),
+            mma_ss(tmem + C::col_s(buf), sdesc_kmajor(qa + (ks / 4) * QPANEL + (ks % 4) * 32),
                    sdesc_kmajor(ka + (ks / 4) * C::NK * KPANEL + (ks % 4) * 32), idesc_qk, ks != 0);
-          if (TANGENT) {
-            const uint32_t dqa = smem_u32(s.q[C::NQ - 1][t]);
 #pragma unroll
-            for (int ks = 0; ks < HD / 16; ++ks)
-              mma_ss(tb + C::col_ds(buf), sdesc_kmajor(dqa + (ks / 4) * QPANEL + (ks % 4) * 32),
-                     sdesc_kmajor(ka + (ks / 4) * C::NK * KPANEL + (ks % 4) * 32), idesc_dqk, 1);
-          }
-          tc_commit(&s.s_full[t][buf]);
-          tc_commit(&s.k_empty[st]);      // counted once per stage: see the calls
+          for (int ks = 0; ks < HD / 16; ++ks)
+            mma_ss(tmem + C::col_ds(buf), sdesc_kmajor(dqa + (ks / 4) * QPANEL + (ks % 4) * 32),
+                   sdesc_kmajor(ka + (ks / 4) * C::NK * KPANEL + (ks % 4) * 32), idesc_dqk, 1);
+          tc_commit(&s.s_full[0][buf]);
+          tc_commit(&s.k_empty[st]);
         };
-        // `last`: the segment's final P V.  The epilogue waits on o_final, whose phases are
-        // each waited on exactly once.  It cannot use o_done: with Q K^T issued ahead, the
+        // tangent: O and dO.  `last`: the segment's final P V.  The epilogue waits on o_final, whose
+        // phases are each waited on exactly once.  It cannot use o_done: with Q K^T issued ahead, the
         // softmax warps may get there while o_done is still two phases back, and a parity
         // wait cannot tell a phase from the one two before it.
-        auto issue_pv = [&](int t, int buf, int st, bool first, bool last) {
-          const uint32_t tb = tmem + t * C::TILE_COLS;
+        auto issue_pv = [&](int buf, int st, bool first, bool last) {
           const uint32_t va = smem_u32(s.v[st][0]);
 #pragma unroll
           for (int ks = 0; ks < BN / 16; ++ks)
-            mma_ts(tb + C::COL_O, tb + C::col_p(buf) + ks * 8, sdesc_mnmajor(va + ks * 2048, KPANEL),
+            mma_ts(tmem + C::COL_O, tmem + C::col_p(buf) + ks * 8, sdesc_mnmajor(va + ks * 2048, KPANEL),
                    idesc_pv, !(first && ks == 0));
-          if (TANGENT) {
 #pragma unroll
-            for (int ks = 0; ks < BN / 16; ++ks)
-              mma_ts(tb + C::COL_DO, tb + C::col_ds(buf) + ks * 8,
-                     sdesc_mnmajor(va + ks * 2048, KPANEL), idesc_tv, 1);
-          }
-          tc_commit(&s.o_done[t]);
-          if (last) tc_commit(&s.o_final[t]);
+          for (int ks = 0; ks < BN / 16; ++ks)
+            mma_ts(tmem + C::COL_DO, tmem + C::col_ds(buf) + ks * 8,
+                   sdesc_mnmajor(va + ks * 2048, KPANEL), idesc_tv, 1);
+          tc_commit(&s.o_done[0]);
+          if (last) tc_commit(&s.o_final[0]);
         };
         const uint64_t q_desc = sdesc_kmajor(smem_u32(s.q[0][0])), k_desc = sdesc_kmajor(smem_u32(s.k[0][0]));
         long kv_it = 0, it = 0;
@@ -278,7 +272,7 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           if constexpr (C::SBUF == 2) {
             // one tile, two S buffers: Q K^T of iteration it + 1 is issued before waiting for
             // the softmax of iteration it
-            issue_qk(0, (int)(it & 1), (int)(kv_it % C::STAGES));
+            issue_qk((int)(it & 1), (int)(kv_it % C::STAGES));
             if (n_j == 1) tc_commit(&s.q_empty);
             for (int jj = 0; jj < n_j && ok; ++jj, ++kv_it, ++it) {
               const int st = (int)(kv_it % C::STAGES);
@@ -289,7 +283,7 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                                p.status, STATUS_TIMEOUT_TMA);
                 if (!ok) break;
                 tc_fence_after();
-                issue_qk(0, (int)((it + 1) & 1), st1);
+                issue_qk((int)((it + 1) & 1), st1);
                 if (jj + 2 == n_j) tc_commit(&s.q_empty);
               }
               ok = mbar_wait(&s.p_full[0][it & 1], (uint32_t)((it >> 1) & 1), abort_flag, p.status,
@@ -301,7 +295,7 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                                STATUS_TIMEOUT_SOFTMAX);
               if (!ok) break;
               tc_fence_after();
-              issue_pv(0, (int)(it & 1), st, jj == 0, jj + 1 == n_j);
+              issue_pv((int)(it & 1), st, jj == 0, jj + 1 == n_j);
               tc_commit(&s.v_empty[st]);
             }
           } else {
