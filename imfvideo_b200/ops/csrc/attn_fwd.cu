@@ -10,8 +10,8 @@
 // flash-JVP kernel (reference models/flash_jvp_kernel.py:51-570,
 // models/triton_block_jvp.py:228-346) and the FA/SDPA primal forward.
 //
-// The tangent is attn_jvp.cu's business except for short problems of more query tiles than SMs, see
-// tangent_pairs.  Work item = NT 128-row query tiles that share every 64-row K/V tile, of one (batch,
+// The tangent is attn_jvp.cu's business except for some short problems of more query tiles than SMs,
+// see tangent_pairs.  Work item = NT 128-row query tiles that share every 64-row K/V tile, of one (batch,
 // head): four tiles in the primal kernel (three or two where rounding L up to 512 rows wastes more
 // than that gains or SMs would stand idle, see primal_form), two in the tangent kernel; TMEM (512
 // columns) holds no more.  Warps
@@ -318,8 +318,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           // have while the maximum of the new scores is taken alongside: the chain S -> max -> exp
           // becomes S -> exp.  Only when a row has outgrown its reference by more than 2^8 (or has
           // none yet) is the reference moved, O rescaled and the tile, still in TMEM, done again.
-          // (B 1, H 4, L 29,140: 2.23 -> 2.12 ms.  The primal kernel, with four warps per scheduler
-          // to fill the gaps, gets slower this way: 1.08 -> 1.31 ms.)
+          // (Measured where this form still took long problems, B 1, H 4, L 29,140: 2.23 -> 2.12 ms.  The
+          // primal kernel, with four warps per scheduler to fill the gaps, gets slower this way:
+          // 1.08 -> 1.31 ms.)
           const bool first = j == sg.j0;
           uint32_t pk[BN / 2];
           uint32_t tk[BN / 2];
