@@ -559,17 +559,17 @@ attn_jvp_combine_kernel(const Params p, int G) {
 }
 
 // Whole items, CTA c taking items c, c + G, ..., or equal shares of the (item, K/V tile) space with a
-// merge.  Either way an item costs some 5 us besides its K/V tiles (queries' load, empty pipeline,
-// epilogue), so only what differs is counted, in K/V tiles of 0.57 to 0.7 us.  Shares of more items than
-// SMs cost 18 for the two parts that each CTA stores and the merge; where all heads' K | dK | V | dV,
-// which shares walk at once and rounds a few heads at a time, are more than L2 holds, 5 % of the walk
-// besides (half of such shapes lose more, up to 40 %).  Shares of fewer items cost what fwd_share_cost
-// says with PART_COST.  986 shapes of 1 to 128 heads and 64 to 32,760 rows in 2 to 70 rounds, either way
-// timed in turn: 0.2 % behind the better one on average (8 % when a round was charged 12 tiles and shares
-// 32).  Whole and shared: B 3, H 96, L 192, four rounds 30.6 us and 58.4; H 16, L 7,820 642 and 617;
-// H 4, L 29,140 2,173 and 1,988; B 4, H 4, L 29,140 8,304 and 11,438.
-constexpr float PART_COST = 2.2f, ALL_SPLIT_COST = 18.f, L2_COST = 0.05f;
-constexpr long L2_BYTES = 126000000;
+// merge.  More items than SMs: walks of up to SHORT_WALK tiles always whole, since a share saves less than a
+// walk and the two parts that each CTA stores and the merge cost some 18 tiles, 10 us (632 shapes of
+// 1 to 128 heads, either way timed in turn, whole the faster in each: B 3, H 96, L 192, four rounds 30.6 us
+// against 58.4; B 8, H 20, L 768 86.1 and 116.8).  Longer walks by an account in K/V tiles, of 0.57 to 0.7 us:
+// a further round is charged 12 and shares 32 (H 4, L 29,140 2,173 us whole, 1,988 shared; H 16, L 7,820
+// 642 and 617; 354 shapes, 4 % behind the better way on average: whole rounds are faster where the last is
+// nearly full, and where K, V and tangents of all heads, which shares walk at once and rounds a few heads
+// at a time, are beyond L2: B 4, H 4, L 29,140 8.3 ms whole, 11.4 shared).  Fewer items: fwd_share_cost
+// with PART_COST (1 head, 6,500 rows 63.5 us whole, 41.8 shared; 8 heads, 2,068 rows 28.4 and 37.1).
+constexpr float PART_COST = 2.2f, ROUND_COST = 12.f, ALL_SPLIT_COST = 32.f;
+constexpr int SHORT_WALK = 16;
 struct Plan {
   int G;
   bool whole;
@@ -580,12 +580,10 @@ static Plan plan(int B, int L, int H) {
   const long total = n * n_kv, rounds = (n + sms - 1) / sms;
   const int one = (int)(n < sms ? n : sms);                       // CTAs that take whole items
   const int g = (int)(total / 2 < sms ? total / 2 : sms);         // .. shares of two tiles at least
-  if (g <= one && n <= sms) return {one, true};
-  const float walk = (float)((total + g - 1) / g);
-  const bool spills = (long)B * L * H * (4 * HD * 2) > L2_BYTES;
-  const float cost = n > sms ? ALL_SPLIT_COST + (spills ? L2_COST * walk : 0.f)
-                             : 1.f + fwd_share_cost(n, n_kv, g, PART_COST);
-  return walk + cost < (float)(rounds * n_kv) ? Plan{g, false} : Plan{one, true};
+  if (n > sms ? n_kv <= SHORT_WALK : g <= one) return {one, true};
+  const float t_whole = (float)(rounds * n_kv) + ROUND_COST * (float)(rounds - 1);
+  const float cost = n > sms ? ALL_SPLIT_COST : 1.f + fwd_share_cost(n, n_kv, g, PART_COST);
+  return (float)((total + g - 1) / g) + cost < t_whole ? Plan{g, false} : Plan{one, true};
 }
 
 static int make_map(CUtensorMap* m, const void* ptr, const JvpArgs& a, const int64_t* st, int rows) {
