@@ -22,17 +22,17 @@
 //
 // What bounds it.  The tensor core needs 832 clocks a step (Q [K | dK] 4 x 64, dQ K 4 x 48: 6 KB of
 // operands at 128 B / clock, P [V | dV] 4 x 64, T V 4 x 32), the exponential unit 512.  B 1, H 4,
-// L 29,140: 1.81 ms, 1,220 clocks a step (2.05 ms in a form with two query tiles per item, one S | dS
-// buffer per tile with P over it and one issuing thread); in a loop, at the power cap, 2.14 ms at
-// 1,480 MHz (2.40 at 1,670).  What counted:
+// L 29,140: 1.84 ms alone, 2.14 ms in a loop at the power cap, 1,030 clocks a step either way by the SM's
+// own counter (2.05 and 2.40 ms in a form with two query tiles per item, one S | dS buffer per tile with P
+// over it and one issuing thread).  What counted, alone, as measured when each was made:
 //  - two issuing warps: an MMA costs its thread some 20 clocks, a commit or a satisfied wait 60 to 150,
 //    so one thread with a step's 16 MMAs, 5 commits and 4 waits took 1,600 clocks (2.23 -> 2.09 ms);
 //  - the reference maximum handed over as one tagged word in shared memory instead of named
 //    barriers (2.09 -> 2.05 ms);
 //  - dS loaded only after the maximum has been taken: with S and dS live at once the compiler moves
 //    registers about, 558 -> 539 instructions a step (2.05 -> 1.92 ms);
-//  - a scale that is a power of two multiplied into q and dq in shared memory, once per item and
-//    exactly, instead of into every T (1.90 -> 1.81 ms).
+//  - a scale that is a power of two multiplied into q and dq in shared memory, once per item, instead of
+//    into every T (1.90 -> 1.81 ms).
 // Exponentials against a stale reference with the tile done again where it was outgrown, and loads
 // issued a step ahead, were slower (2.11 to 2.65 ms: registers moved).
 //
@@ -647,7 +647,8 @@ long attn_jvp_scratch_bytes(int B, int L, int H) {
 }
 
 int attn_jvp_launch(const JvpArgs& a) {
-  // scales that are powers of two (head_dim 64: 1/8) go into q and dq, exactly
+  // Scales that are powers of two (head_dim 64: 1/8) go into q and dq, from 2^-8 to 1: nothing can
+  // overflow, and only elements below 2^-118 lose bits.
   int e;
   const bool unit = a.scale > 0x1p-9f && a.scale <= 1.f && frexpf(a.scale, &e) == 0.5f;
   return unit ? jvp::launch<true>(a) : jvp::launch<false>(a);
